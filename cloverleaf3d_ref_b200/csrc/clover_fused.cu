@@ -1330,7 +1330,7 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
   using I3 = std::integral_constant<int, 3>;
   if (dir == 1 && x_maps && !tg.plan) {
     // one pass, its planes staged in shared memory
-    launch_mom_x_tma<S>(tg.g, s, sweep, kMarchSeg, *x_maps, ga, vel_out, level0, status);
+    launch_mom_x_tma<S>(tg.g, s, sweep, *x_maps, ga, vel_out, level0, status);
   } else if (dir == 1) {
     // one pass for the three velocities
     auto sweep_x = [&](auto var) {

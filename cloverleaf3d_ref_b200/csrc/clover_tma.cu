@@ -13,6 +13,7 @@
 //                 cell planes l-1, l, l+1; one thread refills the buffer of
 //                 plane l-1 with plane l-1+R once the block is done with l.
 #include <cfloat>
+#include <cmath>
 #include <cstdio>
 
 #include <cudaTypedefs.h>
@@ -2197,7 +2198,33 @@ k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellX
 }
 
 constexpr int kViscRing = 4;
-constexpr int kViscSeg = 32;
+
+// Planes per block of a staged march over `planes` planes with `tiles` blocks
+// per plane. A block pays for about three planes before its first result (its
+// ring fills, and its first planes are read twice), which long segments
+// spread, and the launch's last wave takes a whole segment, which short ones
+// keep short: with T = tiles * planes the sum T/R (1 + 3/seg) + seg over R
+// resident blocks is smallest near seg = sqrt(3 T / R), R = 148 SMs * 2 to 3.
+// sqrt(T / 120) follows the best segments measured, FP64 and mixed, step time
+// at the best against at 32 planes (the register forms in brackets):
+// 1 at 32^3 (201 us, [454]), 4 at 96^3 (582 against 940 [805]), 8 at 128^3
+// (927 against 1126 [1148]), 8 at 160^3 (1408 against 1633 [1727]), 16 at
+// 203 x 311 x 118 (2030 against 2107 [2557]), 24 at 256^3 (3939 against 3990), 32
+// from 300^3 on (48 gains and loses less than 1% at 512^3).
+int plane_seg(long long tiles, int planes) {
+  int seg = (int)(sqrt((double)tiles * planes / 120.0) + 0.5);
+  if (seg > 32) seg = 32;
+  if (seg > planes) seg = planes;
+  if (seg < 1) seg = 1;
+  const int n = (planes + seg - 1) / seg;  // segments of even length
+  return (planes + n - 1) / n;
+}
+
+// The launch grid of a staged march (x, y tiles; z segments), and its segment.
+dim3 plane_grid(int tiles_x, int tiles_y, int planes, int* seg) {
+  *seg = plane_seg((long long)tiles_x * tiles_y, planes);
+  return dim3(tiles_x, tiles_y, (planes + *seg - 1) / *seg);
+}
 
 }  // namespace
 
@@ -2233,9 +2260,10 @@ void launch_visc_dt_tma(const Geom& g, cudaStream_t s, const ViscMaps& maps, con
                         unsigned long long* min_key, int* status) {
   auto kern = k_visc_dt_tma<S, kViscRing, kViscMinBlocks<S>>;
   const int smem = kViscRing * ViscPlane<S>::kBytes;
-  const dim3 grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
-                  (g.z_max - g.z_min + kViscSeg) / kViscSeg);
-  kern<<<grid, dim3(TX, TY), smem, s>>>(g, kViscSeg, ga, g_small, dtc_safe, dtu_safe, dtv_safe,
+  int seg;
+  const dim3 grid = plane_grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
+                               g.z_max - g.z_min + 1, &seg);
+  kern<<<grid, dim3(TX, TY), smem, s>>>(g, seg, ga, g_small, dtc_safe, dtu_safe, dtv_safe,
                                          dtw_safe, dtdiv_safe, maps, pressure,
                                          viscosity, soundspeed, min_key, status);
 }
@@ -2255,11 +2283,12 @@ bool mom_x_tma_prepare() {
 }
 
 template <class S>
-void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, int seg, const MomXMaps& maps,
+void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
                       const Level0<S>& level0, int* status) {
-  const dim3 grid((g.x_max + 1 - g.x_min + 1 + 28) / 29, (g.y_max + 1 - g.y_min + 1 + TY - 1) / TY,
-                  (g.z_max + 1 - g.z_min + 1 + seg - 1) / seg);
+  int seg;
+  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + 1 + 28) / 29,
+                               (g.y_max + 1 - g.y_min + 1 + TY - 1) / TY, g.z_max - g.z_min + 2, &seg);
   // post_vol variant: 0 on sweep 1, 4 (the cell volume) on sweep 3
   if (sweep == 1)
     k_mom_sweep_x_tma<S, 0, kMomXRing, kMomXMinBlocks<S>>
@@ -2289,7 +2318,7 @@ __global__ void k_wait_selftest(long long cycles, int* status) {
   if (!done && threadIdx.x == 0) atomicOr(status, CLOVER_STATUS_TIMEOUT);
 }
 
-constexpr int kStencilRing = 4, kStencilSeg = 32;
+constexpr int kStencilRing = 4;
 // blocks per SM: FP64 holds three (56-72 registers, 60-69 KB of plane
 // buffers), the mixed forms four
 template <class S>
@@ -2306,18 +2335,6 @@ bool stencils_tma_prepare() {
          cudaFuncSetAttribute(k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                               kStencilRing * FluxPlane<S>::kBytes) == cudaSuccess;
-}
-
-// Planes per block of a staged drop-in stencil over nz planes with xy blocks
-// per plane: 32 where that leaves at least eight blocks per SM (148 SMs),
-// fewer on small chunks (down to 4), whose blocks would otherwise each march
-// a long column of planes with most SMs idle.
-int drop_seg(int nz, int xy) {
-  const long long want = 148LL * 8;
-  long long seg = ((long long)nz * xy + want - 1) / want;
-  if (seg > kStencilSeg) seg = kStencilSeg;
-  if (seg < 4) seg = 4;
-  return (int)seg;
 }
 
 // blocks per SM of the drop-in PdV: the corrector's plane (six velocity
@@ -2340,8 +2357,8 @@ void launch_pdv_dropin_tma(const Geom& g, cudaStream_t s, bool predict, double d
                            double* density1, const double* energy0, double* energy1,
                            const double* pressure, const double* viscosity, int* status) {
   const int gx = (g.x_max - g.x_min + TX) / TX, gy = (g.y_max - g.y_min + TY) / TY;
-  const int nz = g.z_max - g.z_min + 1, seg = drop_seg(nz, gx * gy);
-  const dim3 grid(gx, gy, (nz + seg - 1) / seg);
+  int seg;
+  const dim3 grid = plane_grid(gx, gy, g.z_max - g.z_min + 1, &seg);
   if (predict)
     k_pdv_dropin_tma<true, kStencilRing, kPdvDropMinBlocks<true>>
         <<<grid, dim3(TX, TY), kStencilRing * PdvDropPlane<true>::kBytes, s>>>(
@@ -2374,8 +2391,8 @@ void launch_calc_dt_dropin_tma(const Geom& g, cudaStream_t s, const GeomArrays& 
                                double dtdiv_safe, const DtDropMaps& maps, double* dt_min,
                                unsigned long long* min_key, int* status) {
   const int gx = (g.x_max - g.x_min + TX) / TX, gy = (g.y_max - g.y_min + TY) / TY;
-  const int nz = g.z_max - g.z_min + 1, seg = drop_seg(nz, gx * gy);
-  const dim3 grid(gx, gy, (nz + seg - 1) / seg);
+  int seg;
+  const dim3 grid = plane_grid(gx, gy, g.z_max - g.z_min + 1, &seg);
   k_calc_dt_dropin_tma<kStencilRing, kDropMinBlocks>
       <<<grid, dim3(TX, TY), kStencilRing * DtDropPlane::kBytes, s>>>(
           g, seg, ga, g_small, dtc_safe, dtu_safe, dtv_safe, dtw_safe, dtdiv_safe, maps,
@@ -2385,8 +2402,8 @@ void launch_calc_dt_dropin_tma(const Geom& g, cudaStream_t s, const GeomArrays& 
 void launch_viscosity_dropin_tma(const Geom& g, cudaStream_t s, const GeomArrays& ga,
                                  const ViscDropMaps& maps, double* viscosity, int* status) {
   const int gx = (g.x_max - g.x_min + TX) / TX, gy = (g.y_max - g.y_min + TY) / TY;
-  const int nz = g.z_max - g.z_min + 1, seg = drop_seg(nz, gx * gy);
-  const dim3 grid(gx, gy, (nz + seg - 1) / seg);
+  int seg;
+  const dim3 grid = plane_grid(gx, gy, g.z_max - g.z_min + 1, &seg);
   k_viscosity_dropin_tma<kStencilRing, kDropMinBlocks>
       <<<grid, dim3(TX, TY), kStencilRing * ViscDropPlane::kBytes, s>>>(g, seg, ga, maps,
                                                                          viscosity, status);
@@ -2396,8 +2413,8 @@ void launch_accelerate_dropin_tma(const Geom& g, cudaStream_t s, double dt,
                                   const AccDropMaps& maps, double* xvel1, double* yvel1,
                                   double* zvel1, int* status) {
   const int gx = (g.x_max + 1 - g.x_min + TX) / TX, gy = (g.y_max + 1 - g.y_min + TY) / TY;
-  const int nz = g.z_max - g.z_min + 2, seg = drop_seg(nz, gx * gy);
-  const dim3 grid(gx, gy, (nz + seg - 1) / seg);
+  int seg;
+  const dim3 grid = plane_grid(gx, gy, g.z_max - g.z_min + 2, &seg);
   k_accelerate_dropin_tma<kStencilRing, kDropMinBlocks>
       <<<grid, dim3(TX, TY), kStencilRing * AccDropPlane::kBytes, s>>>(g, seg, dt, maps, xvel1,
                                                                         yvel1, zvel1, status);
@@ -2421,17 +2438,17 @@ void launch_mom_node_dropin_tma(const Geom& g, cudaStream_t s, int dir, const No
   const int smem = kStencilRing * NodeDropPlane::kBytes;
   if (dir == 1) {  // nodes x_min-2..x_max+2, 32 per tile
     const int gx = (g.x_max - g.x_min + 5 + TX - 1) / TX, gy = (g.y_max - g.y_min + 2 + TY - 1) / TY;
-    const int nz = g.z_max - g.z_min + 2, seg = drop_seg(nz, gx * gy);
-    k_mom_node_x_dropin_tma<kStencilRing, 4><<<dim3(gx, gy, (nz + seg - 1) / seg), dim3(TX, TY),
-                                               smem, s>>>(g, seg, maps, node_flux, node_mass_post,
+    int seg;
+    const dim3 grid = plane_grid(gx, gy, g.z_max - g.z_min + 2, &seg);
+    k_mom_node_x_dropin_tma<kStencilRing, 4><<<grid, dim3(TX, TY), smem, s>>>(g, seg, maps, node_flux, node_mass_post,
                                                           node_mass_pre, status);
     return;
   }
   const int nr = (dir == 2 ? g.z_max - g.z_min : g.y_max - g.y_min) + 2;
   const int np = (dir == 2 ? g.y_max - g.y_min : g.z_max - g.z_min) + 5;
   const int gx = (g.x_max + 1 - g.x_min + TX) / TX, gy = (nr + TY - 1) / TY;
-  const int seg = drop_seg(np, gx * gy);
-  const dim3 grid(gx, gy, (np + seg - 1) / seg);
+  int seg;
+  const dim3 grid = plane_grid(gx, gy, np, &seg);
   if (dir == 2)
     k_mom_node_dropin_tma<2, kStencilRing, 4><<<grid, dim3(TX, TY), smem, s>>>(
         g, seg, maps, node_flux, node_mass_post, node_mass_pre, status);
@@ -2461,25 +2478,27 @@ void launch_cell_sweep_x_tma(const Geom& g, cudaStream_t s, int sweep, const Cel
                              typename S::ene_t* e_out, typename S::mf_t* mass_flux_x,
                              const Level0<S>& level0, int* status) {
   // faces x_min..x_max+2, 31 per warp
-  const dim3 grid((g.x_max - g.x_min + 3 + kCellXLanes - 1) / kCellXLanes,
-                  (g.y_max - g.y_min + TY) / TY, (g.z_max - g.z_min + kStencilSeg) / kStencilSeg);
+  int seg;
+  const dim3 grid = plane_grid((g.x_max - g.x_min + 3 + kCellXLanes - 1) / kCellXLanes,
+                               (g.y_max - g.y_min + TY) / TY, g.z_max - g.z_min + 1, &seg);
   if (sweep == 1)
     k_cell_sweep_x_tma<S, 0, kStencilRing, kCellXMinBlocks<S>>
         <<<grid, dim3(TX, TY), kStencilRing * CellXPlane<S, 0>::kBytes, s>>>(
-            g, kStencilSeg, ga, maps, d_out, e_out, mass_flux_x, level0, status);
+            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, status);
   else
     k_cell_sweep_x_tma<S, 1, kStencilRing, kCellXMinBlocks<S>>
         <<<grid, dim3(TX, TY), kStencilRing * CellXPlane<S, 1>::kBytes, s>>>(
-            g, kStencilSeg, ga, maps, d_out, e_out, mass_flux_x, level0, status);
+            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, status);
 }
 
 template <class S>
 void launch_pdv_predict_eos_tma(const Geom& g, cudaStream_t s, const double* dt_ptr,
                                 const PdvMaps& maps, typename S::cs_t* pressure, int* status) {
-  const dim3 grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
-                  (g.z_max - g.z_min + kStencilSeg) / kStencilSeg);
+  int seg;
+  const dim3 grid = plane_grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
+                               g.z_max - g.z_min + 1, &seg);
   k_pdv_predict_eos_tma<S, kStencilRing, kStencilMinBlocks<S>>
-      <<<grid, dim3(TX, TY), kStencilRing * PdvPlane<S>::kBytes, s>>>(g, kStencilSeg, dt_ptr, maps,
+      <<<grid, dim3(TX, TY), kStencilRing * PdvPlane<S>::kBytes, s>>>(g, seg, dt_ptr, maps,
                                                                        pressure, status);
 }
 
@@ -2487,10 +2506,11 @@ template <class S>
 void launch_accelerate_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
                            typename S::vel_t* xvel1, typename S::vel_t* yvel1,
                            typename S::vel_t* zvel1, int* status) {
-  const dim3 grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
-                  (g.z_max + 1 - g.z_min + kStencilSeg) / kStencilSeg);
+  int seg;
+  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
+                               g.z_max - g.z_min + 2, &seg);
   k_accelerate_tma<S, kStencilRing, kStencilMinBlocks<S>>
-      <<<grid, dim3(TX, TY), kStencilRing * AccPlane<S>::kBytes, s>>>(g, kStencilSeg, dt_ptr, maps,
+      <<<grid, dim3(TX, TY), kStencilRing * AccPlane<S>::kBytes, s>>>(g, seg, dt_ptr, maps,
                                                                       xvel1, yvel1, zvel1, status);
 }
 
@@ -2501,11 +2521,12 @@ void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, co
                          const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
                          typename S::vf_t* vol_flux_z, int* status) {
-  const dim3 grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
-                  (g.z_max + 1 - g.z_min + kStencilSeg) / kStencilSeg);
+  int seg;
+  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
+                               g.z_max - g.z_min + 2, &seg);
   k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>
       <<<grid, dim3(TX, TY), kStencilRing * FluxPlane<S>::kBytes, s>>>(
-          g, kStencilSeg, dt_ptr, maps, density0, density1, energy0, energy1, pressure, viscosity,
+          g, seg, dt_ptr, maps, density0, density1, energy0, energy1, pressure, viscosity,
           vol_flux_x, vol_flux_y, vol_flux_z, status);
 }
 
@@ -2531,9 +2552,10 @@ void launch_mom_node_tma(const Geom& g, cudaStream_t s, int dir, int var, const 
                          typename S::nd_t* node_flux, typename S::nd_t* node_mass_post,
                          typename S::nd_t* node_mass_pre, int* status) {
   auto go = [&](auto kern, int bytes, const MarchRange& r) {
-    const dim3 grid((r.jhi - r.jlo + 1 + 30) / 31, (r.chi - r.clo + 1 + TY - 1) / TY,
-                    (r.phi - r.plo + 1 + kStencilSeg - 1) / kStencilSeg);
-    kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, kStencilSeg, maps, node_flux,
+    int seg;
+    const dim3 grid = plane_grid((r.jhi - r.jlo + 1 + 30) / 31, (r.chi - r.clo + 1 + TY - 1) / TY,
+                                 r.phi - r.plo + 1, &seg);
+    kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, seg, maps, node_flux,
                                                           node_mass_post, node_mass_pre, status);
   };
   if (dir == 3) {
@@ -2569,10 +2591,11 @@ void launch_mom_vel_tma(const Geom& g, cudaStream_t s, int dir, const VelMaps& m
                         const typename S::nd_t* node_mass_pre, typename S::vel_t* const* vel_in,
                         typename S::vel_t* const* vel_out, const Level0<S>& level0, int* status) {
   auto go = [&](auto kern, const MarchRange& r) {
-    const dim3 grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY,
-                    (r.phi - r.plo + kStencilSeg) / kStencilSeg);
+    int seg;
+    const dim3 grid = plane_grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY,
+                                 r.phi - r.plo + 1, &seg);
     kern<<<grid, dim3(TX, TY), kVelRing * VelPlane<S>::kBytes, s>>>(
-        g, kStencilSeg, ga, maps, node_flux, node_mass_pre, vel_in[0], vel_in[1], vel_in[2],
+        g, seg, ga, maps, node_flux, node_mass_pre, vel_in[0], vel_in[1], vel_in[2],
         vel_out[0], vel_out[1], vel_out[2], level0, status);
   };
   if (dir == 2) go(k_mom_vel_tma<S, 2, kVelRing, kVelMinBlocks<S>>, mom_vel_range<2>(g));
@@ -2604,9 +2627,9 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                            const typename S::vf_t* vfy, const typename S::vf_t* vfz,
                            typename S::mf_t* mass_flux, const Level0<S>& level0, int* status) {
   auto go = [&](auto kern, int bytes, const MarchRange& r, int pcells) {
-    const dim3 grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY,
-                    (pcells + kStencilSeg - 1) / kStencilSeg);
-    kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, kStencilSeg, ga, maps, d_in, e_in,
+    int seg;
+    const dim3 grid = plane_grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY, pcells, &seg);
+    kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, seg, ga, maps, d_in, e_in,
                                                           d_out, e_out, vfx, vfy, vfz, mass_flux,
                                                           level0, status);
   };
@@ -2653,7 +2676,7 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                                        const S::rho_t*, S::rho_t*, const S::ene_t*, S::ene_t*,   \
                                        const S::cs_t*, const S::cs_t*, S::vf_t*, S::vf_t*,       \
                                        S::vf_t*, int*);                                          \
-  template void launch_mom_x_tma<S>(const Geom&, cudaStream_t, int, int, const MomXMaps&,        \
+  template void launch_mom_x_tma<S>(const Geom&, cudaStream_t, int, const MomXMaps&,             \
                                     const GeomArrays&, S::vel_t* const*, const Level0<S>&, int*); \
   template void launch_visc_dt_tma<S>(const Geom&, cudaStream_t, const ViscMaps&, const GeomArrays&, \
                                       double, double, double, double, double, double, S::cs_t*,  \

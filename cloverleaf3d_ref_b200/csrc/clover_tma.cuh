@@ -54,9 +54,9 @@ struct MomXMaps {
 template <class S>
 bool mom_x_tma_prepare();
 // The x momentum sweep of one chunk (sweep 1 or 3 of the step), its planes
-// staged by bulk-tensor copies; seg planes per block along z.
+// staged by bulk-tensor copies.
 template <class S>
-void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, int seg, const MomXMaps& maps,
+void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
                       const Level0<S>& level0, int* status);
 

@@ -1,0 +1,38 @@
+"""Staged marches whose segments end unevenly.
+
+The planes a staged block marches follow from the launch's tiles and planes, so
+the first, last and shortest segments fall on other planes as a grid grows: one
+plane per block on the smallest grids, up to 32 on the largest."""
+import numpy as np
+import pytest
+
+import cloverleaf3d_ref_b200 as C
+import decks
+import oracle_lib as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(3, 3, 3), (33, 9, 5), (31, 8, 61), (64, 65, 33), (40, 130, 97), (130, 40, 67)])
+def test_native_and_dropin_bitwise_over_segments(nx, ny, nz):
+    d = decks.shock(nx, ny, nz, 5, states=decks.MIXED_STATES)
+    ref = O.run(d, want_fields=True)
+    ch = C.Chunk(decks.to_deck(d))
+    assert ch.use_tma(True)
+    di = C.DropIn(decks.to_deck(d))
+    for run in (ch, di):
+        assert run.run() == ref["steps"]
+        assert np.array_equal(run.dt_history(), ref["dt"])
+        for name, want in ref["fields"].items():
+            assert np.array_equal(run.field(name), want), name
+        run.close()
+    # FP32 storage: staged against register forms
+    out = []
+    for tma in (True, False):
+        ch = C.Chunk(decks.to_deck(d), C.PRECISION_MIXED)
+        assert ch.use_tma(tma) == tma
+        ch.run()
+        out.append([ch.field(n) for n in C.FIELD_NAMES])
+        ch.close()
+    for a, b, name in zip(*out, C.FIELD_NAMES):
+        assert np.array_equal(a, b), name
