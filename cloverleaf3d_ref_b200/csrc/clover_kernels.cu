@@ -1401,6 +1401,134 @@ __global__ void k_halo_x(M m, HaloLaunch h, int depth, int do_low, int do_high) 
   });
 }
 
+// ---------------------------------------------------------------------------
+// The same update in one launch, for grids of three or more cells per axis
+// with every face external. There the three face passes compose: a halo cell
+// ends up with the (signed) value of one interior cell, its index mirrored on
+// each axis, whatever the halo held before. Only the x- and y-face fluxes
+// keep one exception: the z faces stop one short of their far edge
+// (update_halo_kernel.f90:1018-1280, max+depth instead of max+1+depth along
+// the flux's own axis), so in the z halo planes that edge keeps the mirror of
+// what the plane held BEFORE the call. The thread that rewrites the mirrored
+// cell of such a plane loads its old value and writes the edge from it too;
+// no other thread reads a halo cell, so the passes need no order.
+//
+// Tiles: z faces, 32 x 8 of (j, k); y faces, 32 x 8 of (j, l); x faces, 32 x 8
+// of (k, l); tile.y = field. A thread copies both layers of both sides, its
+// loads all in flight before its stores. Bounds: launches and latency on
+// small grids (three dependent kernels of up to 19 fields in series, 23 us
+// for a sweep's seven fields at 32^3, 1.9 us in one launch here), the 32-byte
+// sector behind every x-face element on large ones.
+struct HaloOne {
+  void* f[19];
+  void* also[19];  // a second array that takes the same halo, or null
+  signed char bytes[19], kind[19], comp[19];
+  int n;
+};
+
+// Last interior index past the cell count on an axis (0 or 1).
+__host__ __device__ __forceinline__ int halo_hi(int kind, int comp, int axis) {
+  return kind == 1 || (kind == 2 && comp == axis) ? 1 : 0;
+}
+// The interior index a halo index x of an axis of n cells mirrors; flips neg
+// where the reference negates.
+__device__ __forceinline__ int halo_mirror(int kind, int comp, int axis, int n, int x, bool& neg) {
+  const int hi = halo_hi(kind, comp, axis);
+  if (x >= 1 && x <= n + hi) return x;
+  if (kind != 0 && comp == axis) neg = !neg;
+  if (x < 1) return (kind == 0 ? 0 : 1) + 1 - x;
+  return n + (kind == 2 && comp != axis ? 0 : 1) - (x - n - hi);
+}
+
+// One tile of the faces normal to AX of one field; w tiles per tile row.
+template <int D, int AX, class T>
+__device__ __forceinline__ void halo_faces(const Geom& g, const HaloOne& h, int fi, int r, int w) {
+  const int kind = h.kind[fi], comp = h.comp[fi];
+  T* __restrict__ p = (T*)h.f[fi];
+  T* __restrict__ p2 = (T*)h.also[fi];
+  const int n[3] = {g.x_max, g.y_max, g.z_max};
+  const int hi[3] = {halo_hi(kind, comp, 0), halo_hi(kind, comp, 1), halo_hi(kind, comp, 2)};
+  const int u = (r % w) * 32 + (int)threadIdx.x, v = (r / w) * 8 + (int)threadIdx.y;
+  // the tangential extents: z faces whole planes, y faces interior planes, x
+  // faces interior rows of interior planes
+  int c[3] = {AX == 0 ? 0 : 1 - D + u, AX == 0 ? 1 + u : AX == 2 ? 1 - D + v : 0, AX == 2 ? 0 : 1 + v};
+  if (AX != 0 && c[0] > n[0] + hi[0] + D) return;
+  if (AX != 1 && c[1] > n[1] + hi[1] + (AX == 2 ? D : 0)) return;
+  if (AX != 2 && c[2] > n[2] + hi[2]) return;
+  bool neg = false;
+  int s[3] = {0, 0, 0};
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    if (a != AX) s[a] = halo_mirror(kind, comp, a, n[a], c[a], neg);
+  // the z planes of an x or y flux: its own axis (ce of ne), the other (co of no)
+  const bool flux = AX == 2 && kind == 2 && comp < 2;
+  const int ce = comp == 0 ? c[0] : c[1], ne = comp == 0 ? n[0] : n[1];
+  const int co = comp == 0 ? c[1] : c[0], no = comp == 0 ? n[1] : n[0];
+  if (flux && ce == ne + 1 + D) return;  // the far edge is written with its mirrored cell, below
+  const bool edge = flux && ce == ne + 1 - D && co >= 1 && co <= no;
+  T val[2 * D], old[2 * D];
+  long long to[2 * D];
+#pragma unroll
+  for (int q = 0; q < 2 * D; q++) {
+    const int m = q / 2 + 1;
+    c[AX] = q & 1 ? n[AX] + hi[AX] + m : 1 - m;
+    bool ng = neg;
+    s[AX] = halo_mirror(kind, comp, AX, n[AX], c[AX], ng);
+    to[q] = off3(g, c[0], c[1], c[2]);
+    const T x = p[off3(g, s[0], s[1], s[2])];
+    val[q] = ng ? -x : x;
+    old[q] = edge ? p[to[q]] : T(0);
+  }
+#pragma unroll
+  for (int q = 0; q < 2 * D; q++) {
+    p[to[q]] = val[q];
+    if (p2) p2[to[q]] = val[q];
+  }
+  if constexpr (AX == 2) {
+    if (!edge) return;
+    // the far edge in this row, and in the halo rows that mirror it
+    for (int i = -D; i <= D; i++) {
+      const int row = i == 0 ? co : i < 0 ? 1 + i : no + i;
+      bool ng = false;
+      if (halo_mirror(2, comp, 1 - comp, no, row, ng) != co) continue;
+#pragma unroll
+      for (int q = 0; q < 2 * D; q++) {
+        const int l = q & 1 ? n[2] + q / 2 + 1 : -(q / 2);
+        const long long at = comp == 0 ? off3(g, ne + 1 + D, row, l) : off3(g, row, ne + 1 + D, l);
+        p[at] = -old[q];
+        if (p2) p2[at] = -old[q];
+      }
+    }
+  }
+}
+
+template <int D, class T>
+__device__ __forceinline__ void halo_one(const Geom& g, const HaloOne& h, int fi, int tile) {
+  const int wx = (g.x_max + 2 * D + 1 + 31) / 32, wy = (g.y_max + 1 + 31) / 32;
+  const int tz = wx * ((g.y_max + 2 * D + 1 + 7) / 8), ty = wx * ((g.z_max + 1 + 7) / 8);
+  if (tile < tz) halo_faces<D, 2, T>(g, h, fi, tile, wx);
+  else if (tile < tz + ty) halo_faces<D, 1, T>(g, h, fi, tile - tz, wx);
+  else halo_faces<D, 0, T>(g, h, fi, tile - tz - ty, wy);
+}
+
+template <int D, class M>
+__global__ void __launch_bounds__(BX * BY) k_halo_one(M m, const __grid_constant__ HaloOne h) {
+  m.run([&](const Geom& g, const Tile& t) {
+    if (h.bytes[t.y] == 8) halo_one<D, double>(g, h, t.y, t.x);
+    else halo_one<D, float>(g, h, t.y, t.x);
+  });
+}
+
+// tiles of k_halo_one; aux = fields
+template <int D>
+dim3 grid_halo_one(const Geom& g, int fields) {
+  const int nx = g.x_max, ny = g.y_max, nz = g.z_max;
+  const int wx = (nx + 2 * D + 1 + 31) / 32;
+  return dim3(wx * ((ny + 2 * D + 1 + 7) / 8) + wx * ((nz + 1 + 7) / 8) +
+                  ((ny + 1 + 31) / 32) * ((nz + 1 + 7) / 8),
+              fields, 1);
+}
+
 // tasks of k_halo_x in blocks of BX * BY; aux = tasks per row (fields * 2 * depth)
 dim3 grid_halo_x_tasks(const Geom& g, int per_row, int depth) {
   const long long na = g.y_max - g.y_min + 2 + 2 * depth, nb = g.z_max - g.z_min + 2 + 2 * depth;
@@ -1758,10 +1886,32 @@ static int elem_bytes_of(int id) {
 
 template <class S>
 void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, const int* fields,
-                        int depth, const int* external_faces) {
+                        int depth, const int* external_faces, bool composed, const HaloFields* also) {
   // field id -> (kind, component)
   static const int kind[19] = {0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2};
   static const int comp[19] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 2, 2, 0, 1, 2, 0, 1, 2};
+  if (composed) {
+    HaloOne h{};
+    for (int id = 1; id <= 19; id++) {
+      if (fields[id - 1] != 1) continue;
+      const int i = h.n++;
+      h.f[i] = f.f[id - 1];
+      h.also[i] = also ? also->f[id - 1] : nullptr;
+      h.bytes[i] = (signed char)elem_bytes_of<S>(id);
+      h.kind[i] = (signed char)kind[id - 1];
+      h.comp[i] = (signed char)comp[id - 1];
+    }
+    if (h.n == 0) return;
+    const dim3 blk(BX, BY);
+    const unsigned key = kKeyHalo | (unsigned)(depth << 5) | (unsigned)h.n;
+    if (depth == 1)
+      launch_mapped(tg, s, key, grid_halo_one<1>, h.n, false, blk, k_halo_one<1, MapSingle>,
+                    k_halo_one<1, MapBatchFree>, h);
+    else
+      launch_mapped(tg, s, key, grid_halo_one<2>, h.n, false, blk, k_halo_one<2, MapSingle>,
+                    k_halo_one<2, MapBatchFree>, h);
+    return;
+  }
   // faces: 0 left, 1 right, 2 bottom, 3 top, 4 back, 5 front; axis order y, x, z
   const int axes[3] = {1, 0, 2};
   for (int ai = 0; ai < 3; ai++) {
@@ -1880,7 +2030,7 @@ void launch_fill(cudaStream_t s, T* p, long long elems, T value) {
                                               const S::cs_t*, const S::vel_t*, const S::vel_t*, \
                                               const S::vel_t*, double*, double*);              \
   template void launch_update_halo<S>(const Target&, cudaStream_t, const HaloFields&, const int*,  \
-                                      int, const int*);                                        \
+                                      int, const int*, bool, const HaloFields*);                \
   template void launch_generate_chunk<S>(const Geom&, cudaStream_t, const GeomArrays&,          \
                                          S::rho_t*, S::ene_t*, S::vel_t*, S::vel_t*,           \
                                          S::vel_t*, const StateTable&);

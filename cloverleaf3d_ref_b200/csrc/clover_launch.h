@@ -324,11 +324,19 @@ void launch_field_summary(const Geom& g, cudaStream_t s, const double* volume,
                           const typename S::vel_t* yvel0, const typename S::vel_t* zvel0,
                           double* partials, double* out5);
 
-// update_halo_kernel: fields[i] != 0 selects field id i+1; all faces external.
-// Element size of every selected field comes from the policy S.
+// update_halo_kernel: fields[i] != 0 selects field id i+1. Element size of
+// every selected field comes from the policy S. composed: every face is
+// external and every deck has three or more cells per axis from index 1
+// (halo_composes), so that one launch writes all faces, and the same halo into
+// also's arrays where they are given; otherwise one pass per axis, in the
+// reference's order, over the external faces.
+inline bool halo_composes(const Geom& g) {
+  return g.x_min == 1 && g.y_min == 1 && g.z_min == 1 && g.x_max >= 3 && g.y_max >= 3 && g.z_max >= 3;
+}
 template <class S>
 void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, const int* fields,
-                        int depth, const int* external_faces /*6: left..front*/);
+                        int depth, const int* external_faces /*6: left..front*/, bool composed,
+                        const HaloFields* also = nullptr);
 
 // initialise_chunk_kernel + generate_chunk_kernel on the device.
 struct StateTable {
@@ -400,7 +408,7 @@ void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const Geom
 // All three velocities of one sweep; vel_in/vel_out are the two buffers of
 // each velocity pair, and with copy_shell the shell outside [min,max+1]^3 is
 // copied across (left out where a depth-2 halo update of the velocities
-// comes before the next read of the shell).
+// comes before the next read of the shell, or has written it to both buffers).
 // vol: the uniform cell volume of the chunk (dx*dy*dz).
 // x_maps (one chunk, x sweep): the tensor maps of the sweep's inputs, to run
 // its shared-memory staged form (clover_tma.cu), which reports a copy that

@@ -313,10 +313,16 @@ struct Chunk : ChunkBase {
     return h;
   }
 
-  void halo(std::initializer_list<int> ids, int depth, int vb = 0, int cb = 0) {
+  // shell_vb: the time-level-1 velocities' halo goes to that buffer of their
+  // pairs too (one-launch updates only)
+  void halo(std::initializer_list<int> ids, int depth, int vb = 0, int cb = 0, int shell_vb = -1) {
     int fields[19] = {0};
     for (int id : ids) fields[id - 1] = 1;
-    launch_update_halo<S>(tg, stream, halo_fields(vb, cb), fields, depth, ext);
+    HaloFields also{};
+    if (shell_vb >= 0)
+      for (int c3 = 0; c3 < 3; c3++) also.f[8 + 2 * c3] = vel1(c3, shell_vb);
+    launch_update_halo<S>(tg, stream, halo_fields(vb, cb), fields, depth, ext, halo_repeat_free,
+                          shell_vb >= 0 ? &also : nullptr);
   }
 
   int deck_blocks() const { return (nd + 127) / 128; }
@@ -922,18 +928,19 @@ struct Chunk : ChunkBase {
         pend("advec_cell_yz", n * (nvf * VF8 + (2 + nl0) * (R8 + E8) + MF8));
       }
       pbeg();
-      // mass_flux_z changes only in the z sweep and is updated right after it
-      if (dir != 3 && halo_repeat_free) halo({2, 4, 9, 11, 13, 17, 18}, 2, vc, cb);
-      else halo({2, 4, 9, 11, 13, 17, 18, 19}, 2, vc, cb);
+      // mass_flux_z changes only in the z sweep and is updated right after it.
+      // After sweeps 1 and 2 the next post-sweep update rewrites the output
+      // velocities' shell before anything reads it; after sweep 3 the shell
+      // carries the step's final halo, which this update writes to both buffers
+      const int shell = sweep_number == 3 && halo_repeat_free ? vc ^ 1 : -1;
+      if (dir != 3 && halo_repeat_free) halo({2, 4, 9, 11, 13, 17, 18}, 2, vc, cb, shell);
+      else halo({2, 4, 9, 11, 13, 17, 18, 19}, 2, vc, cb, shell);
       pend("update_halo", 0);
       // post_vol reads two volume fluxes on sweep 1, one on sweep 2, none on sweep 3
       const double npv = sweep_number == 1 ? 2 : sweep_number == 2 ? 1 : 0;
       V* vin[3] = {vel1(0, vc), vel1(1, vc), vel1(2, vc)};
       V* vout[3] = {vel1(0, vc ^ 1), vel1(1, vc ^ 1), vel1(2, vc ^ 1)};
       pbeg();
-      // after sweeps 1 and 2 the next post-sweep depth-2 halo update rewrites
-      // the velocities' shell before anything reads it; after sweep 3 the
-      // shell carries the step's final halo values
       MomXMaps xm;
       NodeMaps nm;
       const bool x_tma = dir == 1 && tma && use_tma && mom_x_maps(rho1(cb), vin, &xm);
@@ -945,7 +952,7 @@ struct Chunk : ChunkBase {
       launch_advec_mom_fused<S>(tg, stream, axi, sweep_number, dir, cell_volume, ga, rho1(cb),
                                 mass_flux_x, mass_flux_y, mass_flux_z, vol_flux_x, vol_flux_y,
                                 vol_flux_z, work[0], work[1], work[2], vin, vout,
-                                sweep_number == 3 || !halo_repeat_free, l0,
+                                !halo_repeat_free, l0,
                                 x_tma ? &xm : nullptr, &sc->status, node_tma ? &nm : nullptr,
                                 vel_tma ? &vm : nullptr);
       // x: one pass; y, z: node pass + velocity pass
