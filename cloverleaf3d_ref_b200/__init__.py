@@ -150,6 +150,8 @@ def _declare(L):
     L.clover_chunk_dt_history.restype = ctypes.c_int
     L.clover_chunk_summaries.argtypes = [P, P, P, ctypes.c_int]
     L.clover_chunk_summaries.restype = ctypes.c_int
+    L.clover_chunk_summary_count.argtypes = [P]
+    L.clover_chunk_summary_count.restype = ctypes.c_int
     L.clover_chunk_read_field.argtypes = [P, ctypes.c_int, P]
     L.clover_chunk_read_field.restype = ctypes.c_int
     L.clover_chunk_write_field.argtypes = [P, ctypes.c_int, P]
@@ -390,6 +392,7 @@ class Chunk:
         return out[:got]
 
     def summaries(self, cap=100000):
+        cap = min(cap, lib().clover_chunk_summary_count(self.h))
         out = np.zeros((cap, 5))
         st = np.zeros(cap, dtype=np.int32)
         n = lib().clover_chunk_summaries(self.h, out.ctypes.data, st.ctypes.data, cap)
@@ -516,6 +519,7 @@ class Ensemble(Chunk):
         return out[:got]
 
     def deck_summaries(self, d, cap=100000):
+        cap = min(cap, lib().clover_chunk_summary_count(self.h))
         out = np.zeros((cap, 5))
         st = np.zeros(cap, dtype=np.int32)
         n = lib().clover_ensemble_summaries(self.h, d, out.ctypes.data, st.ctypes.data, cap)

@@ -106,6 +106,8 @@ int clover_chunk_steps(clover_chunk *c);
 double clover_chunk_time(clover_chunk *c);
 int clover_chunk_dt_history(clover_chunk *c, double *out, int cap);
 int clover_chunk_summaries(clover_chunk *c, double *out5, int *steps, int cap);
+/* Number of recorded field summaries (does not synchronise). */
+int clover_chunk_summary_count(clover_chunk *c);
 /* Device status bits (CLOVER_STATUS_* of clover_kernels.h). */
 int clover_chunk_status(clover_chunk *c);
 
