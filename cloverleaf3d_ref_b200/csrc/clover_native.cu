@@ -867,29 +867,51 @@ struct Chunk : ChunkBase {
     pend("update_halo", 0);
     pbeg();
     AccMaps acc_m;
-    if (tma && use_tma && tmap(density0, sizeof(R), 9, &acc_m.d) &&
-        tmap(pressure, sizeof(C), 9, &acc_m.p) && tmap(viscosity, sizeof(C), 9, &acc_m.q) &&
-        tmap(xvel0, sizeof(V), 8, &acc_m.u) && tmap(yvel0, sizeof(V), 8, &acc_m.v) &&
-        tmap(zvel0, sizeof(V), 8, &acc_m.w))
-      launch_accelerate_tma<S>(g, stream, dtp, acc_m, vel1(0, vc), vel1(1, vc), vel1(2, vc),
-                               &sc->status);
-    else
-      launch_accelerate<S>(tg, stream, 0.0, dtp, ga, density0, pressure, viscosity, xvel0, yvel0,
-                           zvel0, vel1(0, vc), vel1(1, vc), vel1(2, vc), true);
-    pend("accelerate", n * (R8 + 2 * C8 + 6 * V8));
-    pbeg();
-    FluxMaps flux_m;
-    if (tma && use_tma && tmap(xvel0, sizeof(V), 9, &flux_m.u0) &&
-        tmap(yvel0, sizeof(V), 9, &flux_m.v0) && tmap(zvel0, sizeof(V), 9, &flux_m.w0) &&
-        tmap(vel1(0, vc), sizeof(V), 9, &flux_m.u1) && tmap(vel1(1, vc), sizeof(V), 9, &flux_m.v1) &&
-        tmap(vel1(2, vc), sizeof(V), 9, &flux_m.w1))
-      launch_pdv_flux_tma<S>(g, stream, dtp, flux_m, density0, rho1(cb), energy0, ene1(cb),
-                             pressure, viscosity, vol_flux_x, vol_flux_y, vol_flux_z, &sc->status);
-    else
-      launch_pdv_flux<S>(tg, stream, dtp, ga, density0, rho1(cb), energy0, ene1(cb), pressure,
-                         viscosity, xvel0, vel1(0, vc), yvel0, vel1(1, vc), zvel0, vel1(2, vc),
-                         vol_flux_x, vol_flux_y, vol_flux_z);
-    pend("pdv_flux", n * (2 * R8 + 2 * E8 + 2 * C8 + 6 * V8 + 3 * VF8));
+    const bool acc_tma = tma && use_tma && tmap(density0, sizeof(R), 9, &acc_m.d) &&
+                         tmap(pressure, sizeof(C), 9, &acc_m.p) &&
+                         tmap(viscosity, sizeof(C), 9, &acc_m.q) && tmap(xvel0, sizeof(V), 8, &acc_m.u) &&
+                         tmap(yvel0, sizeof(V), 8, &acc_m.v) && tmap(zvel0, sizeof(V), 8, &acc_m.w);
+    bool fused_flux = false;
+    if constexpr (kFusedAccFlux<S>) {
+      fused_flux = acc_tma;
+      if (fused_flux) {
+        launch_acc_flux_tma<S>(g, stream, dtp, acc_m, rho1(cb), energy0, ene1(cb), vel1(0, vc),
+                               vel1(1, vc), vel1(2, vc), vol_flux_x, vol_flux_y, vol_flux_z, &sc->status);
+        pend("accelerate_pdv_flux", n * (2 * R8 + 2 * E8 + 2 * C8 + 6 * V8 + 3 * VF8));
+      }
+    }
+    if (!fused_flux) {
+      bool staged = false;
+      if constexpr (!kFusedAccFlux<S>) {
+        staged = acc_tma;
+        if (staged)
+          launch_accelerate_tma<S>(g, stream, dtp, acc_m, vel1(0, vc), vel1(1, vc), vel1(2, vc),
+                                   &sc->status);
+      }
+      if (!staged)
+        launch_accelerate<S>(tg, stream, 0.0, dtp, ga, density0, pressure, viscosity, xvel0, yvel0,
+                             zvel0, vel1(0, vc), vel1(1, vc), vel1(2, vc), true);
+      pend("accelerate", n * (R8 + 2 * C8 + 6 * V8));
+      pbeg();
+      staged = false;
+      if constexpr (!kFusedAccFlux<S>) {
+        FluxMaps flux_m;
+        staged = tma && use_tma && tmap(xvel0, sizeof(V), 9, &flux_m.u0) &&
+                 tmap(yvel0, sizeof(V), 9, &flux_m.v0) && tmap(zvel0, sizeof(V), 9, &flux_m.w0) &&
+                 tmap(vel1(0, vc), sizeof(V), 9, &flux_m.u1) &&
+                 tmap(vel1(1, vc), sizeof(V), 9, &flux_m.v1) &&
+                 tmap(vel1(2, vc), sizeof(V), 9, &flux_m.w1);
+        if (staged)
+          launch_pdv_flux_tma<S>(g, stream, dtp, flux_m, density0, rho1(cb), energy0, ene1(cb),
+                                 pressure, viscosity, vol_flux_x, vol_flux_y, vol_flux_z,
+                                 &sc->status);
+      }
+      if (!staged)
+        launch_pdv_flux<S>(tg, stream, dtp, ga, density0, rho1(cb), energy0, ene1(cb), pressure,
+                           viscosity, xvel0, vel1(0, vc), yvel0, vel1(1, vc), zvel0, vel1(2, vc),
+                           vol_flux_x, vol_flux_y, vol_flux_z);
+      pend("pdv_flux", n * (2 * R8 + 2 * E8 + 2 * C8 + 6 * V8 + 3 * VF8));
+    }
     // advection.f90:43-179. The last sweep also writes time level 0 (the
     // interior density/energy and node velocities reset_field copies), so
     // reset_field needs no pass of its own.

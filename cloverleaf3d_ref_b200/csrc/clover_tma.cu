@@ -674,7 +674,7 @@ k_pdv_predict_eos_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
 
 // ---------------------------------------------------------------------------
 // accelerate_kernel.f90:61-109 on the uniform mesh, as k_accelerate
-// (clover_kernels.cu) forms it. Plane p: density0, pressure and viscosity of
+// (clover_kernels.cu) forms it; the mixed policy's step. Plane p: density0, pressure and viscosity of
 // cell plane p (rows k0-1..k0+7) and the three node velocities of node plane
 // p (rows k0..k0+7). Node l reads cell planes l-1, l and node plane l.
 template <class S>
@@ -921,6 +921,268 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     energy1[o] = st<typename S::ene_t>(((A)e0_s - energy_change));
     density1[o] = st<typename S::rho_t>(d0 * vol_change_s);
   });
+}
+
+// ---------------------------------------------------------------------------
+// accelerate_kernel.f90:61-109, then PdV_kernel.f90:120-166 (corrector) and
+// flux_calc_kernel.f90:58-91 on the velocities just formed, operation for
+// operation as k_accelerate (clover_kernels.cu) and k_pdv_flux
+// (clover_fused.cu). Plane p: density0, pressure and viscosity of cell plane p
+// (rows k0-1..k0+TYN-1) and the three time-level-0 velocities of node plane p
+// (rows k0..). A block's 32 x TYN threads form the new velocities of node
+// plane l+1 into one of two planes in shared memory (and store the nodes the
+// block owns, 31 x (TYN-1) of segment planes), then the corrector, the face
+// fluxes and their sums of index plane l from node planes l and l+1. The last
+// lane, the last row and one plane per segment are formed twice, by the block
+// that owns them and by its neighbour.
+//
+// The FP64 step's form: the separate kernels move 192 B per cell, this one 120
+// B (the new velocities are not read back, density0, pressure, viscosity and
+// the old velocities are read once), 4.63 -> 4.22 ms at 512^3. It is not bound
+// by HBM any more (2.6 ms): three blocks per SM wait on shared memory, two
+// barriers a plane and FP64 issue. Taller blocks (12 rows, two per SM: 4.39 ms)
+// and two blocks per SM (6.1 ms) lose more warps than they save. The mixed
+// policy keeps the separate kernels: its 136 B per cell fall to 68 B, but its
+// FP32 arithmetic issues longer fused (2.77 -> 2.91 ms).
+template <class S, int TYN>
+struct AccFluxPlane {
+  using V = typename S::vel_t;
+  using R = typename S::rho_t;
+  using C = typename S::cs_t;
+  static constexpr int kRho = round128((TYN + 1) * kTmaWidth<R> * (int)sizeof(R));
+  static constexpr int kCs = round128((TYN + 1) * kTmaWidth<C> * (int)sizeof(C));
+  static constexpr int kVel = round128(TYN * kTmaWidth<V> * (int)sizeof(V));
+  static constexpr int kBytes = kRho + 2 * kCs + 3 * kVel;
+  static constexpr int kNew = 3 * TYN * TX * (int)sizeof(V);  // one plane of new velocities
+  static constexpr unsigned kTx = box_bytes<R>(TYN + 1) + 2 * box_bytes<C>(TYN + 1) + 3 * box_bytes<V>(TYN);
+  __device__ static R* rho(unsigned char* p) { return (R*)p; }
+  __device__ static C* cs(unsigned char* p, int q) { return (C*)(p + kRho + q * kCs); }
+  __device__ static V* vel(unsigned char* p, int q) { return (V*)(p + kRho + 2 * kCs + q * kVel); }
+};
+
+// Box x coordinate for a block whose first wanted column is x_min + d + 31 t,
+// and that column's place in the box.
+template <class T>
+__device__ __forceinline__ void x_box31(int t, int d, int& x, int& shift) {
+  constexpr int H = kTmaHalo<T>;
+  const int c = 31 * t + H + d;
+  x = c / H * H;
+  shift = c - x;
+}
+
+template <class S, int TYN, int RING, int MINB>
+__global__ void __launch_bounds__(TX * TYN, MINB)
+k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_constant__ AccMaps maps,
+               typename S::rho_t* __restrict__ density1, const typename S::ene_t* __restrict__ energy0,
+               typename S::ene_t* __restrict__ energy1, typename S::vel_t* __restrict__ xvel1,
+               typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1,
+               typename S::vf_t* __restrict__ vol_flux_x, typename S::vf_t* __restrict__ vol_flux_y,
+               typename S::vf_t* __restrict__ vol_flux_z, int* __restrict__ status) {
+  using P = AccFluxPlane<S, TYN>;
+  using A = typename S::arith_t;
+  using V = typename S::vel_t;
+  using R = typename S::rho_t;
+  using C = typename S::cs_t;
+  using En = typename S::ene_t;
+  using F = typename S::vf_t;
+  extern __shared__ __align__(128) unsigned char ring[];
+  __shared__ unsigned long long full[RING];
+  V* const fresh = (V*)(ring + RING * P::kBytes);  // new velocities of node planes of both parities
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
+  const int j = g.x_min + 31 * (int)blockIdx.x + tx, k0 = g.y_min + (TYN - 1) * (int)blockIdx.y;
+  const int k = k0 + ty;
+  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int l1 = l0 + seg - 1 < g.z_max + 1 ? l0 + seg - 1 : g.z_max + 1;
+  const int pfirst = l0 - 1, plast = l1 + 1 < g.z_max + 1 ? l1 + 1 : g.z_max + 1;
+  const bool in_node = j <= g.x_max + 1 && k <= g.y_max + 1;
+  const bool own = in_node && tx < TX - 1 && ty < TYN - 1;
+  const bool jin = j <= g.x_max, kin = k <= g.y_max;
+  const double dt = dt_ptr[0];
+  constexpr int WV = kTmaWidth<V>, WR = kTmaWidth<R>, WC = kTmaWidth<C>;
+  int xr, cr, xc, cc, xv, cv;
+  x_box31<R>(blockIdx.x, -1, xr, cr);
+  x_box31<C>(blockIdx.x, -1, xc, cc);
+  x_box31<V>(blockIdx.x, 0, xv, cv);
+  // this thread's cell (j, k) and node (j, k) in the boxes
+  cr += (ty + 1) * WR + tx + 1;
+  cc += (ty + 1) * WC + tx + 1;
+  cv += ty * WV + tx;
+  if (tid == 0) {
+    for (int r = 0; r < RING; r++) mbar_init(&full[r], 1);
+    mbar_init_fence();
+  }
+  __syncthreads();
+  int issued_hi = pfirst - 1;
+  auto buf = [&](int p) { return ring + ((p - pfirst) % RING) * P::kBytes; };
+  auto issue = [&](int p) {
+    issued_hi = p;
+    unsigned char* b = buf(p);
+    unsigned long long* bar = &full[(p - pfirst) % RING];
+    mbar_arrive_expect_tx(bar, P::kTx);
+    const int y1 = k0 - g.y_min + 1, z = p - g.z_min + 2;
+    tma_load_box(P::rho(b), &maps.d, bar, xr, y1, z);
+    tma_load_box(P::cs(b, 0), &maps.p, bar, xc, y1, z);
+    tma_load_box(P::cs(b, 1), &maps.q, bar, xc, y1, z);
+    tma_load_box(P::vel(b, 0), &maps.u, bar, xv, y1 + 1, z);
+    tma_load_box(P::vel(b, 1), &maps.v, bar, xv, y1 + 1, z);
+    tma_load_box(P::vel(b, 2), &maps.w, bar, xv, y1 + 1, z);
+  };
+  auto wait = [&](int p) {
+    const int u = p - pfirst;
+    return mbar_wait_bounded(&full[u % RING], (unsigned)(u / RING) & 1u);
+  };
+  if (tid == 0)
+    for (int p = pfirst; p <= plast && p < pfirst + RING; p++) issue(p);
+  // the cell's own energy0, loaded one plane ahead
+  En c_e = En(0);
+  auto fetch = [&](int l) {
+    if (own && jin && kin && l >= l0 && l <= l1 && l <= g.z_max) c_e = __ldg(&energy0[off3(g, j, k, l)]);
+  };
+  fetch(l0);
+  bool late = !wait(pfirst);
+  // the z face sum of node plane l (zvel0 x4 then zvel1 x4), carried; the rest
+  // of a plane is read again from shared memory when the plane above comes
+  // (28 more carried values took the kernel to two blocks per SM, 4.2 -> 6.1
+  // ms at 512^3 FP64)
+  double zs = 0.0;
+  // the masses, pressures and viscosities of the plane's cells around the node,
+  // in the order (-1,-1), (0,-1), (0,0), (-1,0)
+  auto cells = [&](unsigned char* b, double (&m)[4], A (&pr)[4], A (&qv)[4]) {
+    const R* d = P::rho(b) + cr;
+    const C* pp = P::cs(b, 0) + cc;
+    const C* qq = P::cs(b, 1) + cc;
+    m[0] = (double)d[-WR - 1] * g.vol; m[1] = (double)d[-WR] * g.vol;
+    m[2] = (double)d[0] * g.vol; m[3] = (double)d[-1] * g.vol;
+    pr[0] = (A)pp[-WC - 1]; pr[1] = (A)pp[-WC]; pr[2] = (A)pp[0]; pr[3] = (A)pp[-1];
+    qv[0] = (A)qq[-WC - 1]; qv[1] = (A)qq[-WC]; qv[2] = (A)qq[0]; qv[3] = (A)qq[-1];
+  };
+  int l = l0 - 1;
+  for (; l <= l1; l++) {
+    unsigned char* bl = buf(l);
+    unsigned char* bu = buf(l + 1);
+    V* const n0 = fresh + (l & 1) * (P::kNew / (int)sizeof(V));
+    V* const n1 = fresh + ((l + 1) & 1) * (P::kNew / (int)sizeof(V));
+    const bool more = l <= g.z_max;  // node plane l+1 exists
+    if (more && !late) late = !wait(l + 1);
+    V un = V(0), vn = V(0), wn = V(0);
+    if (more && in_node && !late) {
+      // accelerate at node (j, k, l+1): cell planes l+1 (upper) and l (lower)
+      double um[4], lm[4];
+      A up[4], uq[4], lp[4], lq[4];
+      cells(bu, um, up, uq);
+      cells(bl, lm, lp, lq);
+      const double nodal_mass =
+          (um[0] + um[1] + um[2] + um[3] + lm[0] + lm[1] + lm[2] + lm[3]) * 0.125;
+      const A sm = (A)(0.25 * dt / nodal_mass);
+      const A xa = (A)g.xa, ya = (A)g.ya, za = (A)g.za;
+      // the gradient sums of values a (upper plane) and b (lower): index 0 (-1,-1), 1 (0,-1), 2 (0,0), 3 (-1,0)
+      auto gx = [&](const A (&a)[4], const A (&b)[4]) {
+        return sm * (xa * (a[2] - a[3]) + xa * (a[1] - a[0]) + xa * (b[2] - b[3]) + xa * (b[1] - b[0]));
+      };
+      auto gy = [&](const A (&a)[4], const A (&b)[4]) {
+        return sm * (ya * (a[2] - a[1]) + ya * (a[3] - a[0]) + ya * (b[2] - b[1]) + ya * (b[3] - b[0]));
+      };
+      auto gz = [&](const A (&a)[4], const A (&b)[4]) {
+        return sm * (za * (a[2] - b[2]) + za * (a[1] - b[1]) + za * (a[3] - b[3]) + za * (a[0] - b[0]));
+      };
+      un = st<V>((A)P::vel(bu, 0)[cv] - gx(up, lp) - gx(uq, lq));
+      vn = st<V>((A)P::vel(bu, 1)[cv] - gy(up, lp) - gy(uq, lq));
+      wn = st<V>((A)P::vel(bu, 2)[cv] - gz(up, lp) - gz(uq, lq));
+      n1[tid] = un;
+      n1[TYN * TX + tid] = vn;
+      n1[2 * TYN * TX + tid] = wn;
+      if (own && l + 1 >= l0 && l + 1 <= l1) {
+        const long long o = off3(g, j, k, l + 1);
+        xvel1[o] = un;
+        yvel1[o] = vn;
+        zvel1[o] = wn;
+      }
+    }
+    if (__syncthreads_or(late)) break;
+    if (own) {
+      // velocity q of node (j+a, k+b): time level 0 of buffer bb, level 1 of plane nn
+#define N0(bb, q, a, b) ((A)P::vel(bb, q)[cv + (b) * WV + (a)])
+#define N1(nn, q, a, b) ((A)nn[(q) * TYN * TX + tid + (b) * TX + (a)])
+      // node plane l+1: its z face flux (the plane the segment owns) and sum
+      double zsu = 0.0;
+      if (more && jin && kin) {
+        const A a0 = N0(bu, 2, 0, 0), a1 = N0(bu, 2, 1, 0), a2 = N0(bu, 2, 0, 1), a3 = N0(bu, 2, 1, 1);
+        const A b0 = (A)wn, b1 = N1(n1, 2, 1, 0), b2 = N1(n1, 2, 0, 1), b3 = N1(n1, 2, 1, 1);
+        zsu = (double)(a0 + a1 + a2 + a3 + b0 + b1 + b2 + b3);
+        // flux_calc_kernel.f90:86 repeats zvel0(j+1,k,l) and omits zvel0(j,k+1,l)
+        const double bz = (double)(a0 + a1 + a1 + a3 + b0 + b1 + b2 + b3);
+        if (l + 1 >= l0 && l + 1 <= l1) vol_flux_z[off3(g, j, k, l + 1)] = st<F>(0.125 * dt * g.za * bz);
+      }
+      if (l >= l0 && more) {
+        auto xsum = [&](int a) {
+          return (double)(N0(bl, 0, a, 0) + N0(bl, 0, a, 1) + N0(bu, 0, a, 0) + N0(bu, 0, a, 1) +
+                          N1(n0, 0, a, 0) + N1(n0, 0, a, 1) + N1(n1, 0, a, 0) + N1(n1, 0, a, 1));
+        };
+        auto ysum = [&](int b) {
+          return (double)(N0(bl, 1, 0, b) + N0(bl, 1, 1, b) + N0(bu, 1, 0, b) + N0(bu, 1, 1, b) +
+                          N1(n0, 1, 0, b) + N1(n0, 1, 1, b) + N1(n1, 1, 0, b) + N1(n1, 1, 1, b));
+        };
+        const long long o = off3(g, j, k, l);
+        double sx = 0, sy = 0;
+        F vfx0 = F(0), vfy0 = F(0);
+        if (kin) {
+          sx = xsum(0);
+          vfx0 = st<F>(0.125 * dt * g.xa * sx);
+          vol_flux_x[o] = vfx0;
+        }
+        if (jin) {
+          sy = ysum(0);
+          vfy0 = st<F>(0.125 * dt * g.ya * sy);
+          vol_flux_y[o] = vfy0;
+        }
+        if (jin && kin) {
+          const En e0_s = c_e;
+          fetch(l + 1);
+          double left_flux, right_flux, bottom_flux, top_flux, back_flux, front_flux;
+          if (sizeof(F) == 8) {  // PdV_kernel.f90:120-131 order
+            left_flux = (g.xa * sx) * 0.125 * dt;
+            right_flux = (g.xa * xsum(1)) * 0.125 * dt;
+            bottom_flux = (g.ya * sy) * 0.125 * dt;
+            top_flux = (g.ya * ysum(1)) * 0.125 * dt;
+            back_flux = (g.za * zs) * 0.125 * dt;
+            front_flux = (g.za * zsu) * 0.125 * dt;
+          } else {
+            // FP32 volume fluxes: the corrector's face fluxes as the volume
+            // fluxes are stored (the z faces from the corrector's own node sums)
+            auto stored = [&](double area, double s) { return (double)st<F>(0.125 * dt * area * s); };
+            left_flux = (double)vfx0;
+            right_flux = stored(g.xa, xsum(1));
+            bottom_flux = (double)vfy0;
+            top_flux = stored(g.ya, ysum(1));
+            back_flux = stored(g.za, zs);
+            front_flux = stored(g.za, zsu);
+          }
+          const double total_flux =
+              right_flux - left_flux + top_flux - bottom_flux + front_flux - back_flux;
+          const double vol = g.vol;
+          const double vol_change_s = vol / (vol + total_flux);
+          const double d0 = (double)P::rho(bl)[cr];
+          const A ad0 = (A)d0;
+          const A energy_change = ((A)P::cs(bl, 0)[cc] / ad0 + (A)P::cs(bl, 1)[cc] / ad0) *
+                                  (A)total_flux * geo_rvol<A>(g);
+          energy1[o] = st<En>(((A)e0_s - energy_change));
+          density1[o] = st<R>(d0 * vol_change_s);
+        }
+      }
+      zs = zsu;
+#undef N1
+#undef N0
+    }
+    // every thread is done with plane l and with the new velocities of parity l
+    __syncthreads();
+    if (tid == 0 && l + RING <= plast) issue(l + RING);
+  }
+  if (l <= l1 && tid == 0) {
+    // a plane's copies did not arrive in time: report it, and give the copies
+    // still in flight a bounded wait before the shared memory is released
+    atomicOr(status, CLOVER_STATUS_TIMEOUT);
+    for (int p = l + 1; p <= issued_hi; p++) wait(p);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2324,17 +2586,27 @@ constexpr int kStencilRing = 4;
 template <class S>
 constexpr int kStencilMinBlocks = sizeof(typename S::arith_t) == 4 ? 4 : 3;
 
+// shared memory of the accelerate + corrector + flux kernel
+template <class S>
+constexpr int kAccFluxSmem = kStencilRing * AccFluxPlane<S, TY>::kBytes +
+                             2 * AccFluxPlane<S, TY>::kNew;
+
 template <class S>
 bool stencils_tma_prepare() {
-  return cudaFuncSetAttribute(k_pdv_predict_eos_tma<S, kStencilRing, kStencilMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kStencilRing * PdvPlane<S>::kBytes) == cudaSuccess &&
-         cudaFuncSetAttribute(k_accelerate_tma<S, kStencilRing, kStencilMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kStencilRing * AccPlane<S>::kBytes) == cudaSuccess &&
-         cudaFuncSetAttribute(k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kStencilRing * FluxPlane<S>::kBytes) == cudaSuccess;
+  if (cudaFuncSetAttribute(k_pdv_predict_eos_tma<S, kStencilRing, kStencilMinBlocks<S>>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kStencilRing * PdvPlane<S>::kBytes) != cudaSuccess)
+    return false;
+  if constexpr (kFusedAccFlux<S>)
+    return cudaFuncSetAttribute(k_acc_flux_tma<S, TY, kStencilRing, 3>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, kAccFluxSmem<S>) == cudaSuccess;
+  else
+    return cudaFuncSetAttribute(k_accelerate_tma<S, kStencilRing, kStencilMinBlocks<S>>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kStencilRing * AccPlane<S>::kBytes) == cudaSuccess &&
+           cudaFuncSetAttribute(k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kStencilRing * FluxPlane<S>::kBytes) == cudaSuccess;
 }
 
 // blocks per SM of the drop-in PdV: the corrector's plane (six velocity
@@ -2531,6 +2803,22 @@ void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, co
 }
 
 template <class S>
+void launch_acc_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
+                         typename S::rho_t* density1, const typename S::ene_t* energy0,
+                         typename S::ene_t* energy1, typename S::vel_t* xvel1,
+                         typename S::vel_t* yvel1, typename S::vel_t* zvel1,
+                         typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
+                         typename S::vf_t* vol_flux_z, int* status) {
+  int seg;
+  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX - 1) / (TX - 1),
+                               (g.y_max + 1 - g.y_min + TY - 1) / (TY - 1), g.z_max - g.z_min + 2, &seg);
+  k_acc_flux_tma<S, TY, kStencilRing, 3>
+      <<<grid, dim3(TX, TY), kAccFluxSmem<S>, s>>>(g, seg, dt_ptr, maps, density1, energy0, energy1,
+                                                     xvel1, yvel1, zvel1, vol_flux_x, vol_flux_y,
+                                                     vol_flux_z, status);
+}
+
+template <class S>
 constexpr int kNodeMinBlocks = sizeof(typename S::arith_t) == 4 ? 5 : 5;
 
 template <class S>
@@ -2670,12 +2958,6 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                                            const Level0<S>&, int*);                              \
   template void launch_pdv_predict_eos_tma<S>(const Geom&, cudaStream_t, const double*,         \
                                               const PdvMaps&, S::cs_t*, int*);                   \
-  template void launch_accelerate_tma<S>(const Geom&, cudaStream_t, const double*,               \
-                                         const AccMaps&, S::vel_t*, S::vel_t*, S::vel_t*, int*); \
-  template void launch_pdv_flux_tma<S>(const Geom&, cudaStream_t, const double*, const FluxMaps&, \
-                                       const S::rho_t*, S::rho_t*, const S::ene_t*, S::ene_t*,   \
-                                       const S::cs_t*, const S::cs_t*, S::vf_t*, S::vf_t*,       \
-                                       S::vf_t*, int*);                                          \
   template void launch_mom_x_tma<S>(const Geom&, cudaStream_t, int, const MomXMaps&,             \
                                     const GeomArrays&, S::vel_t* const*, const Level0<S>&, int*); \
   template void launch_visc_dt_tma<S>(const Geom&, cudaStream_t, const ViscMaps&, const GeomArrays&, \
@@ -2683,6 +2965,15 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                                       S::cs_t*, S::cs_t*, unsigned long long*, int*);
 INST_TMA(F64)
 INST_TMA(F32Mixed)
+template void launch_acc_flux_tma<F64>(const Geom&, cudaStream_t, const double*, const AccMaps&, 
+                                       F64::rho_t*, const F64::ene_t*, F64::ene_t*, F64::vel_t*,         
+                                       F64::vel_t*, F64::vel_t*, F64::vf_t*, F64::vf_t*, F64::vf_t*, int*);
+template void launch_accelerate_tma<F32Mixed>(const Geom&, cudaStream_t, const double*,               
+                                         const AccMaps&, F32Mixed::vel_t*, F32Mixed::vel_t*, F32Mixed::vel_t*, int*); 
+template void launch_pdv_flux_tma<F32Mixed>(const Geom&, cudaStream_t, const double*, const FluxMaps&, 
+                                       const F32Mixed::rho_t*, F32Mixed::rho_t*, const F32Mixed::ene_t*, F32Mixed::ene_t*,   
+                                       const F32Mixed::cs_t*, const F32Mixed::cs_t*, F32Mixed::vf_t*, F32Mixed::vf_t*,       
+                                       F32Mixed::vf_t*, int*);                                          
 
 void launch_wait_selftest(cudaStream_t s, long long cycles, int* status) {
   k_wait_selftest<<<1, 32, 0, s>>>(cycles, status);

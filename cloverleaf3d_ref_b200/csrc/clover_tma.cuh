@@ -60,11 +60,11 @@ void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& 
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
                       const Level0<S>& level0, int* status);
 
-// The maps of the one-cell-per-thread stencils: the PdV predictor + EOS
-// (node velocities 9 rows, density0, energy0, pressure, viscosity 8 rows),
-// accelerate (density0, pressure, viscosity 9 rows from k0-1, node
-// velocities 8 rows) and the PdV corrector + flux_calc (time level 0 and 1
-// velocities, 9 rows).
+// The maps of the PdV predictor + EOS (node velocities 9 rows, density0,
+// energy0, pressure, viscosity 8 rows), of accelerate, alone or with the
+// corrector and flux_calc (density0, pressure, viscosity 9 rows from k0-1, time
+// level 0 node velocities 8 rows), and of the PdV corrector + flux_calc (time
+// level 0 and 1 velocities, 9 rows).
 struct PdvMaps {
   CUtensorMap u, v, w, d, e, p, q;
 };
@@ -74,6 +74,10 @@ struct AccMaps {
 struct FluxMaps {
   CUtensorMap u0, v0, w0, u1, v1, w1;
 };
+// Whether the step runs accelerate, corrector and flux_calc as one staged
+// kernel (measured faster in FP64 only).
+template <class S>
+constexpr bool kFusedAccFlux = sizeof(typename S::arith_t) == 8;
 template <class S>
 bool stencils_tma_prepare();
 template <class S>
@@ -88,6 +92,13 @@ void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, co
                          const typename S::rho_t* density0, typename S::rho_t* density1,
                          const typename S::ene_t* energy0, typename S::ene_t* energy1,
                          const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
+                         typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
+                         typename S::vf_t* vol_flux_z, int* status);
+template <class S>
+void launch_acc_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
+                         typename S::rho_t* density1, const typename S::ene_t* energy0,
+                         typename S::ene_t* energy1, typename S::vel_t* xvel1,
+                         typename S::vel_t* yvel1, typename S::vel_t* zvel1,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
                          typename S::vf_t* vol_flux_z, int* status);
 
