@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
     typename S::cs_t* __restrict__ pressure, typename S::cs_t* __restrict__ viscosity,
     typename S::cs_t* __restrict__ soundspeed,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
-    const typename S::vel_t* __restrict__ zvel0, unsigned long long* __restrict__ min_key) {
+    const typename S::vel_t* __restrict__ zvel0, unsigned long long* __restrict__ min_key, bool xh) {
   __shared__ unsigned long long wmin[BX * BY / 32];
   m.run([&](const Geom& g, const Tile& t) {
   // viscosity and dt criteria in the policy's arithmetic (FP64, or FP32 in
@@ -194,7 +194,10 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
     using C = typename S::cs_t;
 #define PN(jj, kk, ll) \
   ((A)st<C>(((A(1.4) - A(1.0)) * LA(density0, jj, kk, ll) * LA(energy0, jj, kk, ll))))
-    A pgradx = (PN(j + 1, k, l) - PN(j - 1, k, l)) / (cdx + AG(GX, ga.celldx, j + 1));
+    // with xh the x-face halo of density0 and energy0 is written below: a
+    // cell at the face takes its own value, which that halo mirrors
+    const int jm = xh && j == g.x_min ? j : j - 1, jp = xh && j == g.x_max ? j : j + 1;
+    A pgradx = (PN(jp, k, l) - PN(jm, k, l)) / (cdx + AG(GX, ga.celldx, j + 1));
     A pgrady = (PN(j, k + 1, l) - PN(j, k - 1, l)) / (cdy + AG(GY, ga.celldy, k + 1));
     A pgradz = (PN(j, k, l + 1) - PN(j, k, l - 1)) / (cdz + AG(GZ, ga.celldz, l + 1));
 #undef PN
@@ -219,6 +222,12 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
   }
   using C = typename S::cs_t;
   E(viscosity, j, k, l) = st<C>(q);
+  if (xh && xh_edge(j, g.x_max)) {
+    const long long o = off3(g, j, k, l);
+    xh_cell<1>(viscosity, o, j, g.x_max, st<C>(q));
+    xh_cell<1>(const_cast<typename S::rho_t*>(density0), o, j, g.x_max, __ldg(density0 + o));
+    xh_cell<1>(const_cast<typename S::ene_t*>(energy0), o, j, g.x_max, __ldg(energy0 + o));
+  }
   // calc_dt_kernel.f90:102-149 (the viscosity as stored)
   const A visc = (A)st<C>(q);
   const A d0 = LA(density0, j, k, l);
@@ -292,7 +301,7 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 6 : 8) k_pdv_predict_eos(M
     GeomArrays ga, const typename S::rho_t* __restrict__ density0,
     const typename S::ene_t* __restrict__ energy0, typename S::cs_t* __restrict__ pressure,
     const typename S::cs_t* __restrict__ viscosity, const typename S::vel_t* __restrict__ xvel0,
-    const typename S::vel_t* __restrict__ yvel0, const typename S::vel_t* __restrict__ zvel0) {
+    const typename S::vel_t* __restrict__ yvel0, const typename S::vel_t* __restrict__ zvel0, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
   const Box b = interior(g);
   int j, k;
@@ -342,7 +351,9 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 6 : 8) k_pdv_predict_eos(M
   // the predicted state goes through the storage types, as it would in memory
   const A e1 = (A)st<En>((LA(energy0, j, k, l) - energy_change));
   const A d1 = (A)st<R>((d0 * vol_change_s));
-  E(pressure, j, k, l) = st<typename S::cs_t>(((A(1.4) - A(1.0)) * d1 * e1));
+  const typename S::cs_t pn = st<typename S::cs_t>(((A(1.4) - A(1.0)) * d1 * e1));
+  E(pressure, j, k, l) = pn;
+  if (xh) xh_cell<1>(pressure, off3(g, j, k, l), j, g.x_max, pn);
 #undef EGA
 #undef LA
   });
@@ -361,7 +372,7 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
     const typename S::vel_t* __restrict__ xvel1, const typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ yvel1, const typename S::vel_t* __restrict__ zvel0,
     const typename S::vel_t* __restrict__ zvel1, typename S::vf_t* __restrict__ vol_flux_x,
-    typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z) {
+    typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
   const Box b = nodes(g);
   int j, k;
@@ -369,6 +380,8 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
   const int l = b.l0 + t.z;
   const double dt = dt_ptr[(long long)t.d * kScalarStride];
   const bool jin = j <= g.x_max, kin = k <= g.y_max, lin = l <= g.z_max;
+  const bool xe = xh && xh_edge(j, g.x_max);
+  const long long o = off3(g, j, k, l);
   using F = typename S::vf_t;
   // face sums of the node velocities, reference order (vel0 x4 then vel1 x4),
   // in the policy's arithmetic: FP64, or in the mixed path the FP32 sum of
@@ -397,12 +410,14 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
   if (kin && lin) {
     sx = xsum(j);
     vfx0 = st<F>(0.125 * dt * g.xa * sx);
-    E(vol_flux_x, j, k, l) = vfx0;
+    vol_flux_x[o] = vfx0;
+    if (xe) xh_node<2>(vol_flux_x, o, j, g.x_max, -vfx0);
   }
   if (jin && lin) {
     sy = ysum(k);
     vfy0 = st<F>(0.125 * dt * g.ya * sy);
-    E(vol_flux_y, j, k, l) = vfy0;
+    vol_flux_y[o] = vfy0;
+    if (xe) xh_face<2>(vol_flux_y, o, j, g.x_max, vfy0);
   }
   if (jin && kin) {
     // flux_calc_kernel.f90:86 repeats zvel0(j+1,k,l) and omits zvel0(j,k+1,l)
@@ -410,7 +425,9 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
                                LA(zvel0, j + 1, k, l) + LA(zvel0, j + 1, k + 1, l) +
                                LA(zvel1, j, k, l) + LA(zvel1, j + 1, k, l) +
                                LA(zvel1, j, k + 1, l) + LA(zvel1, j + 1, k + 1, l));
-    E(vol_flux_z, j, k, l) = st<F>(0.125 * dt * g.za * bz);
+    const F vfz0 = st<F>(0.125 * dt * g.za * bz);
+    vol_flux_z[o] = vfz0;
+    if (xe) xh_face<2>(vol_flux_z, o, j, g.x_max, vfz0);
     sz = zsum(l);
   }
   if (!(jin && kin && lin)) return;
@@ -444,8 +461,14 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
   const A ad0 = (A)d0;
   const A energy_change = (LA(pressure, j, k, l) / ad0 + LA(viscosity, j, k, l) / ad0) *
                           (A)total_flux * geo_rvol<A>(g);
-  E(energy1, j, k, l) = st<typename S::ene_t>((LA(energy0, j, k, l) - energy_change));
-  E(density1, j, k, l) = st<typename S::rho_t>(d0 * vol_change_s);
+  const typename S::ene_t e1 = st<typename S::ene_t>((LA(energy0, j, k, l) - energy_change));
+  const typename S::rho_t d1 = st<typename S::rho_t>(d0 * vol_change_s);
+  energy1[o] = e1;
+  density1[o] = d1;
+  if (xe) {
+    xh_cell<2>(energy1, o, j, g.x_max, e1);
+    xh_cell<2>(density1, o, j, g.x_max, d1);
+  }
 #undef LA
   });
 }
@@ -490,7 +513,7 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 4 : (sizeof(typename S::ar
     typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
     const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
     const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-    Level0<S> lz) {
+    Level0<S> lz, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
   const int lane = threadIdx.x;
   const int c = g.x_min - 2 + t.x * 28 + lane;
@@ -540,7 +563,13 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 4 : (sizeof(typename S::ar
     // the cell update takes the FP64 face fluxes; the stored mass flux
     // (mf_t) feeds only the momentum sweep
     mf_st = mflux;
-    if (lane <= 29) E(mass_flux, c, k, l) = st<MF>(mflux);
+    if (lane <= 29) {
+      const long long o = off3(g, c, k, l);
+      const MF mf0 = st<MF>(mflux);
+      // with xh face x_max+2 is halo, written with its mirrored face
+      if (!xh || c <= g.x_max + 1) mass_flux[o] = mf0;
+      if (xh && xh_edge(c, g.x_max)) xh_node<2>(mass_flux, o, c, g.x_max, -mf0);
+    }
     const AL sigmam = div_rn((AL)fabs(mflux), (AL)d_don * (AL)pv_don);
     diffuw = (AL)(e_don - e_up);
     diffdw = (AL)(e_dn - e_don);
@@ -560,6 +589,11 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 4 : (sizeof(typename S::ar
     const typename S::ene_t en = st<typename S::ene_t>(poe);
     E(d_out, c, k, l) = dn;
     E(e_out, c, k, l) = en;
+    if (xh && xh_edge(c, g.x_max)) {
+      const long long o = off3(g, c, k, l);
+      xh_cell<2>(d_out, o, c, g.x_max, dn);
+      xh_cell<2>(e_out, o, c, g.x_max, en);
+    }
     if (lz.density0) {  // last sweep of the step: reset_field
       E(lz.density0, c, k, l) = dn;
       E(lz.energy0, c, k, l) = en;
@@ -733,7 +767,7 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && !
     const typename S::nd_t* __restrict__ node_mass_pre, const typename S::vel_t* __restrict__ u_in,
     const typename S::vel_t* __restrict__ v_in, const typename S::vel_t* __restrict__ w_in,
     typename S::vel_t* __restrict__ u_out, typename S::vel_t* __restrict__ v_out,
-    typename S::vel_t* __restrict__ w_out, Level0<S> lz) {
+    typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
   const MarchRange r = mom_vel_range<DIR>(g);
   const int jlo = r.jlo, jhi = r.jhi, clo = r.clo, chi = r.chi, plo = r.plo, phi = r.phi;
@@ -798,6 +832,10 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && !
       const V vn1 = st<V>(vn[q]);
       EI(out[q], IDX(p)) = vn1;
       if (lz.xvel0) EI(lev0[q], IDX(p)) = vn1;  // last sweep of the step: reset_field
+      if (xh && xh_edge(j, g.x_max)) {  // the last sweep's buffer carries its input's halo
+        const V hv = lz.xvel0 ? st<V>(vw[q][1]) : vn1;
+        xh_node<2>(out[q], off3(g, IDX(p)), j, g.x_max, q == 0 ? -hv : hv);
+      }
     }
     pre_0 = pre_p;
   }
@@ -825,7 +863,7 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && M
     typename S::rho_t* __restrict__ density1, typename S::ene_t* __restrict__ energy1,
     const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
     const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-    Level0<S> lz) {
+    Level0<S> lz, bool xh) {
   // old density/energy of cells c1+1, c1+2 of each thread's segment
   __shared__ double s_end[4][BY][BX];
   m.run([&](const Geom& g, const Tile& t) {
@@ -872,6 +910,7 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && M
   const double* vd = DIR == 2 ? ga.vertexdy : ga.vertexdz;
 #define VD(p) vd[g.o1 + (p) - pmin + 2]
   const bool update = c <= r.cmax;
+  const bool xe = xh && xh_edge(j, g.x_max);
   using R = typename S::rho_t;
   using En = typename S::ene_t;
   using MF = typename S::mf_t;
@@ -916,7 +955,11 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && M
     AL diffdw = (AL)(d_dn - d_don);
     AL limiter = cell_limiter<AL>(sigmat, sigma3, sigma4, diffuw, diffdw);
     const double mflux = vf * (d_don + (double)limiter);
-    if (p <= c1 || last) EI(mass_flux, IDX(p)) = st<MF>(mflux);
+    if (p <= c1 || last) {
+      const MF mf0 = st<MF>(mflux);
+      EI(mass_flux, IDX(p)) = mf0;
+      if (xe) xh_face<2>(mass_flux, off3(g, IDX(p)), j, g.x_max, mf0);
+    }
     const double mf_stored = mflux;  // FP64 in the cell update; mf_t storage feeds the momentum sweep
     const AL sigmam = div_rn((AL)fabs(mflux), (AL)d_don * (AL)pv_don);
     diffuw = (AL)(e_don - e_up);
@@ -933,6 +976,11 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && M
       const En en = st<En>(poe);
       EI(density1, IDX(p - 1)) = dn;
       EI(energy1, IDX(p - 1)) = en;
+      if (xe) {
+        const long long o = off3(g, IDX(p - 1));
+        xh_cell<2>(density1, o, j, g.x_max, dn);
+        xh_cell<2>(energy1, o, j, g.x_max, en);
+      }
       if (lz.density0) {  // last sweep of the step: reset_field
         EI(lz.density0, IDX(p - 1)) = dn;
         EI(lz.energy0, IDX(p - 1)) = en;
@@ -967,7 +1015,7 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat || sizeof(typename S::arith_
     const typename S::vel_t* __restrict__ u_in, const typename S::vel_t* __restrict__ v_in,
     const typename S::vel_t* __restrict__ w_in, typename S::vel_t* __restrict__ u_out,
     typename S::vel_t* __restrict__ v_out, typename S::vel_t* __restrict__ w_out,
-    Level0<S> lz) {
+    Level0<S> lz, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
   const int seg = m.seg;
   const int lane = threadIdx.x;
@@ -1018,7 +1066,7 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat || sizeof(typename S::arith_
     using A = typename S::arith_t;
     const MomNodeTerms<A> nt =
         mom_node_terms<A>((A)nf, (A)nmpre, (A)nmpre_p, (A)cd_0, (A)cd_m1, (A)cd_p1);
-    A vn[3];
+    A vn[3], vi[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) {
       A mf = A(0.0), v0 = A(0.0);
@@ -1030,6 +1078,7 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat || sizeof(typename S::arith_
       }
       const A mf_m = __shfl_up_sync(0xffffffffu, mf, 1);
       vn[q] = v0 * (A)nmpre + mf_m - mf;
+      vi[q] = v0;
     }
     if (has_up) {
       div3_rn(vn, (A)nmp);  // the three updates share node_mass_post
@@ -1038,6 +1087,10 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat || sizeof(typename S::arith_
         const V vn1 = st<V>(vn[q]);
         E(out[q], j, k, l) = vn1;
         if (lz.xvel0) E(lev0[q], j, k, l) = vn1;  // last sweep of the step: reset_field
+        if (xh && xh_edge(j, g.x_max)) {  // the last sweep's buffer carries its input's halo
+          const V hv = lz.xvel0 ? st<V>(vi[q]) : vn1;
+          xh_node<2>(out[q], off3(g, j, k, l), j, g.x_max, q == 0 ? -hv : hv);
+        }
       }
     }
     fm_a = f_a; fm_b = f_b; fm_c = f_c; fm_d = f_d;
@@ -1185,11 +1238,11 @@ void launch_visc_dt(const Target& tg, cudaStream_t s, const GeomArrays& ga, doub
                     const typename S::ene_t* energy0, typename S::cs_t* pressure,
                     typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
                     const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
-                    const typename S::vel_t* zvel0, unsigned long long* min_key) {
+                    const typename S::vel_t* zvel0, unsigned long long* min_key, bool xh) {
   launch_mapped2(tg, s, kKeyTimestepVisc, grid_visc, grid_visc_flat, 0, false, kBlk, k_visc_dt<S, MapSingle>,
                 k_visc_dt<S, MapBatch>, ga, g_small, dtc_safe, dtu_safe, dtv_safe, dtw_safe,
                 dtdiv_safe, density0, energy0, pressure, viscosity, soundspeed, xvel0, yvel0,
-                zvel0, min_key);
+                zvel0, min_key, xh);
 }
 
 template <class S>
@@ -1197,10 +1250,10 @@ void launch_pdv_predict_eos(const Target& tg, cudaStream_t s, const double* dt_p
                             const GeomArrays& ga, const typename S::rho_t* density0,
                             const typename S::ene_t* energy0, typename S::cs_t* pressure,
                             const typename S::cs_t* viscosity, const typename S::vel_t* xvel0,
-                            const typename S::vel_t* yvel0, const typename S::vel_t* zvel0) {
+                            const typename S::vel_t* yvel0, const typename S::vel_t* zvel0, bool xh) {
   launch_mapped2(tg, s, kKeyPdvPredict, grid_interior, grid_interior_flat, 0, false, kBlk,
                 k_pdv_predict_eos<S, MapSingle>, k_pdv_predict_eos<S, MapBatchFree>, dt_ptr, ga,
-                density0, energy0, pressure, viscosity, xvel0, yvel0, zvel0);
+                density0, energy0, pressure, viscosity, xvel0, yvel0, zvel0, xh);
 }
 
 template <class S>
@@ -1212,11 +1265,11 @@ void launch_pdv_flux(const Target& tg, cudaStream_t s, const double* dt_ptr, con
                      const typename S::vel_t* yvel0, const typename S::vel_t* yvel1,
                      const typename S::vel_t* zvel0, const typename S::vel_t* zvel1,
                      typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                     typename S::vf_t* vol_flux_z) {
+                     typename S::vf_t* vol_flux_z, bool xh) {
   launch_mapped2(tg, s, kKeyPdvFlux, grid_nodes, grid_nodes_flat, 0, false, kBlk, k_pdv_flux<S, MapSingle>,
                 k_pdv_flux<S, MapBatchFree>, dt_ptr, ga, density0, density1, energy0, energy1,
                 pressure, viscosity, xvel0, xvel1, yvel0, yvel1, zvel0, zvel1, vol_flux_x,
-                vol_flux_y, vol_flux_z);
+                vol_flux_y, vol_flux_z, xh);
 }
 
 template <class S>
@@ -1226,7 +1279,7 @@ void launch_advec_cell_fused(const Target& tg, cudaStream_t s, int advect_x, int
                              const typename S::vf_t* vol_flux_x, typename S::mf_t* mass_flux_y,
                              const typename S::vf_t* vol_flux_y, typename S::mf_t* mass_flux_z,
                              const typename S::vf_t* vol_flux_z, typename S::wk_t* ener_flux,
-                             const Level0<S>& level0) {
+                             const Level0<S>& level0, bool xh) {
   (void)ener_flux;
   // pre_vol variant (the sweep's volume-flux terms) as a kernel template
   // argument: y is sweep 2 (2: after x, 3: after z); z is sweep 1 (4) or 3 (5)
@@ -1236,14 +1289,14 @@ void launch_advec_cell_fused(const Target& tg, cudaStream_t s, int advect_x, int
     launch_mapped2(tg, s, kKeyCellSweep | 2u | (V << 4), grid_cell_sweep<2>,
                    grid_cell_sweep_flat<2>, 0, false, kBlk,
                    k_cell_sweep_march<S, 2, V, MapSingle>, k_cell_sweep_march<S, 2, V, MapBatch>,
-                   ga, density1, energy1, vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_y, level0);
+                   ga, density1, energy1, vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_y, level0, xh);
   };
   auto sweep_z = [&](auto var) {
     constexpr int V = decltype(var)::value;
     launch_mapped2(tg, s, kKeyCellSweep | 3u | (V << 4), grid_cell_sweep<3>,
                    grid_cell_sweep_flat<3>, 0, false, kBlk,
                    k_cell_sweep_march<S, 3, V, MapSingle>, k_cell_sweep_march<S, 3, V, MapBatch>,
-                   ga, density1, energy1, vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_z, level0);
+                   ga, density1, energy1, vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_z, level0, xh);
   };
   // one marching pass, in place
   if (dir == 2) {
@@ -1261,22 +1314,22 @@ void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const Geom
                          typename S::rho_t* density1_out, typename S::ene_t* energy1_out,
                          const typename S::vf_t* vol_flux_x, const typename S::vf_t* vol_flux_y,
                          const typename S::vf_t* vol_flux_z, typename S::mf_t* mass_flux_x,
-                         bool copy_shell, const Level0<S>& level0, const CellXMaps* maps,
+                         bool copy_shell, const Level0<S>& level0, bool xh, const CellXMaps* maps,
                          int* status) {
   // pre_vol variant: 0 on sweep 1 (all three flux differences), 1 on sweep 3
   if (maps && !tg.plan)  // one chunk: planes staged by bulk-tensor copies
     launch_cell_sweep_x_tma<S>(tg.g, s, sweep, *maps, ga, density1_out, energy1_out, mass_flux_x,
-                               level0, status);
+                               level0, xh, status);
   else if (sweep == 1)
     launch_mapped(tg, s, kKeyCellSweepX, grid_cell_sweep_x, 0, false, kBlk,
                   k_cell_sweep_x<S, 0, MapSingle>, k_cell_sweep_x<S, 0, MapBatchFree>, ga,
                   density1_in, energy1_in, density1_out, energy1_out, vol_flux_x, vol_flux_y,
-                  vol_flux_z, mass_flux_x, level0);
+                  vol_flux_z, mass_flux_x, level0, xh);
   else
     launch_mapped(tg, s, kKeyCellSweepX | (1u << 4), grid_cell_sweep_x, 0, false, kBlk,
                   k_cell_sweep_x<S, 1, MapSingle>, k_cell_sweep_x<S, 1, MapBatchFree>, ga,
                   density1_in, energy1_in, density1_out, energy1_out, vol_flux_x, vol_flux_y,
-                  vol_flux_z, mass_flux_x, level0);
+                  vol_flux_z, mass_flux_x, level0, xh);
   // the cells the sweep does not update keep their values in the output pair
   if (copy_shell) {
     using R = typename S::rho_t;
@@ -1296,7 +1349,7 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
                             typename S::wk_t* node_flux, typename S::wk_t* node_mass_post,
                             typename S::wk_t* node_mass_pre, typename S::vel_t* const* vel_in,
                             typename S::vel_t* const* vel_out, bool copy_shell,
-                            const Level0<S>& level0, const MomXMaps* x_maps, int* status,
+                            const Level0<S>& level0, bool xh, const MomXMaps* x_maps, int* status,
                             const NodeMaps* node_maps, const VelMaps* vel_maps) {
   // the node arrays of the y/z sweeps live in three work arrays, as nd_t
   using ND = typename S::nd_t;
@@ -1319,18 +1372,18 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
                     vol_flux_z, nd_flux, nd_post, nd_pre);
     if (vel_maps && !tg.plan)
       launch_mom_vel_tma<S>(tg.g, s, D, *vel_maps, ga, nd_flux, nd_pre, vel_in, vel_out, level0,
-                            status);
+                            xh, status);
     else
       launch_mapped2(tg, s, kKeyMomVel3 | D, grid_mom_vel<D>, grid_mom_vel_flat<D>, kMarchSeg,
                      true, kBlk, k_mom_vel3_march<S, D, MapSingle>,
                      k_mom_vel3_march<S, D, MapBatchFree>, ga, nd_flux, nd_post, nd_pre,
-                     vel_in[0], vel_in[1], vel_in[2], vel_out[0], vel_out[1], vel_out[2], level0);
+                     vel_in[0], vel_in[1], vel_in[2], vel_out[0], vel_out[1], vel_out[2], level0, xh);
   };
   using I2 = std::integral_constant<int, 2>;
   using I3 = std::integral_constant<int, 3>;
   if (dir == 1 && x_maps && !tg.plan) {
     // one pass, its planes staged in shared memory
-    launch_mom_x_tma<S>(tg.g, s, sweep, *x_maps, ga, vel_out, level0, status);
+    launch_mom_x_tma<S>(tg.g, s, sweep, *x_maps, ga, vel_out, level0, xh, status);
   } else if (dir == 1) {
     // one pass for the three velocities
     auto sweep_x = [&](auto var) {
@@ -1338,7 +1391,7 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
       launch_mapped(tg, s, kKeyMomSweepX | (V << 4), grid_mom_sweep_x, kMarchSeg, true, kBlk,
                     k_mom_sweep_x<S, V, MapSingle>, k_mom_sweep_x<S, V, MapBatchFree>, ga,
                     mass_flux_x, density1, vol_flux_x, vol_flux_y, vol_flux_z, vel_in[0],
-                    vel_in[1], vel_in[2], vel_out[0], vel_out[1], vel_out[2], level0);
+                    vel_in[1], vel_in[2], vel_out[0], vel_out[1], vel_out[2], level0, xh);
     };
     if (sweep == 1) sweep_x(std::integral_constant<int, 0>{});
     else sweep_x(std::integral_constant<int, 4>{});
@@ -1366,31 +1419,31 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
                                   double, double, double, double, const S::rho_t*,             \
                                   const S::ene_t*, S::cs_t*, S::cs_t*, S::cs_t*,               \
                                   const S::vel_t*, const S::vel_t*, const S::vel_t*,           \
-                                  unsigned long long*);                                        \
+                                  unsigned long long*, bool);                                  \
   template void launch_pdv_predict_eos<S>(const Target&, cudaStream_t, const double*,            \
                                           const GeomArrays&, const S::rho_t*, const S::ene_t*, \
                                           S::cs_t*, const S::cs_t*, const S::vel_t*,           \
-                                          const S::vel_t*, const S::vel_t*);                   \
+                                          const S::vel_t*, const S::vel_t*, bool);             \
   template void launch_pdv_flux<S>(const Target&, cudaStream_t, const double*, const GeomArrays&, \
                                    const S::rho_t*, S::rho_t*, const S::ene_t*, S::ene_t*,     \
                                    const S::cs_t*, const S::cs_t*, const S::vel_t*,            \
                                    const S::vel_t*, const S::vel_t*, const S::vel_t*,          \
                                    const S::vel_t*, const S::vel_t*, S::vf_t*, S::vf_t*,       \
-                                   S::vf_t*);                                                  \
+                                   S::vf_t*, bool);                                            \
   template void launch_advec_cell_fused<S>(const Target&, cudaStream_t, int, int, int,           \
                                            const GeomArrays&, S::rho_t*, S::ene_t*, S::mf_t*,  \
                                            const S::vf_t*, S::mf_t*, const S::vf_t*, S::mf_t*, \
-                                           const S::vf_t*, S::wk_t*, const Level0<S>&);        \
+                                           const S::vf_t*, S::wk_t*, const Level0<S>&, bool);  \
   template void launch_advec_cell_x<S>(const Target&, cudaStream_t, int, const GeomArrays&,      \
                                        const S::rho_t*, const S::ene_t*, S::rho_t*, S::ene_t*,  \
                                        const S::vf_t*, const S::vf_t*, const S::vf_t*,          \
-                                       S::mf_t*, bool, const Level0<S>&, const CellXMaps*, int*); \
+                                       S::mf_t*, bool, const Level0<S>&, bool, const CellXMaps*, int*); \
   template void launch_advec_mom_fused<S>(const Target&, cudaStream_t, int, int, int, double,    \
                                           const GeomArrays&, const S::rho_t*, const S::mf_t*,  \
                                           const S::mf_t*, const S::mf_t*, const S::vf_t*,      \
                                           const S::vf_t*, const S::vf_t*, S::wk_t*, S::wk_t*,  \
                                           S::wk_t*, S::vel_t* const*, S::vel_t* const*, bool,  \
-                                          const Level0<S>&, const MomXMaps*, int*,            \
+                                          const Level0<S>&, bool, const MomXMaps*, int*,      \
                                           const NodeMaps*, const VelMaps*);
 
 INSTF(F64)

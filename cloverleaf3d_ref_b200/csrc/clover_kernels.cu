@@ -16,6 +16,7 @@
 #include "../../include/clover_kernels.h"
 #include "clover_div.cuh"
 #include "clover_launch.h"
+#include "clover_stencil.cuh"
 #include "clover_sum.cuh"
 
 namespace clover {
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(BX * BY, UM ? 5 : 4) k_accelerate(M m, double 
     const typename S::cs_t* __restrict__ pressure, const typename S::cs_t* __restrict__ viscosity,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ zvel0, typename S::vel_t* __restrict__ xvel1,
-    typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1) {
+    typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
   TILE_THREAD(nodes(g), t);
   const double dt = dt_ptr ? dt_ptr[(long long)t.d * kScalarStride] : dt_val;
@@ -440,15 +441,26 @@ __global__ void __launch_bounds__(BX * BY, UM ? 5 : 4) k_accelerate(M m, double 
                       za3 * (p110 - p111));
 #undef LA
   using V = typename S::vel_t;
-  E(xvel1, j, k, l) = st<V>(xvel1_s -
+  const long long o = off3(g, j, k, l);
+  const V un = st<V>(xvel1_s -
       stepbymass_s * (xa0 * (q000 - q100) + xa1 * (q010 - q110) + xa2 * (q001 - q101) +
                       xa3 * (q011 - q111)));
-  E(yvel1, j, k, l) = st<V>(yvel1_s -
+  const V vn = st<V>(yvel1_s -
       stepbymass_s * (ya0 * (q000 - q010) + ya1 * (q100 - q110) + ya2 * (q001 - q011) +
                       ya3 * (q101 - q111)));
-  E(zvel1, j, k, l) = st<V>(zvel1_s -
+  const V wn = st<V>(zvel1_s -
       stepbymass_s * (za0 * (q000 - q001) + za1 * (q010 - q011) + za2 * (q100 - q101) +
                       za3 * (q110 - q111)));
+  xvel1[o] = un;
+  yvel1[o] = vn;
+  zvel1[o] = wn;
+  if (xh && xh_edge(j, g.x_max)) {
+    xh_node<2>(xvel1, o, j, g.x_max, -un);
+    xh_node<2>(yvel1, o, j, g.x_max, vn);
+    xh_node<2>(zvel1, o, j, g.x_max, wn);
+    xh_node<1>(const_cast<V*>(xvel0), o, j, g.x_max, -__ldg(xvel0 + o));
+    xh_node<1>(const_cast<V*>(yvel0), o, j, g.x_max, __ldg(yvel0 + o));
+  }
   });
 }
 
@@ -1502,30 +1514,31 @@ __device__ __forceinline__ void halo_faces(const Geom& g, const HaloOne& h, int 
   }
 }
 
-template <int D, class T>
+// X: with the x faces
+template <int D, bool X, class T>
 __device__ __forceinline__ void halo_one(const Geom& g, const HaloOne& h, int fi, int tile) {
-  const int wx = (g.x_max + 2 * D + 1 + 31) / 32, wy = (g.y_max + 1 + 31) / 32;
+  const int wx = (g.x_max + 2 * D + 1 + 31) / 32;
   const int tz = wx * ((g.y_max + 2 * D + 1 + 7) / 8), ty = wx * ((g.z_max + 1 + 7) / 8);
   if (tile < tz) halo_faces<D, 2, T>(g, h, fi, tile, wx);
   else if (tile < tz + ty) halo_faces<D, 1, T>(g, h, fi, tile - tz, wx);
-  else halo_faces<D, 0, T>(g, h, fi, tile - tz - ty, wy);
+  else if constexpr (X) halo_faces<D, 0, T>(g, h, fi, tile - tz - ty, (g.y_max + 1 + 31) / 32);
 }
 
-template <int D, class M>
+template <int D, bool X, class M>
 __global__ void __launch_bounds__(BX * BY) k_halo_one(M m, const __grid_constant__ HaloOne h) {
   m.run([&](const Geom& g, const Tile& t) {
-    if (h.bytes[t.y] == 8) halo_one<D, double>(g, h, t.y, t.x);
-    else halo_one<D, float>(g, h, t.y, t.x);
+    if (h.bytes[t.y] == 8) halo_one<D, X, double>(g, h, t.y, t.x);
+    else halo_one<D, X, float>(g, h, t.y, t.x);
   });
 }
 
 // tiles of k_halo_one; aux = fields
-template <int D>
+template <int D, bool X>
 dim3 grid_halo_one(const Geom& g, int fields) {
   const int nx = g.x_max, ny = g.y_max, nz = g.z_max;
   const int wx = (nx + 2 * D + 1 + 31) / 32;
   return dim3(wx * ((ny + 2 * D + 1 + 7) / 8) + wx * ((nz + 1 + 7) / 8) +
-                  ((ny + 1 + 31) / 32) * ((nz + 1 + 7) / 8),
+                  (X ? ((ny + 1 + 31) / 32) * ((nz + 1 + 7) / 8) : 0),
               fields, 1);
 }
 
@@ -1712,17 +1725,17 @@ void launch_accelerate(const Target& tg, cudaStream_t s, double dt_val, const do
                        const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
                        const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
                        const typename S::vel_t* zvel0, typename S::vel_t* xvel1,
-                       typename S::vel_t* yvel1, typename S::vel_t* zvel1, bool uniform_mesh) {
+                       typename S::vel_t* yvel1, typename S::vel_t* zvel1, bool uniform_mesh, bool xh) {
   if (uniform_mesh)
     launch_mapped2(tg, s, kKeyAccelerate, grid_nodes, grid_nodes_flat, 0, false, dim3(BX, BY),
                    k_accelerate<S, MapSingle, true>, k_accelerate<S, MapBatchFree, true>, dt_val,
                    dt_ptr, ga, density0, pressure, viscosity, xvel0, yvel0, zvel0, xvel1, yvel1,
-                   zvel1);
+                   zvel1, xh);
   else
     launch_mapped2(tg, s, kKeyAccelerate, grid_nodes, grid_nodes_flat, 0, false, dim3(BX, BY),
                    k_accelerate<S, MapSingle, false>, k_accelerate<S, MapBatchFree, false>, dt_val,
                    dt_ptr, ga, density0, pressure, viscosity, xvel0, yvel0, zvel0, xvel1, yvel1,
-                   zvel1);
+                   zvel1, xh);
 }
 
 template <class S>
@@ -1886,7 +1899,8 @@ static int elem_bytes_of(int id) {
 
 template <class S>
 void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, const int* fields,
-                        int depth, const int* external_faces, bool composed, const HaloFields* also) {
+                        int depth, const int* external_faces, bool composed, const HaloFields* also,
+                        bool x_faces) {
   // field id -> (kind, component)
   static const int kind[19] = {0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2};
   static const int comp[19] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 2, 2, 0, 1, 2, 0, 1, 2};
@@ -1903,13 +1917,19 @@ void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, c
     }
     if (h.n == 0) return;
     const dim3 blk(BX, BY);
-    const unsigned key = kKeyHalo | (unsigned)(depth << 5) | (unsigned)h.n;
-    if (depth == 1)
-      launch_mapped(tg, s, key, grid_halo_one<1>, h.n, false, blk, k_halo_one<1, MapSingle>,
-                    k_halo_one<1, MapBatchFree>, h);
-    else
-      launch_mapped(tg, s, key, grid_halo_one<2>, h.n, false, blk, k_halo_one<2, MapSingle>,
-                    k_halo_one<2, MapBatchFree>, h);
+    const unsigned key = kKeyHalo | (x_faces ? 0u : 128u) | (unsigned)(depth << 5) | (unsigned)h.n;
+    auto go = [&](auto d, auto x) {
+      constexpr int D = decltype(d)::value;
+      constexpr bool X = decltype(x)::value;
+      launch_mapped(tg, s, key, grid_halo_one<D, X>, h.n, false, blk, k_halo_one<D, X, MapSingle>,
+                    k_halo_one<D, X, MapBatchFree>, h);
+    };
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    if (depth == 1 && x_faces) go(One{}, std::true_type{});
+    else if (depth == 1) go(One{}, std::false_type{});
+    else if (x_faces) go(Two{}, std::true_type{});
+    else go(Two{}, std::false_type{});
     return;
   }
   // faces: 0 left, 1 right, 2 bottom, 3 top, 4 back, 5 front; axis order y, x, z
@@ -2005,7 +2025,7 @@ void launch_fill(cudaStream_t s, T* p, long long elems, T value) {
   template void launch_accelerate<S>(const Target&, cudaStream_t, double, const double*,           \
                                      const GeomArrays&, const S::rho_t*, const S::cs_t*,       \
                                      const S::cs_t*, const S::vel_t*, const S::vel_t*,          \
-                                     const S::vel_t*, S::vel_t*, S::vel_t*, S::vel_t*, bool);  \
+                                     const S::vel_t*, S::vel_t*, S::vel_t*, S::vel_t*, bool, bool); \
   template void launch_flux_calc<S>(const Geom&, cudaStream_t, double, const double*,            \
                                     const GeomArrays&, const S::vel_t*, const S::vel_t*,       \
                                     const S::vel_t*, const S::vel_t*, const S::vel_t*,          \
@@ -2030,7 +2050,7 @@ void launch_fill(cudaStream_t s, T* p, long long elems, T value) {
                                               const S::cs_t*, const S::vel_t*, const S::vel_t*, \
                                               const S::vel_t*, double*, double*);              \
   template void launch_update_halo<S>(const Target&, cudaStream_t, const HaloFields&, const int*,  \
-                                      int, const int*, bool, const HaloFields*);                \
+                                      int, const int*, bool, const HaloFields*, bool);                \
   template void launch_generate_chunk<S>(const Geom&, cudaStream_t, const GeomArrays&,          \
                                          S::rho_t*, S::ene_t*, S::vel_t*, S::vel_t*,           \
                                          S::vel_t*, const StateTable&);

@@ -252,7 +252,8 @@ void launch_accelerate(const Target& tg, cudaStream_t s, double dt_val, const do
                        const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
                        const typename S::vel_t* zvel0, typename S::vel_t* xvel1,
                        typename S::vel_t* yvel1, typename S::vel_t* zvel1,
-                       bool uniform_mesh = false);  // volume and areas from Geom::vol, xa, ya, za
+                       bool uniform_mesh = false,  // volume and areas from Geom::vol, xa, ya, za
+                       bool xh = false);
 
 template <class S>
 void launch_flux_calc(const Geom& g, cudaStream_t s, double dt_val, const double* dt_ptr,
@@ -328,7 +329,8 @@ void launch_field_summary(const Geom& g, cudaStream_t s, const double* volume,
 // every selected field comes from the policy S. composed: every face is
 // external and every deck has three or more cells per axis from index 1
 // (halo_composes), so that one launch writes all faces, and the same halo into
-// also's arrays where they are given; otherwise one pass per axis, in the
+// also's arrays where they are given (without x_faces: the y and z faces only,
+// whose planes and rows reach into the x halo columns); otherwise one pass per axis, in the
 // reference's order, over the external faces.
 inline bool halo_composes(const Geom& g) {
   return g.x_min == 1 && g.y_min == 1 && g.z_min == 1 && g.x_max >= 3 && g.y_max >= 3 && g.z_max >= 3;
@@ -336,7 +338,7 @@ inline bool halo_composes(const Geom& g) {
 template <class S>
 void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, const int* fields,
                         int depth, const int* external_faces /*6: left..front*/, bool composed,
-                        const HaloFields* also = nullptr);
+                        const HaloFields* also = nullptr, bool x_faces = true);
 
 // initialise_chunk_kernel + generate_chunk_kernel on the device.
 struct StateTable {
@@ -358,6 +360,11 @@ void launch_generate_chunk(const Geom& g, cudaStream_t s, const GeomArrays& ga,
                            typename S::vel_t* zvel0, const StateTable& st);
 
 // ---- fused kernels of the native step (clover_fused.cu) ----
+// xh (here and in launch_accelerate): each kernel also writes the x-face halo of
+// the rows it stores, as the update_halo that follows would, which then leaves
+// the x faces out (launch_update_halo's x_faces). For decks whose face passes
+// compose. accelerate writes it for xvel0 and yvel0 too, and the viscosity
+// kernel for density0 and energy0 (the step-start update, one layer).
 // viscosity and calc_dt of every interior cell in one pass; the cell minimum
 // folds into min_key (per deck over a plan).
 template <class S>
@@ -367,13 +374,13 @@ void launch_visc_dt(const Target& tg, cudaStream_t s, const GeomArrays& ga, doub
                     const typename S::ene_t* energy0, typename S::cs_t* pressure,
                     typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
                     const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
-                    const typename S::vel_t* zvel0, unsigned long long* min_key);
+                    const typename S::vel_t* zvel0, unsigned long long* min_key, bool xh);
 template <class S>
 void launch_pdv_predict_eos(const Target& tg, cudaStream_t s, const double* dt_ptr,
                             const GeomArrays& ga, const typename S::rho_t* density0,
                             const typename S::ene_t* energy0, typename S::cs_t* pressure,
                             const typename S::cs_t* viscosity, const typename S::vel_t* xvel0,
-                            const typename S::vel_t* yvel0, const typename S::vel_t* zvel0);
+                            const typename S::vel_t* yvel0, const typename S::vel_t* zvel0, bool xh);
 template <class S>
 void launch_pdv_flux(const Target& tg, cudaStream_t s, const double* dt_ptr, const GeomArrays& ga,
                      const typename S::rho_t* density0, typename S::rho_t* density1,
@@ -383,7 +390,7 @@ void launch_pdv_flux(const Target& tg, cudaStream_t s, const double* dt_ptr, con
                      const typename S::vel_t* yvel0, const typename S::vel_t* yvel1,
                      const typename S::vel_t* zvel0, const typename S::vel_t* zvel1,
                      typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                     typename S::vf_t* vol_flux_z);
+                     typename S::vf_t* vol_flux_z, bool xh);
 template <class S>
 void launch_advec_cell_fused(const Target& tg, cudaStream_t s, int advect_x, int dir, int sweep,
                              const GeomArrays& ga, typename S::rho_t* density1,
@@ -391,7 +398,7 @@ void launch_advec_cell_fused(const Target& tg, cudaStream_t s, int advect_x, int
                              const typename S::vf_t* vol_flux_x, typename S::mf_t* mass_flux_y,
                              const typename S::vf_t* vol_flux_y, typename S::mf_t* mass_flux_z,
                              const typename S::vf_t* vol_flux_z, typename S::wk_t* ener_flux,
-                             const Level0<S>& level0);
+                             const Level0<S>& level0, bool xh);
 // The x cell sweep out of place: density1/energy1 in one buffer pair, the
 // updated values in the other, and with copy_shell a copy of every cell
 // outside the interior (left out where a depth-2 halo update of density1 and
@@ -403,7 +410,7 @@ void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const Geom
                          typename S::rho_t* density1_out, typename S::ene_t* energy1_out,
                          const typename S::vf_t* vol_flux_x, const typename S::vf_t* vol_flux_y,
                          const typename S::vf_t* vol_flux_z, typename S::mf_t* mass_flux_x,
-                         bool copy_shell, const Level0<S>& level0,
+                         bool copy_shell, const Level0<S>& level0, bool xh,
                          const CellXMaps* maps = nullptr, int* status = nullptr);
 // All three velocities of one sweep; vel_in/vel_out are the two buffers of
 // each velocity pair, and with copy_shell the shell outside [min,max+1]^3 is
@@ -427,7 +434,7 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
                             typename S::wk_t* node_flux, typename S::wk_t* node_mass_post,
                             typename S::wk_t* node_mass_pre, typename S::vel_t* const* vel_in,
                             typename S::vel_t* const* vel_out, bool copy_shell,
-                            const Level0<S>& level0, const MomXMaps* x_maps = nullptr,
+                            const Level0<S>& level0, bool xh, const MomXMaps* x_maps = nullptr,
                             int* status = nullptr, const NodeMaps* node_maps = nullptr,
                             const VelMaps* vel_maps = nullptr);
 

@@ -327,14 +327,16 @@ struct Chunk : ChunkBase {
 
   // shell_vb: the time-level-1 velocities' halo goes to that buffer of their
   // pairs too (one-launch updates only)
-  void halo(std::initializer_list<int> ids, int depth, int vb = 0, int cb = 0, int shell_vb = -1) {
+  // x_faces: false where the kernels before it wrote the x faces' halo
+  void halo(std::initializer_list<int> ids, int depth, int vb = 0, int cb = 0, int shell_vb = -1,
+            bool x_faces = true) {
     int fields[19] = {0};
     for (int id : ids) fields[id - 1] = 1;
     HaloFields also{};
     if (shell_vb >= 0)
       for (int c3 = 0; c3 < 3; c3++) also.f[8 + 2 * c3] = vel1(c3, shell_vb);
     launch_update_halo<S>(tg, stream, halo_fields(vb, cb), fields, depth, ext, halo_repeat_free,
-                          shell_vb >= 0 ? &also : nullptr);
+                          shell_vb >= 0 ? &also : nullptr, x_faces);
   }
 
   int deck_blocks() const { return (nd + 127) / 128; }
@@ -824,6 +826,7 @@ struct Chunk : ChunkBase {
     const double n = cells();
     const double R8 = sizeof(R), E8 = sizeof(En), C8 = sizeof(C), V8 = sizeof(V),
                  VF8 = sizeof(VF), MF8 = sizeof(MF), N8 = sizeof(ND);
+    const bool xh = halo_repeat_free;  // the kernels write the x faces' halo of the rows they store
     int vc = ax ? 0 : 1;  // buffer of the velocity pairs at the start of this step
     int cb = ax ? 0 : 1;  // buffer of the density1/energy1 pair at the start of this step
     // timestep.f90:56-126
@@ -834,21 +837,21 @@ struct Chunk : ChunkBase {
     // update of the pressure's halo is left out: the depth-1 update after the
     // predictor rewrites the same cells before anything reads them.
     pbeg();
-    halo({3, 1, 8, 10}, 1, vc, cb);
+    halo({3, 1, 8, 10}, 1, vc, cb, -1, !xh);
     pend("update_halo", 0);
     pbeg();
     if (tma && use_tma)
       launch_visc_dt_tma<S>(g, stream, visc_maps, ga, kGSmall, deck.dtc_safe, deck.dtu_safe,
                             deck.dtv_safe, deck.dtw_safe, deck.dtdiv_safe, pressure, viscosity,
-                            soundspeed, &sc->key, &sc->status);
+                            soundspeed, &sc->key, density0, energy0, xh, &sc->status);
     else
       launch_visc_dt<S>(tg, stream, ga, kGSmall, deck.dtc_safe, deck.dtu_safe, deck.dtv_safe,
                         deck.dtw_safe, deck.dtdiv_safe, density0, energy0, pressure, viscosity,
-                        soundspeed, xvel0, yvel0, zvel0, &sc->key);
+                        soundspeed, xvel0, yvel0, zvel0, &sc->key, xh);
     k_dt_finalize<<<deck_blocks(), 128, 0, stream>>>(sc, nd, dt_hist);
     pend("eos_viscosity_calc_dt", n * (3 * V8 + R8 + E8 + 3 * C8));
     pbeg();
-    halo({6}, 1, vc, cb);  // read by accelerate at its neighbours
+    halo({6}, 1, vc, cb, -1, !xh);  // read by accelerate at its neighbours
     pend("update_halo", 0);
     // PdV.f90:50-107: predictor + EOS on the predicted state; revert is implied
     pbeg();
@@ -857,13 +860,13 @@ struct Chunk : ChunkBase {
         tmap(zvel0, sizeof(V), 9, &pdv_m.w) && tmap(density0, sizeof(R), 8, &pdv_m.d) &&
         tmap(energy0, sizeof(En), 8, &pdv_m.e) && tmap(pressure, sizeof(C), 8, &pdv_m.p) &&
         tmap(viscosity, sizeof(C), 8, &pdv_m.q))
-      launch_pdv_predict_eos_tma<S>(g, stream, dtp, pdv_m, pressure, &sc->status);
+      launch_pdv_predict_eos_tma<S>(g, stream, dtp, pdv_m, pressure, xh, &sc->status);
     else
       launch_pdv_predict_eos<S>(tg, stream, dtp, ga, density0, energy0, pressure, viscosity, xvel0,
-                                yvel0, zvel0);
+                                yvel0, zvel0, xh);
     pend("pdv", n * (R8 + E8 + 3 * C8 + 3 * V8));
     pbeg();
-    halo({5}, 1, vc, cb);
+    halo({5}, 1, vc, cb, -1, !xh);
     pend("update_halo", 0);
     pbeg();
     AccMaps acc_m;
@@ -876,7 +879,8 @@ struct Chunk : ChunkBase {
       fused_flux = acc_tma;
       if (fused_flux) {
         launch_acc_flux_tma<S>(g, stream, dtp, acc_m, rho1(cb), energy0, ene1(cb), vel1(0, vc),
-                               vel1(1, vc), vel1(2, vc), vol_flux_x, vol_flux_y, vol_flux_z, &sc->status);
+                               vel1(1, vc), vel1(2, vc), vol_flux_x, vol_flux_y, vol_flux_z, xvel0,
+                               yvel0, xh, &sc->status);
         pend("accelerate_pdv_flux", n * (2 * R8 + 2 * E8 + 2 * C8 + 6 * V8 + 3 * VF8));
       }
     }
@@ -886,11 +890,11 @@ struct Chunk : ChunkBase {
         staged = acc_tma;
         if (staged)
           launch_accelerate_tma<S>(g, stream, dtp, acc_m, vel1(0, vc), vel1(1, vc), vel1(2, vc),
-                                   &sc->status);
+                                   xvel0, yvel0, xh, &sc->status);
       }
       if (!staged)
         launch_accelerate<S>(tg, stream, 0.0, dtp, ga, density0, pressure, viscosity, xvel0, yvel0,
-                             zvel0, vel1(0, vc), vel1(1, vc), vel1(2, vc), true);
+                             zvel0, vel1(0, vc), vel1(1, vc), vel1(2, vc), true, xh);
       pend("accelerate", n * (R8 + 2 * C8 + 6 * V8));
       pbeg();
       staged = false;
@@ -903,13 +907,13 @@ struct Chunk : ChunkBase {
                  tmap(vel1(2, vc), sizeof(V), 9, &flux_m.w1);
         if (staged)
           launch_pdv_flux_tma<S>(g, stream, dtp, flux_m, density0, rho1(cb), energy0, ene1(cb),
-                                 pressure, viscosity, vol_flux_x, vol_flux_y, vol_flux_z,
+                                 pressure, viscosity, vol_flux_x, vol_flux_y, vol_flux_z, xh,
                                  &sc->status);
       }
       if (!staged)
         launch_pdv_flux<S>(tg, stream, dtp, ga, density0, rho1(cb), energy0, ene1(cb), pressure,
                            viscosity, xvel0, vel1(0, vc), yvel0, vel1(1, vc), zvel0, vel1(2, vc),
-                           vol_flux_x, vol_flux_y, vol_flux_z);
+                           vol_flux_x, vol_flux_y, vol_flux_z, xh);
       pend("pdv_flux", n * (2 * R8 + 2 * E8 + 2 * C8 + 6 * V8 + 3 * VF8));
     }
     // advection.f90:43-179. The last sweep also writes time level 0 (the
@@ -925,8 +929,8 @@ struct Chunk : ChunkBase {
         pbeg();
         // before sweep 2, density1 and energy1 (updated after sweep 1) and
         // vol_flux_z (updated before sweep 1) have not changed since
-        if (sweep_number == 2 && halo_repeat_free) halo({14, 15}, 2, vc, cb);
-        else halo({4, 2, 14, 15, 16}, 2, vc, cb);
+        if (sweep_number == 2 && halo_repeat_free) halo({14, 15}, 2, vc, cb, -1, !xh);
+        else halo({4, 2, 14, 15, 16}, 2, vc, cb, -1, !xh);
         pend("update_halo", 0);
       }
       // volume fluxes read for pre_vol: all three on sweep 1, two on the y sweep,
@@ -940,7 +944,7 @@ struct Chunk : ChunkBase {
         const bool x_tma = tma && use_tma && cell_x_maps(sweep_number, cb, &xm);
         launch_advec_cell_x<S>(tg, stream, sweep_number, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
                                ene1(cb ^ 1), vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_x,
-                               !halo_repeat_free, l0, x_tma ? &xm : nullptr, &sc->status);
+                               !halo_repeat_free, l0, xh, x_tma ? &xm : nullptr, &sc->status);
         cb ^= 1;
         pend("advec_cell_x", n * (nvf * VF8 + (2 + nl0) * (R8 + E8) + MF8));
       } else {
@@ -952,12 +956,12 @@ struct Chunk : ChunkBase {
         if (tma && use_tma && halo_repeat_free && cell_maps(dir, cvar, cb, &cm)) {
           launch_cell_sweep_tma<S>(g, stream, dir, cvar, cm, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
                                    ene1(cb ^ 1), vol_flux_x, vol_flux_y, vol_flux_z,
-                                   dir == 2 ? mass_flux_y : mass_flux_z, l0, &sc->status);
+                                   dir == 2 ? mass_flux_y : mass_flux_z, l0, xh, &sc->status);
           cb ^= 1;
         } else {
           launch_advec_cell_fused<S>(tg, stream, axi, dir, sweep_number, ga, rho1(cb), ene1(cb),
                                      mass_flux_x, vol_flux_x, mass_flux_y, vol_flux_y,
-                                     mass_flux_z, vol_flux_z, work[6], l0);
+                                     mass_flux_z, vol_flux_z, work[6], l0, xh);
         }
         pend("advec_cell_yz", n * (nvf * VF8 + (2 + nl0) * (R8 + E8) + MF8));
       }
@@ -967,8 +971,8 @@ struct Chunk : ChunkBase {
       // velocities' shell before anything reads it; after sweep 3 the shell
       // carries the step's final halo, which this update writes to both buffers
       const int shell = sweep_number == 3 && halo_repeat_free ? vc ^ 1 : -1;
-      if (dir != 3 && halo_repeat_free) halo({2, 4, 9, 11, 13, 17, 18}, 2, vc, cb, shell);
-      else halo({2, 4, 9, 11, 13, 17, 18, 19}, 2, vc, cb, shell);
+      if (dir != 3 && halo_repeat_free) halo({2, 4, 9, 11, 13, 17, 18}, 2, vc, cb, shell, !xh);
+      else halo({2, 4, 9, 11, 13, 17, 18, 19}, 2, vc, cb, shell, !xh);
       pend("update_halo", 0);
       // post_vol reads two volume fluxes on sweep 1, one on sweep 2, none on sweep 3
       const double npv = sweep_number == 1 ? 2 : sweep_number == 2 ? 1 : 0;
@@ -986,7 +990,7 @@ struct Chunk : ChunkBase {
       launch_advec_mom_fused<S>(tg, stream, axi, sweep_number, dir, cell_volume, ga, rho1(cb),
                                 mass_flux_x, mass_flux_y, mass_flux_z, vol_flux_x, vol_flux_y,
                                 vol_flux_z, work[0], work[1], work[2], vin, vout,
-                                !halo_repeat_free, l0,
+                                !halo_repeat_free, l0, xh,
                                 x_tma ? &xm : nullptr, &sc->status, node_tma ? &nm : nullptr,
                                 vel_tma ? &vm : nullptr);
       // x: one pass; y, z: node pass + velocity pass

@@ -56,6 +56,34 @@ __device__ __forceinline__ A lda(const double* p) { return (A)__ldg(p); }
 template <class A>
 __device__ __forceinline__ A lda(const float* p) { return (A)__ldg(p); }
 
+// The x-face halo of the element just stored at column j (counted from 1) of a
+// row, D layers deep, for grids whose face passes compose (update_halo, k_halo_one):
+// the kernels that produce an interior row write its halo columns with it, while
+// the row's ends are at hand. A pass of its own would fetch and rewrite a 32-byte
+// sector per row end (at 512^3 FP64 the x faces were 1.4 ms of the 1.7 ms of a
+// step's halo updates). o: the element's offset; v: the value, negated by the
+// caller where the reference negates.
+// cells: 1-m <- m, nx+m <- nx+1-m
+template <int D, class T>
+__device__ __forceinline__ void xh_cell(T* a, long long o, int j, int nx, T v) {
+  if (j <= D) a[o - (2 * j - 1)] = v;
+  if (j > nx - D) a[o + 2 * (nx - j) + 1] = v;
+}
+// nodes and x faces: 1-m <- 1+m, nx+1+m <- nx+1-m
+template <int D, class T>
+__device__ __forceinline__ void xh_node(T* a, long long o, int j, int nx, T v) {
+  if (j >= 2 && j <= 1 + D) a[o - 2 * (j - 1)] = v;
+  if (j > nx - D && j <= nx) a[o + 2 * (nx + 1 - j)] = v;
+}
+// y and z faces: 1-m <- 1+m, nx+m <- nx-m
+template <int D, class T>
+__device__ __forceinline__ void xh_face(T* a, long long o, int j, int nx, T v) {
+  if (j >= 2 && j <= 1 + D) a[o - 2 * (j - 1)] = v;
+  if (j >= nx - D && j < nx) a[o + 2 * (nx - j)] = v;
+}
+// whether column j's elements have x-face halo to write
+__device__ __forceinline__ bool xh_edge(int j, int nx) { return j <= 3 || j >= nx - 2; }
+
 // vertexd(j) / vertexd(dif) of the limiter: exactly 1 where the two widths
 // are equal (every face of a uniform mesh), without the division
 __device__ __forceinline__ double width_ratio(double a, double b) {

@@ -92,7 +92,8 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
               double dtv_safe, double dtw_safe, double dtdiv_safe,
               const __grid_constant__ ViscMaps maps, typename S::cs_t* __restrict__ pressure,
               typename S::cs_t* __restrict__ viscosity, typename S::cs_t* __restrict__ soundspeed,
-              unsigned long long* __restrict__ min_key, int* __restrict__ status) {
+              unsigned long long* __restrict__ min_key, typename S::rho_t* __restrict__ density0,
+              typename S::ene_t* __restrict__ energy0, bool xh, int* __restrict__ status) {
   using P = ViscPlane<S>;
   using A = typename S::arith_t;
   using C = typename S::cs_t;
@@ -106,6 +107,10 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
   const int l1 = l0 + seg - 1 < g.z_max ? l0 + seg - 1 : g.z_max;
   const int j = j0 + tx, k = k0 + ty;
   const bool in_jk = j <= g.x_max && k <= g.y_max;
+  // with xh the x-face halo of density0 and energy0 is written below: a cell at
+  // the face takes its own value, which that halo mirrors
+  const bool xe = xh && xh_edge(j, g.x_max);
+  const int jm = xh && j == g.x_min ? 0 : -1, jp = xh && j == g.x_max ? 0 : 1;
   const int pfirst = l0 - 1, plast = l1 + 1;  // cell planes the segment reads
   if (tid == 0) {
     for (int r = 0; r < RING; r++) mbar_init(&full[r], 1);
@@ -199,7 +204,7 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
         const A yz = A(0.25) * (vgradz2 - vgradz1) / cdz + A(0.25) * (wgrady2 - wgrady1) / cdy;
         // the neighbours' pressures as ideal_gas stores them
 #define PN(bb, a, b) ((A)st<C>(((A(1.4) - A(1.0)) * DN(bb, a, b) * EN(bb, a, b))))
-        A pgradx = (PN(bl, 1, 0) - PN(bl, -1, 0)) /
+        A pgradx = (PN(bl, jp, 0) - PN(bl, jm, 0)) /
                    (cdx + (A)ga.celldx[g.o1 + j + 1 - g.x_min + 2]);
         A pgrady = (PN(bl, 0, 1) - PN(bl, 0, -1)) /
                    (cdy + (A)ga.celldy[g.o1 + k + 1 - g.y_min + 2]);
@@ -227,6 +232,11 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
       }
       const long long o = off3(g, j, k, l);
       viscosity[o] = st<C>(q);
+      if (xe) {
+        xh_cell<1>(viscosity, o, j, g.x_max, st<C>(q));
+        xh_cell<1>(density0, o, j, g.x_max, P::rho(bl)[(ty + 1) * WR + tx + HR]);
+        xh_cell<1>(energy0, o, j, g.x_max, P::ene(bl)[(ty + 1) * WE + tx + HE]);
+      }
       // calc_dt_kernel.f90:102-149 (the viscosity as stored)
       const A visc = (A)st<C>(q);
       const A d0 = DN(bl, 0, 0);
@@ -364,7 +374,8 @@ template <class S, int VAR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
 k_mom_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ MomXMaps maps,
                   typename S::vel_t* __restrict__ u_out, typename S::vel_t* __restrict__ v_out,
-                  typename S::vel_t* __restrict__ w_out, Level0<S> lz, int* __restrict__ status) {
+                  typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh,
+                  int* __restrict__ status) {
   using P = MomXPlane<S, VAR>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -490,6 +501,10 @@ k_mom_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ MomXMa
           const V vn1 = st<V>(vn[q]);
           out[q][o] = vn1;
           if (lz.xvel0) lev0[q][o] = vn1;  // last sweep of the step: reset_field
+          if (xh && xh_edge(j, g.x_max)) {  // the last sweep's buffer carries its input's halo
+            const V hv = lz.xvel0 ? P::vel(b, q)[ty * WV + cv] : vn1;
+            xh_node<2>(out[q], o, j, g.x_max, q == 0 ? -hv : hv);
+          }
         }
       }
       fm_a = f_a; fm_b = f_b; fm_c = f_c; fm_d = f_d;
@@ -591,7 +606,7 @@ template <class S, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
 k_pdv_predict_eos_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
                       const __grid_constant__ PdvMaps maps, typename S::cs_t* __restrict__ pressure,
-                      int* __restrict__ status) {
+                      bool xh, int* __restrict__ status) {
   using P = PdvPlane<S>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -668,7 +683,10 @@ k_pdv_predict_eos_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     // the predicted state goes through the storage types, as it would in memory
     const A e1 = (A)st<En>(((A)P::ene(bl)[ty * WE + tx + HE] - energy_change));
     const A d1 = (A)st<R>((d0 * vol_change_s));
-    pressure[off3(g, j, k, l)] = st<C>(((A(1.4) - A(1.0)) * d1 * e1));
+    const C pn = st<C>(((A(1.4) - A(1.0)) * d1 * e1));
+    const long long o = off3(g, j, k, l);
+    pressure[o] = pn;
+    if (xh) xh_cell<1>(pressure, o, j, g.x_max, pn);
   });
 }
 
@@ -697,6 +715,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
 k_accelerate_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
                  const __grid_constant__ AccMaps maps, typename S::vel_t* __restrict__ xvel1,
                  typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1,
+                 typename S::vel_t* __restrict__ xvel0, typename S::vel_t* __restrict__ yvel0, bool xh,
                  int* __restrict__ status) {
   using P = AccPlane<S>;
   using A = typename S::arith_t;
@@ -765,15 +784,25 @@ k_accelerate_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
         stepbymass_s * (za0 * (p000 - p001) + za1 * (p010 - p011) + za2 * (p100 - p101) +
                         za3 * (p110 - p111));
     const long long o = off3(g, j, k, l);
-    xvel1[o] = st<V>(xvel1_s -
+    const V un = st<V>(xvel1_s -
         stepbymass_s * (xa0 * (q000 - q100) + xa1 * (q010 - q110) + xa2 * (q001 - q101) +
                         xa3 * (q011 - q111)));
-    yvel1[o] = st<V>(yvel1_s -
+    const V vn = st<V>(yvel1_s -
         stepbymass_s * (ya0 * (q000 - q010) + ya1 * (q100 - q110) + ya2 * (q001 - q011) +
                         ya3 * (q101 - q111)));
-    zvel1[o] = st<V>(zvel1_s -
+    const V wn = st<V>(zvel1_s -
         stepbymass_s * (za0 * (q000 - q001) + za1 * (q010 - q011) + za2 * (q100 - q101) +
                         za3 * (q110 - q111)));
+    xvel1[o] = un;
+    yvel1[o] = vn;
+    zvel1[o] = wn;
+    if (xh && xh_edge(j, g.x_max)) {
+      xh_node<2>(xvel1, o, j, g.x_max, -un);
+      xh_node<2>(yvel1, o, j, g.x_max, vn);
+      xh_node<2>(zvel1, o, j, g.x_max, wn);
+      xh_node<1>(xvel0, o, j, g.x_max, -P::vel(bl, 0)[c]);
+      xh_node<1>(yvel0, o, j, g.x_max, P::vel(bl, 1)[c]);
+    }
   });
 }
 
@@ -799,7 +828,7 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
                typename S::ene_t* __restrict__ energy1, const typename S::cs_t* __restrict__ pressure,
                const typename S::cs_t* __restrict__ viscosity, typename S::vf_t* __restrict__ vol_flux_x,
                typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z,
-               int* __restrict__ status) {
+               bool xh, int* __restrict__ status) {
   using P = FluxPlane<S>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -854,6 +883,7 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     const Cs p_s = c_p, q_s = c_q;
     fetch(l + 1);
     const bool jin = j <= g.x_max, kin = k <= g.y_max, lin = l <= g.z_max;
+    const bool xe = xh && xh_edge(j, g.x_max);
     unsigned char* bl = pm.buf(l);
     unsigned char* bu = pm.buf(l + 1);
     // velocity q (0-2 time level 0, 3-5 time level 1) of node (j+a, k+b) of buffer bb
@@ -877,18 +907,22 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
       sx = xsum(0);
       vfx0 = st<F>(0.125 * dt * g.xa * sx);
       vol_flux_x[o] = vfx0;
+      if (xe) xh_node<2>(vol_flux_x, o, j, g.x_max, -vfx0);
     }
     if (jin && lin) {
       sy = ysum(0);
       vfy0 = st<F>(0.125 * dt * g.ya * sy);
       vol_flux_y[o] = vfy0;
+      if (xe) xh_face<2>(vol_flux_y, o, j, g.x_max, vfy0);
     }
     if (jin && kin) {
       // flux_calc_kernel.f90:86 repeats zvel0(j+1,k,l) and omits zvel0(j,k+1,l)
       const double bz = (double)(NV(bl, 2, 0, 0) + NV(bl, 2, 1, 0) + NV(bl, 2, 1, 0) +
                                  NV(bl, 2, 1, 1) + NV(bl, 5, 0, 0) + NV(bl, 5, 1, 0) +
                                  NV(bl, 5, 0, 1) + NV(bl, 5, 1, 1));
-      vol_flux_z[o] = st<F>(0.125 * dt * g.za * bz);
+      const F vfz0 = st<F>(0.125 * dt * g.za * bz);
+      vol_flux_z[o] = vfz0;
+      if (xe) xh_face<2>(vol_flux_z, o, j, g.x_max, vfz0);
       sz = zsum(bl);
     }
 #undef NV
@@ -918,8 +952,14 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     const double d0 = (double)d0_s;
     const A ad0 = (A)d0;
     const A energy_change = ((A)p_s / ad0 + (A)q_s / ad0) * (A)total_flux * geo_rvol<A>(g);
-    energy1[o] = st<typename S::ene_t>(((A)e0_s - energy_change));
-    density1[o] = st<typename S::rho_t>(d0 * vol_change_s);
+    const En e1 = st<En>(((A)e0_s - energy_change));
+    const R d1 = st<R>(d0 * vol_change_s);
+    energy1[o] = e1;
+    density1[o] = d1;
+    if (xe) {
+      xh_cell<2>(energy1, o, j, g.x_max, e1);
+      xh_cell<2>(density1, o, j, g.x_max, d1);
+    }
   });
 }
 
@@ -977,7 +1017,8 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
                typename S::ene_t* __restrict__ energy1, typename S::vel_t* __restrict__ xvel1,
                typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1,
                typename S::vf_t* __restrict__ vol_flux_x, typename S::vf_t* __restrict__ vol_flux_y,
-               typename S::vf_t* __restrict__ vol_flux_z, int* __restrict__ status) {
+               typename S::vf_t* __restrict__ vol_flux_z, typename S::vel_t* __restrict__ xvel0,
+               typename S::vel_t* __restrict__ yvel0, bool xh, int* __restrict__ status) {
   using P = AccFluxPlane<S, TYN>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -997,6 +1038,7 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
   const bool in_node = j <= g.x_max + 1 && k <= g.y_max + 1;
   const bool own = in_node && tx < TX - 1 && ty < TYN - 1;
   const bool jin = j <= g.x_max, kin = k <= g.y_max;
+  const bool xe = xh && xh_edge(j, g.x_max);
   const double dt = dt_ptr[0];
   constexpr int WV = kTmaWidth<V>, WR = kTmaWidth<R>, WC = kTmaWidth<C>;
   int xr, cr, xc, cc, xv, cv;
@@ -1096,6 +1138,13 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
         xvel1[o] = un;
         yvel1[o] = vn;
         zvel1[o] = wn;
+        if (xe) {
+          xh_node<2>(xvel1, o, j, g.x_max, -un);
+          xh_node<2>(yvel1, o, j, g.x_max, vn);
+          xh_node<2>(zvel1, o, j, g.x_max, wn);
+          xh_node<1>(xvel0, o, j, g.x_max, -P::vel(bu, 0)[cv]);
+          xh_node<1>(yvel0, o, j, g.x_max, P::vel(bu, 1)[cv]);
+        }
       }
     }
     if (__syncthreads_or(late)) break;
@@ -1111,7 +1160,12 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
         zsu = (double)(a0 + a1 + a2 + a3 + b0 + b1 + b2 + b3);
         // flux_calc_kernel.f90:86 repeats zvel0(j+1,k,l) and omits zvel0(j,k+1,l)
         const double bz = (double)(a0 + a1 + a1 + a3 + b0 + b1 + b2 + b3);
-        if (l + 1 >= l0 && l + 1 <= l1) vol_flux_z[off3(g, j, k, l + 1)] = st<F>(0.125 * dt * g.za * bz);
+        if (l + 1 >= l0 && l + 1 <= l1) {
+          const long long o = off3(g, j, k, l + 1);
+          const F vfz0 = st<F>(0.125 * dt * g.za * bz);
+          vol_flux_z[o] = vfz0;
+          if (xe) xh_face<2>(vol_flux_z, o, j, g.x_max, vfz0);
+        }
       }
       if (l >= l0 && more) {
         auto xsum = [&](int a) {
@@ -1129,11 +1183,13 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
           sx = xsum(0);
           vfx0 = st<F>(0.125 * dt * g.xa * sx);
           vol_flux_x[o] = vfx0;
+          if (xe) xh_node<2>(vol_flux_x, o, j, g.x_max, -vfx0);
         }
         if (jin) {
           sy = ysum(0);
           vfy0 = st<F>(0.125 * dt * g.ya * sy);
           vol_flux_y[o] = vfy0;
+          if (xe) xh_face<2>(vol_flux_y, o, j, g.x_max, vfy0);
         }
         if (jin && kin) {
           const En e0_s = c_e;
@@ -1165,8 +1221,14 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
           const A ad0 = (A)d0;
           const A energy_change = ((A)P::cs(bl, 0)[cc] / ad0 + (A)P::cs(bl, 1)[cc] / ad0) *
                                   (A)total_flux * geo_rvol<A>(g);
-          energy1[o] = st<En>(((A)e0_s - energy_change));
-          density1[o] = st<R>(d0 * vol_change_s);
+          const En e1 = st<En>(((A)e0_s - energy_change));
+          const R d1 = st<R>(d0 * vol_change_s);
+          energy1[o] = e1;
+          density1[o] = d1;
+          if (xe) {
+            xh_cell<2>(energy1, o, j, g.x_max, e1);
+            xh_cell<2>(density1, o, j, g.x_max, d1);
+          }
         }
       }
       zs = zsu;
@@ -1990,7 +2052,7 @@ k_mom_vel_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ VelMaps ma
               const typename S::vel_t* __restrict__ u_in, const typename S::vel_t* __restrict__ v_in,
               const typename S::vel_t* __restrict__ w_in, typename S::vel_t* __restrict__ u_out,
               typename S::vel_t* __restrict__ v_out, typename S::vel_t* __restrict__ w_out,
-              Level0<S> lz, int* __restrict__ status) {
+              Level0<S> lz, bool xh, int* __restrict__ status) {
   using P = VelPlane<S>;
   using W = typename S::nd_t;
   using V = typename S::vel_t;
@@ -2080,6 +2142,10 @@ k_mom_vel_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ VelMaps ma
       const V vn1 = st<V>(vn[q]);
       out[q][o] = vn1;
       if (lz.xvel0) lev0[q][o] = vn1;  // last sweep of the step: reset_field
+      if (xh && xh_edge(j, g.x_max)) {  // the last sweep's buffer carries its input's halo
+        const V hv = lz.xvel0 ? st<V>(vw[q][1]) : vn1;
+        xh_node<2>(out[q], o, j, g.x_max, q == 0 ? -hv : hv);
+      }
     }
     pre_0 = pre_p;
   });
@@ -2135,7 +2201,7 @@ k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMap
                  typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
                  const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
                  const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-                 Level0<S> lz, int* __restrict__ status) {
+                 Level0<S> lz, bool xh, int* __restrict__ status) {
   using P = CellPlane<S, DIR, VAR>;
   using R = typename S::rho_t;
   using En = typename S::ene_t;
@@ -2257,7 +2323,12 @@ k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMap
     AL diffdw = (AL)(d_dn - d_don);
     AL limiter = cell_limiter<AL>(sigmat, sigma3, sigma4, diffuw, diffdw);
     const double mflux = vf * (d_don + (double)limiter);
-    if (p <= q1 || last) mass_flux[off3(g, IDX(p))] = st<MFT>(mflux);
+    if (p <= q1 || last) {
+      const long long o = off3(g, IDX(p));
+      const MFT mf0 = st<MFT>(mflux);
+      mass_flux[o] = mf0;
+      if (xh && xh_edge(j, g.x_max)) xh_face<2>(mass_flux, o, j, g.x_max, mf0);
+    }
     const double mf_stored = mflux;  // FP64 in the cell update; mf_t storage feeds the momentum sweep
     const AL sigmam = div_rn((AL)fabs(mflux), (AL)d_don * (AL)pv_don);
     diffuw = (AL)(e_don - e_up);
@@ -2275,6 +2346,10 @@ k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMap
       const long long o = off3(g, IDX(p - 1));
       d_out[o] = dn;
       e_out[o] = en;
+      if (xh && xh_edge(j, g.x_max)) {
+        xh_cell<2>(d_out, o, j, g.x_max, dn);
+        xh_cell<2>(e_out, o, j, g.x_max, en);
+      }
       if (lz.density0) {  // last sweep of the step: reset_field
         lz.density0[o] = dn;
         lz.energy0[o] = en;
@@ -2338,7 +2413,7 @@ template <class S, int VAR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
 k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellXMaps maps,
                    typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
-                   typename S::mf_t* __restrict__ mass_flux, Level0<S> lz,
+                   typename S::mf_t* __restrict__ mass_flux, Level0<S> lz, bool xh,
                    int* __restrict__ status) {
   using P = CellXPlane<S, VAR>;
   using R = typename S::rho_t;
@@ -2430,7 +2505,13 @@ k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellX
       // the cell update takes the FP64 face fluxes; the stored mass flux
       // (mf_t) feeds only the momentum sweep
       mf_st = mflux;
-      if (lane < kCellXLanes) mass_flux[off3(g, c, k, l)] = st<MF>(mflux);
+      if (lane < kCellXLanes) {
+        const long long o = off3(g, c, k, l);
+        const MF mf0 = st<MF>(mflux);
+        // with xh face x_max+2 is halo, written with its mirrored face
+        if (!xh || c <= g.x_max + 1) mass_flux[o] = mf0;
+        if (xh && xh_edge(c, g.x_max)) xh_node<2>(mass_flux, o, c, g.x_max, -mf0);
+      }
       const AL sigmam = div_rn((AL)fabs(mflux), (AL)d_don * (AL)pv_don);
       diffuw = (AL)(e_don - e_up);
       diffdw = (AL)(e_dn - e_don);
@@ -2451,6 +2532,10 @@ k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellX
       const long long o = off3(g, c, k, l);
       d_out[o] = dn;
       e_out[o] = en;
+      if (xh && xh_edge(c, g.x_max)) {
+        xh_cell<2>(d_out, o, c, g.x_max, dn);
+        xh_cell<2>(e_out, o, c, g.x_max, en);
+      }
       if (lz.density0) {  // last sweep of the step: reset_field
         lz.density0[o] = dn;
         lz.energy0[o] = en;
@@ -2519,7 +2604,8 @@ void launch_visc_dt_tma(const Geom& g, cudaStream_t s, const ViscMaps& maps, con
                         double g_small, double dtc_safe, double dtu_safe, double dtv_safe,
                         double dtw_safe, double dtdiv_safe, typename S::cs_t* pressure,
                         typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
-                        unsigned long long* min_key, int* status) {
+                        unsigned long long* min_key, typename S::rho_t* density0,
+                        typename S::ene_t* energy0, bool xh, int* status) {
   auto kern = k_visc_dt_tma<S, kViscRing, kViscMinBlocks<S>>;
   const int smem = kViscRing * ViscPlane<S>::kBytes;
   int seg;
@@ -2527,7 +2613,7 @@ void launch_visc_dt_tma(const Geom& g, cudaStream_t s, const ViscMaps& maps, con
                                g.z_max - g.z_min + 1, &seg);
   kern<<<grid, dim3(TX, TY), smem, s>>>(g, seg, ga, g_small, dtc_safe, dtu_safe, dtv_safe,
                                          dtw_safe, dtdiv_safe, maps, pressure,
-                                         viscosity, soundspeed, min_key, status);
+                                         viscosity, soundspeed, min_key, density0, energy0, xh, status);
 }
 
 constexpr int kMomXRing = 4;
@@ -2547,7 +2633,7 @@ bool mom_x_tma_prepare() {
 template <class S>
 void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
-                      const Level0<S>& level0, int* status) {
+                      const Level0<S>& level0, bool xh, int* status) {
   int seg;
   const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + 1 + 28) / 29,
                                (g.y_max + 1 - g.y_min + 1 + TY - 1) / TY, g.z_max - g.z_min + 2, &seg);
@@ -2555,11 +2641,11 @@ void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& 
   if (sweep == 1)
     k_mom_sweep_x_tma<S, 0, kMomXRing, kMomXMinBlocks<S>>
         <<<grid, dim3(TX, TY), kMomXRing * MomXPlane<S, 0>::kBytes, s>>>(
-            g, seg, ga, maps, vel_out[0], vel_out[1], vel_out[2], level0, status);
+            g, seg, ga, maps, vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
   else
     k_mom_sweep_x_tma<S, 4, kMomXRing, kMomXMinBlocks<S>>
         <<<grid, dim3(TX, TY), kMomXRing * MomXPlane<S, 4>::kBytes, s>>>(
-            g, seg, ga, maps, vel_out[0], vel_out[1], vel_out[2], level0, status);
+            g, seg, ga, maps, vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
 }
 
 // The bounded wait of the staged kernels, made to run out: one block arms a
@@ -2748,7 +2834,7 @@ template <class S>
 void launch_cell_sweep_x_tma(const Geom& g, cudaStream_t s, int sweep, const CellXMaps& maps,
                              const GeomArrays& ga, typename S::rho_t* d_out,
                              typename S::ene_t* e_out, typename S::mf_t* mass_flux_x,
-                             const Level0<S>& level0, int* status) {
+                             const Level0<S>& level0, bool xh, int* status) {
   // faces x_min..x_max+2, 31 per warp
   int seg;
   const dim3 grid = plane_grid((g.x_max - g.x_min + 3 + kCellXLanes - 1) / kCellXLanes,
@@ -2756,34 +2842,36 @@ void launch_cell_sweep_x_tma(const Geom& g, cudaStream_t s, int sweep, const Cel
   if (sweep == 1)
     k_cell_sweep_x_tma<S, 0, kStencilRing, kCellXMinBlocks<S>>
         <<<grid, dim3(TX, TY), kStencilRing * CellXPlane<S, 0>::kBytes, s>>>(
-            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, status);
+            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, xh, status);
   else
     k_cell_sweep_x_tma<S, 1, kStencilRing, kCellXMinBlocks<S>>
         <<<grid, dim3(TX, TY), kStencilRing * CellXPlane<S, 1>::kBytes, s>>>(
-            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, status);
+            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, xh, status);
 }
 
 template <class S>
 void launch_pdv_predict_eos_tma(const Geom& g, cudaStream_t s, const double* dt_ptr,
-                                const PdvMaps& maps, typename S::cs_t* pressure, int* status) {
+                                const PdvMaps& maps, typename S::cs_t* pressure, bool xh,
+                                int* status) {
   int seg;
   const dim3 grid = plane_grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
                                g.z_max - g.z_min + 1, &seg);
   k_pdv_predict_eos_tma<S, kStencilRing, kStencilMinBlocks<S>>
       <<<grid, dim3(TX, TY), kStencilRing * PdvPlane<S>::kBytes, s>>>(g, seg, dt_ptr, maps,
-                                                                       pressure, status);
+                                                                       pressure, xh, status);
 }
 
 template <class S>
 void launch_accelerate_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
                            typename S::vel_t* xvel1, typename S::vel_t* yvel1,
-                           typename S::vel_t* zvel1, int* status) {
+                           typename S::vel_t* zvel1, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
+                           bool xh, int* status) {
   int seg;
   const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
                                g.z_max - g.z_min + 2, &seg);
   k_accelerate_tma<S, kStencilRing, kStencilMinBlocks<S>>
       <<<grid, dim3(TX, TY), kStencilRing * AccPlane<S>::kBytes, s>>>(g, seg, dt_ptr, maps,
-                                                                      xvel1, yvel1, zvel1, status);
+                                                                      xvel1, yvel1, zvel1, xvel0, yvel0, xh, status);
 }
 
 template <class S>
@@ -2792,14 +2880,14 @@ void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, co
                          const typename S::ene_t* energy0, typename S::ene_t* energy1,
                          const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                         typename S::vf_t* vol_flux_z, int* status) {
+                         typename S::vf_t* vol_flux_z, bool xh, int* status) {
   int seg;
   const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
                                g.z_max - g.z_min + 2, &seg);
   k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>
       <<<grid, dim3(TX, TY), kStencilRing * FluxPlane<S>::kBytes, s>>>(
           g, seg, dt_ptr, maps, density0, density1, energy0, energy1, pressure, viscosity,
-          vol_flux_x, vol_flux_y, vol_flux_z, status);
+          vol_flux_x, vol_flux_y, vol_flux_z, xh, status);
 }
 
 template <class S>
@@ -2808,14 +2896,15 @@ void launch_acc_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, co
                          typename S::ene_t* energy1, typename S::vel_t* xvel1,
                          typename S::vel_t* yvel1, typename S::vel_t* zvel1,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                         typename S::vf_t* vol_flux_z, int* status) {
+                         typename S::vf_t* vol_flux_z, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
+                           bool xh, int* status) {
   int seg;
   const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX - 1) / (TX - 1),
                                (g.y_max + 1 - g.y_min + TY - 1) / (TY - 1), g.z_max - g.z_min + 2, &seg);
   k_acc_flux_tma<S, TY, kStencilRing, 3>
       <<<grid, dim3(TX, TY), kAccFluxSmem<S>, s>>>(g, seg, dt_ptr, maps, density1, energy0, energy1,
                                                      xvel1, yvel1, zvel1, vol_flux_x, vol_flux_y,
-                                                     vol_flux_z, status);
+                                                     vol_flux_z, xvel0, yvel0, xh, status);
 }
 
 template <class S>
@@ -2877,14 +2966,15 @@ template <class S>
 void launch_mom_vel_tma(const Geom& g, cudaStream_t s, int dir, const VelMaps& maps,
                         const GeomArrays& ga, const typename S::nd_t* node_flux,
                         const typename S::nd_t* node_mass_pre, typename S::vel_t* const* vel_in,
-                        typename S::vel_t* const* vel_out, const Level0<S>& level0, int* status) {
+                        typename S::vel_t* const* vel_out, const Level0<S>& level0, bool xh,
+                        int* status) {
   auto go = [&](auto kern, const MarchRange& r) {
     int seg;
     const dim3 grid = plane_grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY,
                                  r.phi - r.plo + 1, &seg);
     kern<<<grid, dim3(TX, TY), kVelRing * VelPlane<S>::kBytes, s>>>(
         g, seg, ga, maps, node_flux, node_mass_pre, vel_in[0], vel_in[1], vel_in[2],
-        vel_out[0], vel_out[1], vel_out[2], level0, status);
+        vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
   };
   if (dir == 2) go(k_mom_vel_tma<S, 2, kVelRing, kVelMinBlocks<S>>, mom_vel_range<2>(g));
   else go(k_mom_vel_tma<S, 3, kVelRing, kVelMinBlocks<S>>, mom_vel_range<3>(g));
@@ -2913,13 +3003,14 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                            const typename S::ene_t* e_in, typename S::rho_t* d_out,
                            typename S::ene_t* e_out, const typename S::vf_t* vfx,
                            const typename S::vf_t* vfy, const typename S::vf_t* vfz,
-                           typename S::mf_t* mass_flux, const Level0<S>& level0, int* status) {
+                           typename S::mf_t* mass_flux, const Level0<S>& level0, bool xh,
+                           int* status) {
   auto go = [&](auto kern, int bytes, const MarchRange& r, int pcells) {
     int seg;
     const dim3 grid = plane_grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY, pcells, &seg);
     kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, seg, ga, maps, d_in, e_in,
                                                           d_out, e_out, vfx, vfy, vfz, mass_flux,
-                                                          level0, status);
+                                                          level0, xh, status);
   };
   const int ny = g.y_max - g.y_min + 1, nz = g.z_max - g.z_min + 1;
   if (dir == 2) {
@@ -2946,34 +3037,36 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
   template void launch_cell_sweep_tma<S>(const Geom&, cudaStream_t, int, int, const CellMaps&,   \
                                          const GeomArrays&, const S::rho_t*, const S::ene_t*,    \
                                          S::rho_t*, S::ene_t*, const S::vf_t*, const S::vf_t*,   \
-                                         const S::vf_t*, S::mf_t*, const Level0<S>&, int*);      \
+                                         const S::vf_t*, S::mf_t*, const Level0<S>&, bool, int*); \
   template void launch_mom_vel_tma<S>(const Geom&, cudaStream_t, int, const VelMaps&,            \
                                       const GeomArrays&, const S::nd_t*, const S::nd_t*,         \
-                                      S::vel_t* const*, S::vel_t* const*, const Level0<S>&, int*); \
+                                      S::vel_t* const*, S::vel_t* const*, const Level0<S>&, bool, int*); \
   template void launch_mom_node_tma<S>(const Geom&, cudaStream_t, int, int, const NodeMaps&,     \
                                        S::nd_t*, S::nd_t*, S::nd_t*, int*);                      \
   template bool cell_sweep_x_tma_prepare<S>();                                                   \
   template void launch_cell_sweep_x_tma<S>(const Geom&, cudaStream_t, int, const CellXMaps&,     \
                                            const GeomArrays&, S::rho_t*, S::ene_t*, S::mf_t*,    \
-                                           const Level0<S>&, int*);                              \
+                                           const Level0<S>&, bool, int*);                        \
   template void launch_pdv_predict_eos_tma<S>(const Geom&, cudaStream_t, const double*,         \
-                                              const PdvMaps&, S::cs_t*, int*);                   \
+                                              const PdvMaps&, S::cs_t*, bool, int*);             \
   template void launch_mom_x_tma<S>(const Geom&, cudaStream_t, int, const MomXMaps&,             \
-                                    const GeomArrays&, S::vel_t* const*, const Level0<S>&, int*); \
+                                    const GeomArrays&, S::vel_t* const*, const Level0<S>&, bool, int*); \
   template void launch_visc_dt_tma<S>(const Geom&, cudaStream_t, const ViscMaps&, const GeomArrays&, \
                                       double, double, double, double, double, double, S::cs_t*,  \
-                                      S::cs_t*, S::cs_t*, unsigned long long*, int*);
+                                      S::cs_t*, S::cs_t*, unsigned long long*, S::rho_t*, S::ene_t*, bool, int*);
 INST_TMA(F64)
 INST_TMA(F32Mixed)
-template void launch_acc_flux_tma<F64>(const Geom&, cudaStream_t, const double*, const AccMaps&, 
-                                       F64::rho_t*, const F64::ene_t*, F64::ene_t*, F64::vel_t*,         
-                                       F64::vel_t*, F64::vel_t*, F64::vf_t*, F64::vf_t*, F64::vf_t*, int*);
-template void launch_accelerate_tma<F32Mixed>(const Geom&, cudaStream_t, const double*,               
-                                         const AccMaps&, F32Mixed::vel_t*, F32Mixed::vel_t*, F32Mixed::vel_t*, int*); 
-template void launch_pdv_flux_tma<F32Mixed>(const Geom&, cudaStream_t, const double*, const FluxMaps&, 
-                                       const F32Mixed::rho_t*, F32Mixed::rho_t*, const F32Mixed::ene_t*, F32Mixed::ene_t*,   
-                                       const F32Mixed::cs_t*, const F32Mixed::cs_t*, F32Mixed::vf_t*, F32Mixed::vf_t*,       
-                                       F32Mixed::vf_t*, int*);                                          
+template void launch_acc_flux_tma<F64>(const Geom&, cudaStream_t, const double*, const AccMaps&,
+                                       F64::rho_t*, const F64::ene_t*, F64::ene_t*, F64::vel_t*,
+                                       F64::vel_t*, F64::vel_t*, F64::vf_t*, F64::vf_t*, F64::vf_t*, F64::vel_t*,
+                                       F64::vel_t*, bool, int*);
+template void launch_accelerate_tma<F32Mixed>(const Geom&, cudaStream_t, const double*,
+                                         const AccMaps&, F32Mixed::vel_t*, F32Mixed::vel_t*, F32Mixed::vel_t*,
+                                         F32Mixed::vel_t*, F32Mixed::vel_t*, bool, int*);
+template void launch_pdv_flux_tma<F32Mixed>(const Geom&, cudaStream_t, const double*, const FluxMaps&,
+                                       const F32Mixed::rho_t*, F32Mixed::rho_t*, const F32Mixed::ene_t*, F32Mixed::ene_t*,
+                                       const F32Mixed::cs_t*, const F32Mixed::cs_t*, F32Mixed::vf_t*, F32Mixed::vf_t*,
+                                       F32Mixed::vf_t*, bool, int*);
 
 void launch_wait_selftest(cudaStream_t s, long long cycles, int* status) {
   k_wait_selftest<<<1, 32, 0, s>>>(cycles, status);

@@ -58,7 +58,7 @@ bool mom_x_tma_prepare();
 template <class S>
 void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
-                      const Level0<S>& level0, int* status);
+                      const Level0<S>& level0, bool xh, int* status);
 
 // The maps of the PdV predictor + EOS (node velocities 9 rows, density0,
 // energy0, pressure, viscosity 8 rows), of accelerate, alone or with the
@@ -82,25 +82,28 @@ template <class S>
 bool stencils_tma_prepare();
 template <class S>
 void launch_pdv_predict_eos_tma(const Geom& g, cudaStream_t s, const double* dt_ptr,
-                                const PdvMaps& maps, typename S::cs_t* pressure, int* status);
+                                const PdvMaps& maps, typename S::cs_t* pressure, bool xh,
+                                int* status);
 template <class S>
 void launch_accelerate_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
                            typename S::vel_t* xvel1, typename S::vel_t* yvel1,
-                           typename S::vel_t* zvel1, int* status);
+                           typename S::vel_t* zvel1, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
+                           bool xh, int* status);
 template <class S>
 void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const FluxMaps& maps,
                          const typename S::rho_t* density0, typename S::rho_t* density1,
                          const typename S::ene_t* energy0, typename S::ene_t* energy1,
                          const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                         typename S::vf_t* vol_flux_z, int* status);
+                         typename S::vf_t* vol_flux_z, bool xh, int* status);
 template <class S>
 void launch_acc_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
                          typename S::rho_t* density1, const typename S::ene_t* energy0,
                          typename S::ene_t* energy1, typename S::vel_t* xvel1,
                          typename S::vel_t* yvel1, typename S::vel_t* zvel1,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                         typename S::vf_t* vol_flux_z, int* status);
+                         typename S::vf_t* vol_flux_z, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
+                           bool xh, int* status);
 
 // The maps of the drop-in PdV (clover_pdv_kernel over the caller's arrays):
 // time level 0 and (corrector) time level 1 node velocities and yarea, 9
@@ -165,7 +168,7 @@ template <class S>
 void launch_cell_sweep_x_tma(const Geom& g, cudaStream_t s, int sweep, const CellXMaps& maps,
                              const GeomArrays& ga, typename S::rho_t* d_out,
                              typename S::ene_t* e_out, typename S::mf_t* mass_flux_x,
-                             const Level0<S>& level0, int* status);
+                             const Level0<S>& level0, bool xh, int* status);
 
 // The bounded wait of the staged kernels made to run out (a barrier phase
 // nothing completes, cycles SM clocks at most), CLOVER_STATUS_TIMEOUT or'd
@@ -202,7 +205,8 @@ template <class S>
 void launch_mom_vel_tma(const Geom& g, cudaStream_t s, int dir, const VelMaps& maps,
                         const GeomArrays& ga, const typename S::nd_t* node_flux,
                         const typename S::nd_t* node_mass_pre, typename S::vel_t* const* vel_in,
-                        typename S::vel_t* const* vel_out, const Level0<S>& level0, int* status);
+                        typename S::vel_t* const* vel_out, const Level0<S>& level0, bool xh,
+                        int* status);
 
 // The maps of the staged y/z cell sweep: density1 and energy1 of the input
 // buffer, the sweep direction's volume flux (8 rows from c0), vol_flux_x (8
@@ -222,7 +226,8 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                            const typename S::ene_t* e_in, typename S::rho_t* d_out,
                            typename S::ene_t* e_out, const typename S::vf_t* vfx,
                            const typename S::vf_t* vfy, const typename S::vf_t* vfz,
-                           typename S::mf_t* mass_flux, const Level0<S>& level0, int* status);
+                           typename S::mf_t* mass_flux, const Level0<S>& level0, bool xh,
+                           int* status);
 
 // The maps of a chunk's velocities (time level 0), density0 and energy0.
 template <class S>
@@ -242,7 +247,8 @@ void launch_visc_dt_tma(const Geom& g, cudaStream_t s, const ViscMaps& maps, con
                         double g_small, double dtc_safe, double dtu_safe, double dtv_safe,
                         double dtw_safe, double dtdiv_safe, typename S::cs_t* pressure,
                         typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
-                        unsigned long long* min_key, int* status);
+                        unsigned long long* min_key, typename S::rho_t* density0,
+                        typename S::ene_t* energy0, bool xh, int* status);
 
 // Bytes of one box.
 template <class T>
