@@ -938,11 +938,8 @@ void clover_update_halo_kernel(const int* x_min, const int* x_max, const int* y_
     else if (i == 14 || i == 17) hf.f[i] = YF(host[i]);
     else hf.f[i] = ZF(host[i]);
   }
-  // one launch where the face passes compose and no array stands for two fields
   bool composed = halo_composes(g);
   for (int f = 0; f < 6; f++) composed = composed && ext[f];
-  for (int i = 0; i < 19; i++)
-    for (int q = 0; q < i; q++) composed = composed && (!hf.f[i] || hf.f[i] != hf.f[q]);
   launch_update_halo<F64>(g, c.stream, hf, fields, *depth, ext, composed);
   check_launch("update_halo");
 }

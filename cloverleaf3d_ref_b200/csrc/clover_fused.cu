@@ -111,9 +111,10 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
     typename S::cs_t* __restrict__ pressure, typename S::cs_t* __restrict__ viscosity,
     typename S::cs_t* __restrict__ soundspeed,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
-    const typename S::vel_t* __restrict__ zvel0, unsigned long long* __restrict__ min_key, bool xh) {
+    const typename S::vel_t* __restrict__ zvel0, unsigned long long* __restrict__ min_key, bool xh_faces) {
   __shared__ unsigned long long wmin[BX * BY / 32];
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   // viscosity and dt criteria in the policy's arithmetic (FP64, or FP32 in
   // the mixed path); the minimum folds as a double key
   using A = typename S::arith_t;
@@ -301,8 +302,9 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 6 : 8) k_pdv_predict_eos(M
     GeomArrays ga, const typename S::rho_t* __restrict__ density0,
     const typename S::ene_t* __restrict__ energy0, typename S::cs_t* __restrict__ pressure,
     const typename S::cs_t* __restrict__ viscosity, const typename S::vel_t* __restrict__ xvel0,
-    const typename S::vel_t* __restrict__ yvel0, const typename S::vel_t* __restrict__ zvel0, bool xh) {
+    const typename S::vel_t* __restrict__ yvel0, const typename S::vel_t* __restrict__ zvel0, bool xh_faces) {
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const Box b = interior(g);
   int j, k;
   if (!tile_jk<M>(b, t, j, k)) return;
@@ -372,8 +374,9 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
     const typename S::vel_t* __restrict__ xvel1, const typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ yvel1, const typename S::vel_t* __restrict__ zvel0,
     const typename S::vel_t* __restrict__ zvel1, typename S::vf_t* __restrict__ vol_flux_x,
-    typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z, bool xh) {
+    typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z, bool xh_faces) {
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const Box b = nodes(g);
   int j, k;
   if (!tile_jk<M>(b, t, j, k)) return;
@@ -513,8 +516,9 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 4 : (sizeof(typename S::ar
     typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
     const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
     const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-    Level0<S> lz, bool xh) {
+    Level0<S> lz, bool xh_faces) {
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const int lane = threadIdx.x;
   const int c = g.x_min - 2 + t.x * 28 + lane;
   const int k = g.y_min + t.y * BY + threadIdx.y;
@@ -767,8 +771,9 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && !
     const typename S::nd_t* __restrict__ node_mass_pre, const typename S::vel_t* __restrict__ u_in,
     const typename S::vel_t* __restrict__ v_in, const typename S::vel_t* __restrict__ w_in,
     typename S::vel_t* __restrict__ u_out, typename S::vel_t* __restrict__ v_out,
-    typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh) {
+    typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh_faces) {
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const MarchRange r = mom_vel_range<DIR>(g);
   const int jlo = r.jlo, jhi = r.jhi, clo = r.clo, chi = r.chi, plo = r.plo, phi = r.phi;
   const int seg = m.seg;
@@ -863,10 +868,11 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && M
     typename S::rho_t* __restrict__ density1, typename S::ene_t* __restrict__ energy1,
     const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
     const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-    Level0<S> lz, bool xh) {
+    Level0<S> lz, bool xh_faces) {
   // old density/energy of cells c1+1, c1+2 of each thread's segment
   __shared__ double s_end[4][BY][BX];
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const MarchRange r = cell_sweep_range<DIR>(g);
   // one chunk: 32 columns j of one cross index c per block; a batch: 32
   // consecutive columns of the deck's (j, c) plane in row order
@@ -1015,8 +1021,9 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat || sizeof(typename S::arith_
     const typename S::vel_t* __restrict__ u_in, const typename S::vel_t* __restrict__ v_in,
     const typename S::vel_t* __restrict__ w_in, typename S::vel_t* __restrict__ u_out,
     typename S::vel_t* __restrict__ v_out, typename S::vel_t* __restrict__ w_out,
-    Level0<S> lz, bool xh) {
+    Level0<S> lz, bool xh_faces) {
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const int seg = m.seg;
   const int lane = threadIdx.x;
   const int j = g.x_min - 2 + t.x * 29 + lane;  // node of this lane

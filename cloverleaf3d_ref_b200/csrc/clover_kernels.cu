@@ -398,8 +398,9 @@ __global__ void __launch_bounds__(BX * BY, UM ? 5 : 4) k_accelerate(M m, double 
     const typename S::cs_t* __restrict__ pressure, const typename S::cs_t* __restrict__ viscosity,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ zvel0, typename S::vel_t* __restrict__ xvel1,
-    typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1, bool xh) {
+    typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1, bool xh_faces) {
   m.run([&](const Geom& g, const Tile& t) {
+  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   TILE_THREAD(nodes(g), t);
   const double dt = dt_ptr ? dt_ptr[(long long)t.d * kScalarStride] : dt_val;
 #define DV(a, bb, c) (L(density0, j + (a), k + (bb), l + (c)) * (UM ? g.vol : E(ga.volume, j + (a), k + (bb), l + (c))))
@@ -1320,7 +1321,7 @@ struct HaloLaunch {
   int elem_bytes[19];
   HaloRule rule[19];
   int nfields;
-  int ids[19];
+  bool serial;  // one array stands for two fields: its copies in the fields' order
 };
 
 template <int AX, class M>
@@ -1336,9 +1337,11 @@ __global__ void k_halo(M m, HaloLaunch h, int depth, int do_low, int do_high) {
                       maxs[tb] + 1 + depth, 0, 0}, t, a, bb))
     return;
   const int n = maxs[AX];
-  for (int fi = 0; fi < h.nfields; fi++) {
+  // one chunk: a field per tile.z unless one array stands for two fields
+  const bool side_by_side = !M::kFlat && !h.serial;
+  const int f1 = side_by_side ? t.z + 1 : h.nfields;
+  for (int fi = side_by_side ? t.z : 0; fi < f1; fi++) {
     const HaloRule r = h.rule[fi];
-    const int id = h.ids[fi];
     for (int side = 0; side < 2; side++) {
       if (side == 0 ? !do_low : !do_high) continue;
       const signed char* ext = side == 0 ? r.ext_lo : r.ext_hi;
@@ -1360,7 +1363,6 @@ __global__ void k_halo(M m, HaloLaunch h, int depth, int do_low, int do_high) {
         }
       }
     }
-    (void)id;
   }
   });
 }
@@ -1527,12 +1529,19 @@ __device__ __forceinline__ void halo_one(const Geom& g, const HaloOne& h, int fi
 template <int D, bool X, class M>
 __global__ void __launch_bounds__(BX * BY) k_halo_one(M m, const __grid_constant__ HaloOne h) {
   m.run([&](const Geom& g, const Tile& t) {
-    if (h.bytes[t.y] == 8) halo_one<D, X, double>(g, h, t.y, t.x);
-    else halo_one<D, X, float>(g, h, t.y, t.x);
+    // one chunk: a field per tile (the most blocks on a small grid); a batch: all
+    // fields of a tile in turn (512 decks of 16..48 cells would be 160000 items
+    // otherwise, each the latency of its deck and one field)
+    const int f1 = M::kFlat ? h.n : t.y + 1;
+#pragma unroll 1
+    for (int f = M::kFlat ? 0 : t.y; f < f1; f++) {
+      if (h.bytes[f] == 8) halo_one<D, X, double>(g, h, f, t.x);
+      else halo_one<D, X, float>(g, h, f, t.x);
+    }
   });
 }
 
-// tiles of k_halo_one; aux = fields
+// tiles of k_halo_one; aux = fields (one chunk)
 template <int D, bool X>
 dim3 grid_halo_one(const Geom& g, int fields) {
   const int nx = g.x_max, ny = g.y_max, nz = g.z_max;
@@ -1541,6 +1550,8 @@ dim3 grid_halo_one(const Geom& g, int fields) {
                   (X ? ((ny + 1 + 31) / 32) * ((nz + 1 + 7) / 8) : 0),
               fields, 1);
 }
+template <int D, bool X>
+dim3 grid_halo_one_batch(const Geom& g, int) { return grid_halo_one<D, X>(g, 1); }
 
 // tasks of k_halo_x in blocks of BX * BY; aux = tasks per row (fields * 2 * depth)
 dim3 grid_halo_x_tasks(const Geom& g, int per_row, int depth) {
@@ -1551,20 +1562,23 @@ template <int D>
 dim3 grid_halo_x(const Geom& g, int per_row) { return grid_halo_x_tasks(g, per_row, D); }
 
 // tile grid of the halo update of the faces normal to AX (32 x 8 tiles over
-// the two tangential axes, each extended by depth)
+// the two tangential axes, each extended by depth); aux = depth, and for one
+// chunk the fields side by side in its upper bits
 template <int AX>
-dim3 grid_halo_flat(const Geom& g, int depth) {
+dim3 grid_halo_flat(const Geom& g, int aux) {
+  const int depth = aux & 0xff;
   const int mins[3] = {g.x_min, g.y_min, g.z_min}, maxs[3] = {g.x_max, g.y_max, g.z_max};
   const int ta = AX == 0 ? 1 : 0, tb = AX == 2 ? 1 : 2;
   return grid_flat(Box{mins[ta] - depth, maxs[ta] + 1 + depth, mins[tb] - depth,
                        maxs[tb] + 1 + depth, 0, 0});
 }
 template <int AX>
-dim3 grid_halo(const Geom& g, int depth) {
+dim3 grid_halo(const Geom& g, int aux) {
+  const int depth = aux & 0xff, fields = aux >> 8;
   const int mins[3] = {g.x_min, g.y_min, g.z_min}, maxs[3] = {g.x_max, g.y_max, g.z_max};
   const int ta = AX == 0 ? 1 : 0, tb = AX == 2 ? 1 : 2;
   const int na = maxs[ta] - mins[ta] + 2 + 2 * depth, nb = maxs[tb] - mins[tb] + 2 + 2 * depth;
-  return dim3((na + 31) / 32, (nb + 7) / 8, 1);
+  return dim3((na + 31) / 32, (nb + 7) / 8, fields > 0 ? fields : 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1904,7 +1918,12 @@ void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, c
   // field id -> (kind, component)
   static const int kind[19] = {0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2};
   static const int comp[19] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 2, 2, 0, 1, 2, 0, 1, 2};
-  if (composed) {
+  // an array given for two fields: the copies keep the fields' order
+  bool alias = false;
+  for (int a = 0; a < 19; a++)
+    for (int b = 0; b < a; b++)
+      alias = alias || (fields[a] == 1 && fields[b] == 1 && f.f[a] && f.f[a] == f.f[b]);
+  if (composed && !alias) {
     HaloOne h{};
     for (int id = 1; id <= 19; id++) {
       if (fields[id - 1] != 1) continue;
@@ -1921,8 +1940,8 @@ void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, c
     auto go = [&](auto d, auto x) {
       constexpr int D = decltype(d)::value;
       constexpr bool X = decltype(x)::value;
-      launch_mapped(tg, s, key, grid_halo_one<D, X>, h.n, false, blk, k_halo_one<D, X, MapSingle>,
-                    k_halo_one<D, X, MapBatchFree>, h);
+      launch_mapped2(tg, s, key, grid_halo_one<D, X>, grid_halo_one_batch<D, X>, h.n, false, blk,
+                     k_halo_one<D, X, MapSingle>, k_halo_one<D, X, MapBatchFree>, h);
     };
     using One = std::integral_constant<int, 1>;
     using Two = std::integral_constant<int, 2>;
@@ -1941,17 +1960,18 @@ void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, c
     if (!do_low && !do_high) continue;
     HaloLaunch h;
     h.nfields = 0;
+    h.serial = alias;
     for (int id = 1; id <= 19; id++) {
       if (fields[id - 1] != 1) continue;
       const int i = h.nfields++;
       h.f[i] = f.f[id - 1];
-      h.ids[i] = id;
       h.elem_bytes[i] = elem_bytes_of<S>(id);
       h.rule[i] = make_rule(kind[id - 1], comp[id - 1], ax, id);
     }
     if (h.nfields == 0) return;
     const dim3 blk(32, 8);
     const unsigned key = kKeyHalo | (unsigned)(ax << 4) | (unsigned)depth;
+    const int aux = depth | (tg.plan || alias ? 0 : h.nfields << 8);
     if (ax == 0) {
       const int per_row = h.nfields * 2 * depth;
       // the schedule depends on the depth as well as the tasks per row (a
@@ -1965,10 +1985,10 @@ void launch_update_halo(const Target& tg, cudaStream_t s, const HaloFields& f, c
                       k_halo_x<MapBatchFree>, h, depth, do_low, do_high);
     }
     else if (ax == 1)
-      launch_mapped2(tg, s, key, grid_halo<1>, grid_halo_flat<1>, depth, false, blk,
+      launch_mapped2(tg, s, key, grid_halo<1>, grid_halo_flat<1>, aux, false, blk,
                      k_halo<1, MapSingle>, k_halo<1, MapBatchFree>, h, depth, do_low, do_high);
     else
-      launch_mapped2(tg, s, key, grid_halo<2>, grid_halo_flat<2>, depth, false, blk,
+      launch_mapped2(tg, s, key, grid_halo<2>, grid_halo_flat<2>, aux, false, blk,
                      k_halo<2, MapSingle>, k_halo<2, MapBatchFree>, h, depth, do_low, do_high);
   }
 }

@@ -328,7 +328,8 @@ void launch_field_summary(const Geom& g, cudaStream_t s, const double* volume,
 // update_halo_kernel: fields[i] != 0 selects field id i+1. Element size of
 // every selected field comes from the policy S. composed: every face is
 // external and every deck has three or more cells per axis from index 1
-// (halo_composes), so that one launch writes all faces, and the same halo into
+// (halo_composes), so that one launch writes all faces (unless one array
+// stands for two fields), and the same halo into
 // also's arrays where they are given (without x_faces: the y and z faces only,
 // whose planes and rows reach into the x halo columns); otherwise one pass per axis, in the
 // reference's order, over the external faces.

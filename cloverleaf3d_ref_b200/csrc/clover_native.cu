@@ -20,6 +20,7 @@
 
 #include "clover_batch.h"
 #include "clover_launch.h"
+#include "clover_stencil.cuh"
 #include "clover_tma.cuh"
 #include "clover_visit.h"
 
@@ -826,7 +827,8 @@ struct Chunk : ChunkBase {
     const double n = cells();
     const double R8 = sizeof(R), E8 = sizeof(En), C8 = sizeof(C), V8 = sizeof(V),
                  VF8 = sizeof(VF), MF8 = sizeof(MF), N8 = sizeof(ND);
-    const bool xh = halo_repeat_free;  // the kernels write the x faces' halo of the rows they store
+    // the kernels write the x faces' halo of the rows they store
+    const bool xh = halo_repeat_free && (!plan || kWritesXh<S, true>);
     int vc = ax ? 0 : 1;  // buffer of the velocity pairs at the start of this step
     int cb = ax ? 0 : 1;  // buffer of the density1/energy1 pair at the start of this step
     // timestep.f90:56-126
