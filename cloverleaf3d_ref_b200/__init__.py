@@ -336,9 +336,9 @@ class Chunk:
         lib().clover_chunk_use_fused(self.h, 1 if on else 0)
 
     def use_tma(self, on):
-        """The fused step's stencils staged by bulk-tensor copies (default, one
-        chunk) or their register-marching forms; True if the staged forms are
-        in use."""
+        """The fused step's stencils staged by bulk-tensor copies (the default of
+        a chunk, and of an ensemble whose decks fill the staged tiles) or their
+        register-marching forms; True if the staged forms are in use."""
         return lib().clover_chunk_use_tma(self.h, 1 if on else 0) == 1
 
     @property

@@ -111,10 +111,9 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
     typename S::cs_t* __restrict__ pressure, typename S::cs_t* __restrict__ viscosity,
     typename S::cs_t* __restrict__ soundspeed,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
-    const typename S::vel_t* __restrict__ zvel0, unsigned long long* __restrict__ min_key, bool xh_faces) {
+    const typename S::vel_t* __restrict__ zvel0, unsigned long long* __restrict__ min_key, bool xh) {
   __shared__ unsigned long long wmin[BX * BY / 32];
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   // viscosity and dt criteria in the policy's arithmetic (FP64, or FP32 in
   // the mixed path); the minimum folds as a double key
   using A = typename S::arith_t;
@@ -302,9 +301,8 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 6 : 8) k_pdv_predict_eos(M
     GeomArrays ga, const typename S::rho_t* __restrict__ density0,
     const typename S::ene_t* __restrict__ energy0, typename S::cs_t* __restrict__ pressure,
     const typename S::cs_t* __restrict__ viscosity, const typename S::vel_t* __restrict__ xvel0,
-    const typename S::vel_t* __restrict__ yvel0, const typename S::vel_t* __restrict__ zvel0, bool xh_faces) {
+    const typename S::vel_t* __restrict__ yvel0, const typename S::vel_t* __restrict__ zvel0, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const Box b = interior(g);
   int j, k;
   if (!tile_jk<M>(b, t, j, k)) return;
@@ -374,9 +372,8 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 5 : 8) k_pdv_flux(M m, con
     const typename S::vel_t* __restrict__ xvel1, const typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ yvel1, const typename S::vel_t* __restrict__ zvel0,
     const typename S::vel_t* __restrict__ zvel1, typename S::vf_t* __restrict__ vol_flux_x,
-    typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z, bool xh_faces) {
+    typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const Box b = nodes(g);
   int j, k;
   if (!tile_jk<M>(b, t, j, k)) return;
@@ -516,9 +513,8 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat ? 4 : (sizeof(typename S::ar
     typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
     const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
     const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-    Level0<S> lz, bool xh_faces) {
+    Level0<S> lz, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const int lane = threadIdx.x;
   const int c = g.x_min - 2 + t.x * 28 + lane;
   const int k = g.y_min + t.y * BY + threadIdx.y;
@@ -771,9 +767,8 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && !
     const typename S::nd_t* __restrict__ node_mass_pre, const typename S::vel_t* __restrict__ u_in,
     const typename S::vel_t* __restrict__ v_in, const typename S::vel_t* __restrict__ w_in,
     typename S::vel_t* __restrict__ u_out, typename S::vel_t* __restrict__ v_out,
-    typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh_faces) {
+    typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const MarchRange r = mom_vel_range<DIR>(g);
   const int jlo = r.jlo, jhi = r.jhi, clo = r.clo, chi = r.chi, plo = r.plo, phi = r.phi;
   const int seg = m.seg;
@@ -868,11 +863,10 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 && M
     typename S::rho_t* __restrict__ density1, typename S::ene_t* __restrict__ energy1,
     const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
     const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
-    Level0<S> lz, bool xh_faces) {
+    Level0<S> lz, bool xh) {
   // old density/energy of cells c1+1, c1+2 of each thread's segment
   __shared__ double s_end[4][BY][BX];
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const MarchRange r = cell_sweep_range<DIR>(g);
   // one chunk: 32 columns j of one cross index c per block; a batch: 32
   // consecutive columns of the deck's (j, c) plane in row order
@@ -1021,9 +1015,8 @@ __global__ void __launch_bounds__(BX * BY, M::kFlat || sizeof(typename S::arith_
     const typename S::vel_t* __restrict__ u_in, const typename S::vel_t* __restrict__ v_in,
     const typename S::vel_t* __restrict__ w_in, typename S::vel_t* __restrict__ u_out,
     typename S::vel_t* __restrict__ v_out, typename S::vel_t* __restrict__ w_out,
-    Level0<S> lz, bool xh_faces) {
+    Level0<S> lz, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   const int seg = m.seg;
   const int lane = threadIdx.x;
   const int j = g.x_min - 2 + t.x * 29 + lane;  // node of this lane
@@ -1321,11 +1314,11 @@ void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const Geom
                          typename S::rho_t* density1_out, typename S::ene_t* energy1_out,
                          const typename S::vf_t* vol_flux_x, const typename S::vf_t* vol_flux_y,
                          const typename S::vf_t* vol_flux_z, typename S::mf_t* mass_flux_x,
-                         bool copy_shell, const Level0<S>& level0, bool xh, const CellXMaps* maps,
+                         bool copy_shell, const Level0<S>& level0, bool xh, const PlaneSrc<CellXMaps>* maps,
                          int* status) {
   // pre_vol variant: 0 on sweep 1 (all three flux differences), 1 on sweep 3
-  if (maps && !tg.plan)  // one chunk: planes staged by bulk-tensor copies
-    launch_cell_sweep_x_tma<S>(tg.g, s, sweep, *maps, ga, density1_out, energy1_out, mass_flux_x,
+  if (maps)  // planes staged by bulk-tensor copies
+    launch_cell_sweep_x_tma<S>(tg, s, sweep, *maps, ga, density1_out, energy1_out, mass_flux_x,
                                level0, xh, status);
   else if (sweep == 1)
     launch_mapped(tg, s, kKeyCellSweepX, grid_cell_sweep_x, 0, false, kBlk,
@@ -1356,8 +1349,8 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
                             typename S::wk_t* node_flux, typename S::wk_t* node_mass_post,
                             typename S::wk_t* node_mass_pre, typename S::vel_t* const* vel_in,
                             typename S::vel_t* const* vel_out, bool copy_shell,
-                            const Level0<S>& level0, bool xh, const MomXMaps* x_maps, int* status,
-                            const NodeMaps* node_maps, const VelMaps* vel_maps) {
+                            const Level0<S>& level0, bool xh, const PlaneSrc<MomXMaps>* x_maps, int* status,
+                            const PlaneSrc<NodeMaps>* node_maps, const PlaneSrc<VelMaps>* vel_maps) {
   // the node arrays of the y/z sweeps live in three work arrays, as nd_t
   using ND = typename S::nd_t;
   static_assert(sizeof(ND) <= sizeof(typename S::wk_t), "node arrays fit the work arrays");
@@ -1370,15 +1363,15 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
   auto node_vel = [&](auto dir_c, auto var) {
     constexpr int D = decltype(dir_c)::value, V = decltype(var)::value;
     // node pass then velocity pass, each marching along the sweep axis in segments
-    if (node_maps && !tg.plan)
-      launch_mom_node_tma<S>(tg.g, s, D, V, *node_maps, nd_flux, nd_post, nd_pre, status);
+    if (node_maps)
+      launch_mom_node_tma<S>(tg, s, D, V, *node_maps, nd_flux, nd_post, nd_pre, status);
     else
       launch_mapped(tg, s, kKeyMomNode | D | (V << 4), grid_mom_node<D>, kMarchSeg, true, kBlk,
                     k_mom_node_march<S, D, V, MapSingle>, k_mom_node_march<S, D, V, MapBatchFree>,
                     ga, D == 2 ? mass_flux_y : mass_flux_z, density1, vol_flux_x, vol_flux_y,
                     vol_flux_z, nd_flux, nd_post, nd_pre);
-    if (vel_maps && !tg.plan)
-      launch_mom_vel_tma<S>(tg.g, s, D, *vel_maps, ga, nd_flux, nd_pre, vel_in, vel_out, level0,
+    if (vel_maps)
+      launch_mom_vel_tma<S>(tg, s, D, *vel_maps, ga, nd_flux, nd_pre, vel_in, vel_out, level0,
                             xh, status);
     else
       launch_mapped2(tg, s, kKeyMomVel3 | D, grid_mom_vel<D>, grid_mom_vel_flat<D>, kMarchSeg,
@@ -1388,9 +1381,9 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
   };
   using I2 = std::integral_constant<int, 2>;
   using I3 = std::integral_constant<int, 3>;
-  if (dir == 1 && x_maps && !tg.plan) {
+  if (dir == 1 && x_maps) {
     // one pass, its planes staged in shared memory
-    launch_mom_x_tma<S>(tg.g, s, sweep, *x_maps, ga, vel_out, level0, xh, status);
+    launch_mom_x_tma<S>(tg, s, sweep, *x_maps, ga, vel_out, level0, xh, status);
   } else if (dir == 1) {
     // one pass for the three velocities
     auto sweep_x = [&](auto var) {
@@ -1444,14 +1437,14 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
   template void launch_advec_cell_x<S>(const Target&, cudaStream_t, int, const GeomArrays&,      \
                                        const S::rho_t*, const S::ene_t*, S::rho_t*, S::ene_t*,  \
                                        const S::vf_t*, const S::vf_t*, const S::vf_t*,          \
-                                       S::mf_t*, bool, const Level0<S>&, bool, const CellXMaps*, int*); \
+                                       S::mf_t*, bool, const Level0<S>&, bool, const PlaneSrc<CellXMaps>*, int*); \
   template void launch_advec_mom_fused<S>(const Target&, cudaStream_t, int, int, int, double,    \
                                           const GeomArrays&, const S::rho_t*, const S::mf_t*,  \
                                           const S::mf_t*, const S::mf_t*, const S::vf_t*,      \
                                           const S::vf_t*, const S::vf_t*, S::wk_t*, S::wk_t*,  \
                                           S::wk_t*, S::vel_t* const*, S::vel_t* const*, bool,  \
-                                          const Level0<S>&, bool, const MomXMaps*, int*,      \
-                                          const NodeMaps*, const VelMaps*);
+                                          const Level0<S>&, bool, const PlaneSrc<MomXMaps>*, int*, \
+                                          const PlaneSrc<NodeMaps>*, const PlaneSrc<VelMaps>*);
 
 INSTF(F64)
 INSTF(F32Mixed)

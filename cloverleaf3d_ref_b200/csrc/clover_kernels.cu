@@ -398,9 +398,8 @@ __global__ void __launch_bounds__(BX * BY, UM ? 5 : 4) k_accelerate(M m, double 
     const typename S::cs_t* __restrict__ pressure, const typename S::cs_t* __restrict__ viscosity,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ zvel0, typename S::vel_t* __restrict__ xvel1,
-    typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1, bool xh_faces) {
+    typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
-  const bool xh = kWritesXh<S, M::kFlat> && xh_faces;
   TILE_THREAD(nodes(g), t);
   const double dt = dt_ptr ? dt_ptr[(long long)t.d * kScalarStride] : dt_val;
 #define DV(a, bb, c) (L(density0, j + (a), k + (bb), l + (c)) * (UM ? g.vol : E(ga.volume, j + (a), k + (bb), l + (c))))

@@ -107,7 +107,8 @@ enum : unsigned {
   kKeyCellSweepX = 8u << 8, kKeyCellShell = 9u << 8, kKeyCellSweep = 10u << 8,
   kKeyMomSweepX = 11u << 8, kKeyMomNode = 12u << 8, kKeyMomVel3 = 13u << 8,
   kKeyShellCopy = 14u << 8, kKeySummary = 15u << 8, kKeyAccelerate = 16u << 8,
-  kKeyHaloX = 17u << 8
+  kKeyHaloX = 17u << 8,
+  kKeyStaged = 1u << 16  // with the key of the register form: the staged form over a batch
 };
 
 // Storage policy: FP64 everywhere (the drop-in / parity path).
@@ -405,6 +406,8 @@ void launch_advec_cell_fused(const Target& tg, cudaStream_t s, int advect_x, int
 // outside the interior (left out where a depth-2 halo update of density1 and
 // energy1 follows, which rewrites all of them from the interior).
 struct CellXMaps;  // clover_tma.cuh
+template <class Maps>
+struct PlaneSrc;
 template <class S>
 void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const GeomArrays& ga,
                          const typename S::rho_t* density1_in, const typename S::ene_t* energy1_in,
@@ -412,7 +415,7 @@ void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const Geom
                          const typename S::vf_t* vol_flux_x, const typename S::vf_t* vol_flux_y,
                          const typename S::vf_t* vol_flux_z, typename S::mf_t* mass_flux_x,
                          bool copy_shell, const Level0<S>& level0, bool xh,
-                         const CellXMaps* maps = nullptr, int* status = nullptr);
+                         const PlaneSrc<CellXMaps>* maps = nullptr, int* status = nullptr);
 // All three velocities of one sweep; vel_in/vel_out are the two buffers of
 // each velocity pair, and with copy_shell the shell outside [min,max+1]^3 is
 // copied across (left out where a depth-2 halo update of the velocities
@@ -435,9 +438,9 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
                             typename S::wk_t* node_flux, typename S::wk_t* node_mass_post,
                             typename S::wk_t* node_mass_pre, typename S::vel_t* const* vel_in,
                             typename S::vel_t* const* vel_out, bool copy_shell,
-                            const Level0<S>& level0, bool xh, const MomXMaps* x_maps = nullptr,
-                            int* status = nullptr, const NodeMaps* node_maps = nullptr,
-                            const VelMaps* vel_maps = nullptr);
+                            const Level0<S>& level0, bool xh, const PlaneSrc<MomXMaps>* x_maps = nullptr,
+                            int* status = nullptr, const PlaneSrc<NodeMaps>* node_maps = nullptr,
+                            const PlaneSrc<VelMaps>* vel_maps = nullptr);
 
 // Fill every element of an array (size elems after the pad) with a value.
 template <class T>

@@ -165,21 +165,62 @@ struct Chunk : ChunkBase {
   bool advect_x = true;  // start.f90:99
   bool use_graphs = true;
   bool fused = true;  // fused kernels (clover_fused.cu) instead of one kernel per reference pass
-  // one chunk: stencils staged through shared memory by bulk-tensor copies
-  // (clover_tma.cu) where their tensor maps could be made; their
-  // register-marching forms otherwise, and for ensembles
+  // stencils staged through shared memory by bulk-tensor copies (clover_tma.cu)
+  // where their tensor maps could be made; their register-marching forms otherwise
   bool tma = false;
   bool use_tma = true;
-  ViscMaps visc_maps;
   // tensor maps of the arrays the staged kernels read, by (array, box rows
   // and orientation): both buffers of the density1 and velocity pairs occur
   std::map<std::pair<const void*, int>, CUtensorMap> tmaps;
+  const Geom* mg = &g;  // the deck whose part of an array tmap() describes
+  // an ensemble's maps, every deck's, in device memory (null: the driver refused one)
+  std::map<unsigned, void*> deck_maps;
+  // The maps of a staged launch, filled by fill(Maps*) for one deck at a time;
+  // key: the launch and the buffers it reads (ensembles, built on first use
+  // like the schedules). False: the register form runs.
+  template <class Maps, class F>
+  bool maps_for(unsigned key, PlaneSrc<Maps>* src, F fill) {
+    if (!(tma && use_tma)) return false;
+    if (!plan) return fill(&src->one);
+    if (!halo_repeat_free) return false;
+    auto it = deck_maps.find(key);
+    if (it == deck_maps.end()) {
+      if (plan->capturing) {
+        plan->missing = true;
+        return false;
+      }
+      std::vector<Maps> all(nd);
+      bool ok = true;
+      for (int d = 0; d < nd && ok; d++) {
+        mg = &geoms[d];
+        ok = fill(&all[d]);
+      }
+      mg = &g;
+      void* dev = nullptr;
+      if (ok && cudaMalloc(&dev, nd * sizeof(Maps)) != cudaSuccess) {
+        cudaGetLastError();
+        dev = nullptr;
+      }
+      // on the launch's stream, and complete before the host copy goes away
+      if (dev && (cudaMemcpyAsync(dev, all.data(), nd * sizeof(Maps), cudaMemcpyHostToDevice, stream) !=
+                      cudaSuccess ||
+                  cudaStreamSynchronize(stream) != cudaSuccess)) {
+        cudaGetLastError();
+        cudaFree(dev);
+        dev = nullptr;
+      }
+      it = deck_maps.emplace(key, dev).first;
+    }
+    src->decks = (const Maps*)it->second;
+    return it->second != nullptr;
+  }
   bool tmap(const void* base, int elem_bytes, int rows, CUtensorMap* out, bool zrows = false) {
-    const auto key = std::make_pair(base, 2 * rows + (zrows ? 1 : 0));
+    const void* at = (const char*)base + mg->o3 * elem_bytes;
+    const auto key = std::make_pair(at, 2 * rows + (zrows ? 1 : 0));
     auto it = tmaps.find(key);
     if (it == tmaps.end()) {
       CUtensorMap m;
-      if (!encode_plane_map(&m, base, elem_bytes, g, rows, zrows)) return false;
+      if (!encode_plane_map(&m, at, elem_bytes, *mg, rows, zrows)) return false;
       it = tmaps.emplace(key, m).first;
     }
     *out = it->second;
@@ -430,13 +471,13 @@ struct Chunk : ChunkBase {
     }
     ga = GeomArrays{volume, xarea, yarea, zarea, cellx, celly, cellz, celldx, celldy, celldz,
                     vertexx, vertexy, vertexz, vertexdx, vertexdy, vertexdz};
-    // one chunk: the stencils that stage their planes with bulk-tensor copies
-    // get their tensor maps (the arrays they read never move)
-    if (!batched)
-      tma = visc_dt_tma_prepare<S>() && mom_x_tma_prepare<S>() && stencils_tma_prepare<S>() &&
-            mom_node_tma_prepare<S>() && mom_vel_tma_prepare<S>() && cell_sweep_tma_prepare<S>() &&
-            cell_sweep_x_tma_prepare<S>() &&
-            visc_dt_tma_maps<S>(g, xvel0, yvel0, zvel0, density0, energy0, &visc_maps);
+    // the stencils that stage their planes with bulk-tensor copies get their
+    // tensor maps when they first run (the arrays they read never move)
+    tma = visc_dt_tma_prepare<S>() && mom_x_tma_prepare<S>() && stencils_tma_prepare<S>() &&
+          mom_node_tma_prepare<S>() && mom_vel_tma_prepare<S>() && cell_sweep_tma_prepare<S>() &&
+          cell_sweep_x_tma_prepare<S>();
+    use_tma = staged_by_default();
+
     dt_cap = deck.end_step < (1 << 22) ? deck.end_step + 16 : (1 << 22);
     sum_cap = dt_cap / (deck.summary_frequency > 0 ? deck.summary_frequency : dt_cap) + 8;
     int planes = 0;
@@ -475,6 +516,21 @@ struct Chunk : ChunkBase {
     const double dz = (d.zmax - d.zmin) / (double)(float)d.z_cells;
     cell_volume = dx * dy * dz;  // initialise_chunk_kernel.f90:155 (deck 0)
     return initial_state();
+  }
+
+  // Staged forms by default: always for one chunk (plane_seg). Over an ensemble
+  // they leave the lanes of a 32 x 8 tile that a deck does not reach idle, where
+  // the register forms pack a deck's cells: by the share of those tiles' lanes
+  // that hold a cell, ms per step staged / register, 0.22: 0.82 / 0.67 (256
+  // decks of 8..12 cells), 0.38: 1.16 / 0.98 (12..16), 0.46: 1.92 / 2.15 (64 of
+  // 33..36), 0.53: 2.80 / 3.25 (256 of 8..40), 0.78: 8.52 / 11.5 (64 of 24..128).
+  bool staged_by_default() const {
+    if (!plan) return true;
+    double lanes = 0.0;
+    for (const Geom& q : geoms)
+      lanes += 256.0 * ((q.x_max - q.x_min + 32) / 32) * ((q.y_max - q.y_min + 8) / 8) *
+               (q.z_max - q.z_min + 1);
+    return cells() >= 0.42 * lanes;
   }
 
   // start.f90:49-136 for every deck on the device: scalars, geometry,
@@ -828,7 +884,7 @@ struct Chunk : ChunkBase {
     const double R8 = sizeof(R), E8 = sizeof(En), C8 = sizeof(C), V8 = sizeof(V),
                  VF8 = sizeof(VF), MF8 = sizeof(MF), N8 = sizeof(ND);
     // the kernels write the x faces' halo of the rows they store
-    const bool xh = halo_repeat_free && (!plan || kWritesXh<S, true>);
+    const bool xh = halo_repeat_free;
     int vc = ax ? 0 : 1;  // buffer of the velocity pairs at the start of this step
     int cb = ax ? 0 : 1;  // buffer of the density1/energy1 pair at the start of this step
     // timestep.f90:56-126
@@ -842,8 +898,13 @@ struct Chunk : ChunkBase {
     halo({3, 1, 8, 10}, 1, vc, cb, -1, !xh);
     pend("update_halo", 0);
     pbeg();
-    if (tma && use_tma)
-      launch_visc_dt_tma<S>(g, stream, visc_maps, ga, kGSmall, deck.dtc_safe, deck.dtu_safe,
+    PlaneSrc<ViscMaps> visc_m;
+    if (maps_for(kKeyTimestepVisc, &visc_m, [&](ViscMaps* m) {
+          return tmap(xvel0, sizeof(V), 9, &m->u) && tmap(yvel0, sizeof(V), 9, &m->v) &&
+                 tmap(zvel0, sizeof(V), 9, &m->w) && tmap(density0, sizeof(R), 10, &m->d) &&
+                 tmap(energy0, sizeof(En), 10, &m->e);
+        }))
+      launch_visc_dt_tma<S>(tg, stream, visc_m, ga, kGSmall, deck.dtc_safe, deck.dtu_safe,
                             deck.dtv_safe, deck.dtw_safe, deck.dtdiv_safe, pressure, viscosity,
                             soundspeed, &sc->key, density0, energy0, xh, &sc->status);
     else
@@ -857,12 +918,14 @@ struct Chunk : ChunkBase {
     pend("update_halo", 0);
     // PdV.f90:50-107: predictor + EOS on the predicted state; revert is implied
     pbeg();
-    PdvMaps pdv_m;
-    if (tma && use_tma && tmap(xvel0, sizeof(V), 9, &pdv_m.u) && tmap(yvel0, sizeof(V), 9, &pdv_m.v) &&
-        tmap(zvel0, sizeof(V), 9, &pdv_m.w) && tmap(density0, sizeof(R), 8, &pdv_m.d) &&
-        tmap(energy0, sizeof(En), 8, &pdv_m.e) && tmap(pressure, sizeof(C), 8, &pdv_m.p) &&
-        tmap(viscosity, sizeof(C), 8, &pdv_m.q))
-      launch_pdv_predict_eos_tma<S>(g, stream, dtp, pdv_m, pressure, xh, &sc->status);
+    PlaneSrc<PdvMaps> pdv_m;
+    if (maps_for(kKeyPdvPredict, &pdv_m, [&](PdvMaps* m) {
+          return tmap(xvel0, sizeof(V), 9, &m->u) && tmap(yvel0, sizeof(V), 9, &m->v) &&
+                 tmap(zvel0, sizeof(V), 9, &m->w) && tmap(density0, sizeof(R), 8, &m->d) &&
+                 tmap(energy0, sizeof(En), 8, &m->e) && tmap(pressure, sizeof(C), 8, &m->p) &&
+                 tmap(viscosity, sizeof(C), 8, &m->q);
+        }))
+      launch_pdv_predict_eos_tma<S>(tg, stream, dtp, pdv_m, pressure, xh, &sc->status);
     else
       launch_pdv_predict_eos<S>(tg, stream, dtp, ga, density0, energy0, pressure, viscosity, xvel0,
                                 yvel0, zvel0, xh);
@@ -871,16 +934,17 @@ struct Chunk : ChunkBase {
     halo({5}, 1, vc, cb, -1, !xh);
     pend("update_halo", 0);
     pbeg();
-    AccMaps acc_m;
-    const bool acc_tma = tma && use_tma && tmap(density0, sizeof(R), 9, &acc_m.d) &&
-                         tmap(pressure, sizeof(C), 9, &acc_m.p) &&
-                         tmap(viscosity, sizeof(C), 9, &acc_m.q) && tmap(xvel0, sizeof(V), 8, &acc_m.u) &&
-                         tmap(yvel0, sizeof(V), 8, &acc_m.v) && tmap(zvel0, sizeof(V), 8, &acc_m.w);
+    PlaneSrc<AccMaps> acc_m;
+    const bool acc_tma = maps_for(kKeyAccelerate, &acc_m, [&](AccMaps* m) {
+      return tmap(density0, sizeof(R), 9, &m->d) && tmap(pressure, sizeof(C), 9, &m->p) &&
+             tmap(viscosity, sizeof(C), 9, &m->q) && tmap(xvel0, sizeof(V), 8, &m->u) &&
+             tmap(yvel0, sizeof(V), 8, &m->v) && tmap(zvel0, sizeof(V), 8, &m->w);
+    });
     bool fused_flux = false;
     if constexpr (kFusedAccFlux<S>) {
       fused_flux = acc_tma;
       if (fused_flux) {
-        launch_acc_flux_tma<S>(g, stream, dtp, acc_m, rho1(cb), energy0, ene1(cb), vel1(0, vc),
+        launch_acc_flux_tma<S>(tg, stream, dtp, acc_m, rho1(cb), energy0, ene1(cb), vel1(0, vc),
                                vel1(1, vc), vel1(2, vc), vol_flux_x, vol_flux_y, vol_flux_z, xvel0,
                                yvel0, xh, &sc->status);
         pend("accelerate_pdv_flux", n * (2 * R8 + 2 * E8 + 2 * C8 + 6 * V8 + 3 * VF8));
@@ -891,7 +955,7 @@ struct Chunk : ChunkBase {
       if constexpr (!kFusedAccFlux<S>) {
         staged = acc_tma;
         if (staged)
-          launch_accelerate_tma<S>(g, stream, dtp, acc_m, vel1(0, vc), vel1(1, vc), vel1(2, vc),
+          launch_accelerate_tma<S>(tg, stream, dtp, acc_m, vel1(0, vc), vel1(1, vc), vel1(2, vc),
                                    xvel0, yvel0, xh, &sc->status);
       }
       if (!staged)
@@ -901,14 +965,14 @@ struct Chunk : ChunkBase {
       pbeg();
       staged = false;
       if constexpr (!kFusedAccFlux<S>) {
-        FluxMaps flux_m;
-        staged = tma && use_tma && tmap(xvel0, sizeof(V), 9, &flux_m.u0) &&
-                 tmap(yvel0, sizeof(V), 9, &flux_m.v0) && tmap(zvel0, sizeof(V), 9, &flux_m.w0) &&
-                 tmap(vel1(0, vc), sizeof(V), 9, &flux_m.u1) &&
-                 tmap(vel1(1, vc), sizeof(V), 9, &flux_m.v1) &&
-                 tmap(vel1(2, vc), sizeof(V), 9, &flux_m.w1);
+        PlaneSrc<FluxMaps> flux_m;
+        staged = maps_for(kKeyPdvFlux | (unsigned)vc, &flux_m, [&](FluxMaps* m) {
+          return tmap(xvel0, sizeof(V), 9, &m->u0) && tmap(yvel0, sizeof(V), 9, &m->v0) &&
+                 tmap(zvel0, sizeof(V), 9, &m->w0) && tmap(vel1(0, vc), sizeof(V), 9, &m->u1) &&
+                 tmap(vel1(1, vc), sizeof(V), 9, &m->v1) && tmap(vel1(2, vc), sizeof(V), 9, &m->w1);
+        });
         if (staged)
-          launch_pdv_flux_tma<S>(g, stream, dtp, flux_m, density0, rho1(cb), energy0, ene1(cb),
+          launch_pdv_flux_tma<S>(tg, stream, dtp, flux_m, density0, rho1(cb), energy0, ene1(cb),
                                  pressure, viscosity, vol_flux_x, vol_flux_y, vol_flux_z, xh,
                                  &sc->status);
       }
@@ -942,8 +1006,10 @@ struct Chunk : ChunkBase {
       if (dir == 1) {
         // one pass, out of place into the other buffer of the pair
         // the post-sweep depth-2 halo update rewrites the output pair's shell
-        CellXMaps xm;
-        const bool x_tma = tma && use_tma && cell_x_maps(sweep_number, cb, &xm);
+        PlaneSrc<CellXMaps> xm;
+        const bool x_tma =
+            maps_for(kKeyCellSweepX | (unsigned)(sweep_number << 1 | cb), &xm,
+                     [&](CellXMaps* m) { return cell_x_maps(sweep_number, cb, m); });
         launch_advec_cell_x<S>(tg, stream, sweep_number, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
                                ene1(cb ^ 1), vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_x,
                                !halo_repeat_free, l0, xh, x_tma ? &xm : nullptr, &sc->status);
@@ -954,9 +1020,10 @@ struct Chunk : ChunkBase {
         // the pair where the depth-2 halo update that follows rewrites the
         // output's shell, in place otherwise
         const int cvar = dir == 2 ? (axi ? 2 : 3) : (sweep_number == 1 ? 4 : 5);
-        CellMaps cm;
-        if (tma && use_tma && halo_repeat_free && cell_maps(dir, cvar, cb, &cm)) {
-          launch_cell_sweep_tma<S>(g, stream, dir, cvar, cm, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
+        PlaneSrc<CellMaps> cm;
+        if (halo_repeat_free && maps_for(kKeyCellSweep | (unsigned)(dir << 6 | cvar << 1 | cb), &cm,
+                                         [&](CellMaps* m) { return cell_maps(dir, cvar, cb, m); })) {
+          launch_cell_sweep_tma<S>(tg, stream, dir, cvar, cm, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
                                    ene1(cb ^ 1), vol_flux_x, vol_flux_y, vol_flux_z,
                                    dir == 2 ? mass_flux_y : mass_flux_z, l0, xh, &sc->status);
           cb ^= 1;
@@ -981,14 +1048,17 @@ struct Chunk : ChunkBase {
       V* vin[3] = {vel1(0, vc), vel1(1, vc), vel1(2, vc)};
       V* vout[3] = {vel1(0, vc ^ 1), vel1(1, vc ^ 1), vel1(2, vc ^ 1)};
       pbeg();
-      MomXMaps xm;
-      NodeMaps nm;
-      const bool x_tma = dir == 1 && tma && use_tma && mom_x_maps(rho1(cb), vin, &xm);
+      PlaneSrc<MomXMaps> xm;
+      PlaneSrc<NodeMaps> nm;
+      PlaneSrc<VelMaps> vm;
       const int node_var = dir == 2 ? (axi ? 2 : 3) : (sweep_number == 1 ? 1 : 4);
+      const bool x_tma = dir == 1 && maps_for(kKeyMomSweepX | (unsigned)(sweep_number << 2 | cb << 1 | vc), &xm,
+                                              [&](MomXMaps* m) { return mom_x_maps(rho1(cb), vin, m); });
       const bool node_tma =
-          dir != 1 && tma && use_tma && mom_node_maps(dir, node_var, rho1(cb), &nm);
-      VelMaps vm;
-      const bool vel_tma = dir != 1 && tma && use_tma && mom_vel_maps(dir, vin, &vm);
+          dir != 1 && maps_for(kKeyMomNode | (unsigned)(dir << 6 | node_var << 1 | cb), &nm,
+                               [&](NodeMaps* m) { return mom_node_maps(dir, node_var, rho1(cb), m); });
+      const bool vel_tma = dir != 1 && maps_for(kKeyMomVel3 | (unsigned)(dir << 6 | vc), &vm,
+                                                [&](VelMaps* m) { return mom_vel_maps(dir, vin, m); });
       launch_advec_mom_fused<S>(tg, stream, axi, sweep_number, dir, cell_volume, ga, rho1(cb),
                                 mass_flux_x, mass_flux_y, mass_flux_z, vol_flux_x, vol_flux_y,
                                 vol_flux_z, work[0], work[1], work[2], vin, vout,
@@ -1305,6 +1375,7 @@ struct Chunk : ChunkBase {
     delete plan;
     cudaFree(plane_base);
     cudaFree(read_buf);
+    for (auto& kv : deck_maps) cudaFree(kv.second);
     cudaFree(sc);
     cudaFree(dt_hist);
     cudaFree(sum_hist);
@@ -1636,7 +1707,7 @@ int clover_chunk_use_tma(clover_chunk* c, int on) {
       ch->use_tma = on != 0;
       ch->drop_graphs();  // the captured steps hold the other kernels
     }
-    return ch->tma && ch->use_tma ? 1 : 0;
+    return ch->tma && ch->use_tma && (!ch->plan || ch->halo_repeat_free) ? 1 : 0;
   };
   return c->f64 ? set(c->f64) : set(c->mixed);
 }

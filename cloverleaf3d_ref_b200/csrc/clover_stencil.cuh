@@ -63,11 +63,6 @@ __device__ __forceinline__ A lda(const float* p) { return (A)__ldg(p); }
 // sector per row end (at 512^3 FP64 the x faces were 1.4 ms of the 1.7 ms of a
 // step's halo updates). o: the element's offset; v: the value, negated by the
 // caller where the reference negates.
-// The FP64 forms over a batch leave it to the halo launches: their item loop has
-// no registers left for it (64 decks of 24..128 cells: 10.4 ms per step without,
-// 10.7 with; 512 mixed decks of 16..48 cells: 6.4 without, 6.0 with).
-template <class S, bool kBatch>
-constexpr bool kWritesXh = !kBatch || sizeof(typename S::arith_t) == 4;
 // cells: 1-m <- m, nx+m <- nx+1-m
 template <int D, class T>
 __device__ __forceinline__ void xh_cell(T* a, long long o, int j, int nx, T v) {

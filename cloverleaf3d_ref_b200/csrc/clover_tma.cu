@@ -15,10 +15,12 @@
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
+#include <type_traits>
 
 #include <cudaTypedefs.h>
 
 #include "../../include/clover_kernels.h"
+#include "clover_batch.h"
 #include "clover_launch.h"
 #include "clover_stencil.cuh"
 #include "clover_tma.cuh"
@@ -63,6 +65,55 @@ namespace {
 
 constexpr int TX = 32, TY = 8;
 
+// Where a staged block works: one chunk (the launch grid is the tile grid, the
+// geometry gp and the tensor maps are kernel parameters; the geometry apart
+// from the map, whose address is taken: read through that it took 1-4% more) or an ensemble's decks (one block per
+// (deck, tile) item of the launch's schedule; a deck's maps and geometry are
+// read from global memory, the geometry through shared memory so that it
+// holds no registers). block(): deck, tile x, y, segment.
+template <class Maps>
+struct PlaneSingle {
+  struct Shared {};
+  int seg;
+  Maps mp;
+  __device__ __forceinline__ int4 block() const {
+    return make_int4(0, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z);
+  }
+  __device__ __forceinline__ const Geom& geom(const Geom& gp, int, Shared&) const { return gp; }
+  __device__ __forceinline__ const Maps& maps(int) const { return mp; }
+  __device__ __forceinline__ int segment(int) const { return seg; }
+};
+template <class Maps>
+struct PlaneBatch {
+  struct Shared {
+    Geom g;
+  };
+  const int4* __restrict__ items;
+  const Geom* __restrict__ decks;
+  const Maps* __restrict__ mp;
+  int seg;
+  __device__ __forceinline__ int4 block() const { return __ldg(items + blockIdx.x); }
+  __device__ __forceinline__ const Geom& geom(const Geom&, int d, Shared& sh) const {
+    const int t = threadIdx.y * TX + threadIdx.x;
+    if (t < (int)(sizeof(Geom) / 4)) ((int*)&sh.g)[t] = __ldg((const int*)(decks + d) + t);
+    __syncthreads();
+    return sh.g;
+  }
+  __device__ __forceinline__ const Maps& maps(int d) const { return mp[d]; }
+  // the even length of this deck's segments of at most seg planes
+  __device__ __forceinline__ int segment(int planes) const {
+    const int n = (planes + seg - 1) / seg;
+    return (planes + n - 1) / n;
+  }
+};
+static_assert(sizeof(Geom) % 4 == 0, "a deck's geometry is copied in words");
+constexpr int kStatusStride = (int)(sizeof(DevScalars) / sizeof(int));  // a deck's status word to the next
+#define PLANE_BLOCK(m)                      \
+  __shared__ typename M::Shared plane_sh;   \
+  const int4 bt = (m).block();              \
+  const Geom& g = (m).geom(gp, bt.x, plane_sh); \
+  const auto& maps = (m).maps(bt.x)
+
 constexpr int round128(int b) { return (b + 127) / 128 * 128; }
 
 // Byte layout of one plane buffer of the viscosity ring.
@@ -86,14 +137,15 @@ struct ViscPlane {
   __device__ static En* ene(unsigned char* p) { return (En*)(p + 3 * kVel + kRho); }
 };
 
-template <class S, int RING, int MINB>
+template <class S, class M, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, double dtu_safe,
+k_visc_dt_tma(const __grid_constant__ M m, Geom gp, GeomArrays ga, double g_small, double dtc_safe, double dtu_safe,
               double dtv_safe, double dtw_safe, double dtdiv_safe,
-              const __grid_constant__ ViscMaps maps, typename S::cs_t* __restrict__ pressure,
+              typename S::cs_t* __restrict__ pressure,
               typename S::cs_t* __restrict__ viscosity, typename S::cs_t* __restrict__ soundspeed,
               unsigned long long* __restrict__ min_key, typename S::rho_t* __restrict__ density0,
               typename S::ene_t* __restrict__ energy0, bool xh, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = ViscPlane<S>;
   using A = typename S::arith_t;
   using C = typename S::cs_t;
@@ -102,15 +154,12 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
   __shared__ unsigned long long wmin[TX * TY / 32];
   __shared__ int stop;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int j0 = g.x_min + TX * (int)blockIdx.x, k0 = g.y_min + TY * (int)blockIdx.y;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int j0 = g.x_min + TX * bt.y, k0 = g.y_min + TY * bt.z;
+  const int seg = m.segment(g.z_max - g.z_min + 1);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max ? l0 + seg - 1 : g.z_max;
   const int j = j0 + tx, k = k0 + ty;
   const bool in_jk = j <= g.x_max && k <= g.y_max;
-  // with xh the x-face halo of density0 and energy0 is written below: a cell at
-  // the face takes its own value, which that halo mirrors
-  const bool xe = xh && xh_edge(j, g.x_max);
-  const int jm = xh && j == g.x_min ? 0 : -1, jp = xh && j == g.x_max ? 0 : 1;
   const int pfirst = l0 - 1, plast = l1 + 1;  // cell planes the segment reads
   if (tid == 0) {
     for (int r = 0; r < RING; r++) mbar_init(&full[r], 1);
@@ -125,7 +174,7 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
     const int s = (p - pfirst) % RING;
     unsigned char* b = ring + s * P::kBytes;
     mbar_arrive_expect_tx(&full[s], P::kTx);
-    const int x = TX * (int)blockIdx.x, z = p - g.z_min + 2;
+    const int x = TX * bt.y, z = p - g.z_min + 2;
     const int yn = k0 - g.y_min + 2, yc = yn - 1;
     tma_load_box(P::vel(b, 0), &maps.u, &full[s], x, yn, z);
     tma_load_box(P::vel(b, 1), &maps.v, &full[s], x, yn, z);
@@ -204,6 +253,9 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
         const A yz = A(0.25) * (vgradz2 - vgradz1) / cdz + A(0.25) * (wgrady2 - wgrady1) / cdy;
         // the neighbours' pressures as ideal_gas stores them
 #define PN(bb, a, b) ((A)st<C>(((A(1.4) - A(1.0)) * DN(bb, a, b) * EN(bb, a, b))))
+        // with xh the x-face halo of density0 and energy0 is written below: a cell at
+        // the face takes its own value, which that halo mirrors
+        const int jm = xh && j == g.x_min ? 0 : -1, jp = xh && j == g.x_max ? 0 : 1;
         A pgradx = (PN(bl, jp, 0) - PN(bl, jm, 0)) /
                    (cdx + (A)ga.celldx[g.o1 + j + 1 - g.x_min + 2]);
         A pgrady = (PN(bl, 0, 1) - PN(bl, 0, -1)) /
@@ -232,7 +284,7 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
       }
       const long long o = off3(g, j, k, l);
       viscosity[o] = st<C>(q);
-      if (xe) {
+      if (xh && xh_edge(j, g.x_max)) {
         xh_cell<1>(viscosity, o, j, g.x_max, st<C>(q));
         xh_cell<1>(density0, o, j, g.x_max, P::rho(bl)[(ty + 1) * WR + tx + HR]);
         xh_cell<1>(energy0, o, j, g.x_max, P::ene(bl)[(ty + 1) * WE + tx + HE]);
@@ -293,7 +345,7 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
     // still in flight (planes from the one waited for last to the last one
     // issued) a bounded wait before the block's shared memory is released
     if (tid == 0) {
-      atomicOr(status, CLOVER_STATUS_TIMEOUT);
+      atomicOr(status + bt.x * kStatusStride, CLOVER_STATUS_TIMEOUT);
       for (int p = (l < l1 ? l : l1) + 1; p <= issued_hi; p++) {
         const int u = p - pfirst;
         mbar_wait_bounded(&full[u % RING], (unsigned)(u / RING) & 1u);
@@ -316,7 +368,7 @@ k_visc_dt_tma(Geom g, int seg, GeomArrays ga, double g_small, double dtc_safe, d
       unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
       key = other < key ? other : key;
     }
-    if (tx == 0 && key != ~0ull) atomicMin(min_key, key);
+    if (tx == 0 && key != ~0ull) atomicMin(min_key + (long long)bt.x * kScalarStride, key);
   }
 }
 
@@ -370,12 +422,12 @@ __device__ __forceinline__ void x_box(int t, int& x, int& shift) {
   shift = c - x;
 }
 
-template <class S, int VAR, int RING, int MINB>
+template <class S, class M, int VAR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_mom_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ MomXMaps maps,
-                  typename S::vel_t* __restrict__ u_out, typename S::vel_t* __restrict__ v_out,
+k_mom_sweep_x_tma(const __grid_constant__ M m, Geom gp, GeomArrays ga, typename S::vel_t* __restrict__ u_out, typename S::vel_t* __restrict__ v_out,
                   typename S::vel_t* __restrict__ w_out, Level0<S> lz, bool xh,
                   int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = MomXPlane<S, VAR>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -387,9 +439,10 @@ k_mom_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ MomXMa
   __shared__ int stop;
   const int lane = threadIdx.x, ty = threadIdx.y, tid = ty * TX + lane;
   const unsigned fullmask = 0xffffffffu;
-  const int j = g.x_min - 2 + 29 * (int)blockIdx.x + lane;  // node of this lane
-  const int k0 = g.y_min + TY * (int)blockIdx.y, k = k0 + ty;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int j = g.x_min - 2 + 29 * bt.y + lane;  // node of this lane
+  const int k0 = g.y_min + TY * bt.z, k = k0 + ty;
+  const int seg = m.segment(g.z_max - g.z_min + 2);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max + 1 ? l0 + seg - 1 : g.z_max + 1;
   const int pfirst = l0 - 1, plast = l1 + 1;
   const bool row = k <= g.y_max + 1;              // the whole warp: k depends on the row only
@@ -397,10 +450,10 @@ k_mom_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ MomXMa
   const bool has_mf = row && lane >= 1 && lane <= 30 && j >= g.x_min - 1 && j <= g.x_max + 1;
   const bool has_up = row && lane >= 2 && lane <= 30 && j >= g.x_min && j <= g.x_max + 1;
   int xm, cm, xr, cr, xf, cf, xv, cv;
-  x_box<MF>(blockIdx.x, xm, cm);
-  x_box<R>(blockIdx.x, xr, cr);
-  x_box<VF>(blockIdx.x, xf, cf);
-  x_box<V>(blockIdx.x, xv, cv);
+  x_box<MF>(bt.y, xm, cm);
+  x_box<R>(bt.y, xr, cr);
+  x_box<VF>(bt.y, xf, cf);
+  x_box<V>(bt.y, xv, cv);
   cm += lane; cr += lane; cf += lane; cv += lane;  // this lane's node in each box
   constexpr int WM = kTmaWidth<MF>, WR = kTmaWidth<R>, WF = kTmaWidth<VF>, WV = kTmaWidth<V>;
   if (tid == 0) {
@@ -517,7 +570,7 @@ k_mom_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ MomXMa
     if (tid == 0 && l - 1 + RING <= plast) issue(l - 1 + RING);
   }
   if (stop && tid == 0) {
-    atomicOr(status, CLOVER_STATUS_TIMEOUT);
+    atomicOr(status + bt.x * kStatusStride, CLOVER_STATUS_TIMEOUT);
     for (int p = (l < l1 ? l : l1) + 1; p <= issued_hi; p++) {
       const int u = p - pfirst;
       mbar_wait_bounded(&full[u % RING], (unsigned)(u / RING) & 1u);
@@ -602,11 +655,12 @@ struct PdvPlane {
   __device__ static C* cs(unsigned char* p, int q) { return (C*)(p + 3 * kVel + kRho + kEne + q * kCs); }
 };
 
-template <class S, int RING, int MINB>
+template <class S, class M, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_pdv_predict_eos_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
-                      const __grid_constant__ PdvMaps maps, typename S::cs_t* __restrict__ pressure,
+k_pdv_predict_eos_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ dt_ptr,
+                      typename S::cs_t* __restrict__ pressure,
                       bool xh, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = PdvPlane<S>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -617,20 +671,21 @@ k_pdv_predict_eos_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
   __shared__ unsigned long long full[RING];
   __shared__ int stop;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int j = g.x_min + TX * (int)blockIdx.x + tx, k0 = g.y_min + TY * (int)blockIdx.y;
+  const int j = g.x_min + TX * bt.y + tx, k0 = g.y_min + TY * bt.z;
   const int k = k0 + ty;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int seg = m.segment(g.z_max - g.z_min + 1);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max ? l0 + seg - 1 : g.z_max;
   const bool in_jk = j <= g.x_max && k <= g.y_max;
   const PlaneMarch<RING, 0, 1> pm{ring, P::kBytes, full, &stop, l0, l1 + 1};
-  const A dt = (A)dt_ptr[0];
+  const A dt = (A)dt_ptr[(long long)bt.x * kScalarStride];
   constexpr int WV = kTmaWidth<V>, HV = kTmaHalo<V>, WR = kTmaWidth<R>, HR = kTmaHalo<R>;
   constexpr int WE = kTmaWidth<En>, HE = kTmaHalo<En>, WC = kTmaWidth<C>, HC = kTmaHalo<C>;
   auto issue = [&](int p) {
     unsigned char* b = pm.buf(p);
     unsigned long long* bar = pm.bar(p);
     mbar_arrive_expect_tx(bar, P::kTx);
-    const int x = TX * (int)blockIdx.x, y = k0 - g.y_min + 2, z = p - g.z_min + 2;
+    const int x = TX * bt.y, y = k0 - g.y_min + 2, z = p - g.z_min + 2;
     tma_load_box(P::vel(b, 0), &maps.u, bar, x, y, z);
     tma_load_box(P::vel(b, 1), &maps.v, bar, x, y, z);
     tma_load_box(P::vel(b, 2), &maps.w, bar, x, y, z);
@@ -639,7 +694,7 @@ k_pdv_predict_eos_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     tma_load_box(P::cs(b, 0), &maps.p, bar, x, y, z);
     tma_load_box(P::cs(b, 1), &maps.q, bar, x, y, z);
   };
-  pm.run(l0, l1, status, issue, [&](int l) {
+  pm.run(l0, l1, status + bt.x * kStatusStride, issue, [&](int l) {
     if (!in_jk) return;
     unsigned char* bl = pm.buf(l);
     unsigned char* bu = pm.buf(l + 1);
@@ -710,13 +765,14 @@ struct AccPlane {
   __device__ static V* vel(unsigned char* p, int q) { return (V*)(p + kRho + 2 * kCs + q * kVel); }
 };
 
-template <class S, int RING, int MINB>
+template <class S, class M, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_accelerate_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
-                 const __grid_constant__ AccMaps maps, typename S::vel_t* __restrict__ xvel1,
+k_accelerate_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ dt_ptr,
+                 typename S::vel_t* __restrict__ xvel1,
                  typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1,
                  typename S::vel_t* __restrict__ xvel0, typename S::vel_t* __restrict__ yvel0, bool xh,
                  int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = AccPlane<S>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -726,20 +782,21 @@ k_accelerate_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
   __shared__ unsigned long long full[RING];
   __shared__ int stop;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int j = g.x_min + TX * (int)blockIdx.x + tx, k0 = g.y_min + TY * (int)blockIdx.y;
+  const int j = g.x_min + TX * bt.y + tx, k0 = g.y_min + TY * bt.z;
   const int k = k0 + ty;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int seg = m.segment(g.z_max - g.z_min + 2);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max + 1 ? l0 + seg - 1 : g.z_max + 1;
   const bool in_jk = j <= g.x_max + 1 && k <= g.y_max + 1;
   const PlaneMarch<RING, 1, 0> pm{ring, P::kBytes, full, &stop, l0 - 1, l1};
-  const double dt = dt_ptr[0];
+  const double dt = dt_ptr[(long long)bt.x * kScalarStride];
   constexpr int WV = kTmaWidth<V>, HV = kTmaHalo<V>, WR = kTmaWidth<R>, HR = kTmaHalo<R>;
   constexpr int WC = kTmaWidth<C>, HC = kTmaHalo<C>;
   auto issue = [&](int p) {
     unsigned char* b = pm.buf(p);
     unsigned long long* bar = pm.bar(p);
     mbar_arrive_expect_tx(bar, P::kTx);
-    const int x = TX * (int)blockIdx.x, y1 = k0 - g.y_min + 1, z = p - g.z_min + 2;
+    const int x = TX * bt.y, y1 = k0 - g.y_min + 1, z = p - g.z_min + 2;
     tma_load_box(P::rho(b), &maps.d, bar, x, y1, z);
     tma_load_box(P::cs(b, 0), &maps.p, bar, x, y1, z);
     tma_load_box(P::cs(b, 1), &maps.q, bar, x, y1, z);
@@ -747,7 +804,7 @@ k_accelerate_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     tma_load_box(P::vel(b, 1), &maps.v, bar, x, y1 + 1, z);
     tma_load_box(P::vel(b, 2), &maps.w, bar, x, y1 + 1, z);
   };
-  pm.run(l0, l1, status, issue, [&](int l) {
+  pm.run(l0, l1, status + bt.x * kStatusStride, issue, [&](int l) {
     if (!in_jk) return;
     unsigned char* bl = pm.buf(l);
     unsigned char* bd = pm.buf(l - 1);
@@ -820,15 +877,16 @@ struct FluxPlane {
   __device__ static V* vel(unsigned char* p, int q) { return (V*)(p + q * kVel); }
 };
 
-template <class S, int RING, int MINB>
+template <class S, class M, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
-               const __grid_constant__ FluxMaps maps, const typename S::rho_t* __restrict__ density0,
+k_pdv_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ dt_ptr,
+               const typename S::rho_t* __restrict__ density0,
                typename S::rho_t* __restrict__ density1, const typename S::ene_t* __restrict__ energy0,
                typename S::ene_t* __restrict__ energy1, const typename S::cs_t* __restrict__ pressure,
                const typename S::cs_t* __restrict__ viscosity, typename S::vf_t* __restrict__ vol_flux_x,
                typename S::vf_t* __restrict__ vol_flux_y, typename S::vf_t* __restrict__ vol_flux_z,
                bool xh, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = FluxPlane<S>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -837,13 +895,14 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
   __shared__ unsigned long long full[RING];
   __shared__ int stop;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int j = g.x_min + TX * (int)blockIdx.x + tx, k0 = g.y_min + TY * (int)blockIdx.y;
+  const int j = g.x_min + TX * bt.y + tx, k0 = g.y_min + TY * bt.z;
   const int k = k0 + ty;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int seg = m.segment(g.z_max - g.z_min + 2);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max + 1 ? l0 + seg - 1 : g.z_max + 1;
   const bool in_jk = j <= g.x_max + 1 && k <= g.y_max + 1;
   const PlaneMarch<RING, 0, 1> pm{ring, P::kBytes, full, &stop, l0, l1 + 1};
-  const double dt = dt_ptr[0];
+  const double dt = dt_ptr[(long long)bt.x * kScalarStride];
   constexpr int WV = kTmaWidth<V>, HV = kTmaHalo<V>;
   // the cell's own density0, energy0, pressure and viscosity, loaded one plane
   // ahead (in flight across the block's barrier)
@@ -868,7 +927,7 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     unsigned char* b = pm.buf(p);
     unsigned long long* bar = pm.bar(p);
     mbar_arrive_expect_tx(bar, P::kTx);
-    const int x = TX * (int)blockIdx.x, y = k0 - g.y_min + 2, z = p - g.z_min + 2;
+    const int x = TX * bt.y, y = k0 - g.y_min + 2, z = p - g.z_min + 2;
     tma_load_box(P::vel(b, 0), &maps.u0, bar, x, y, z);
     tma_load_box(P::vel(b, 1), &maps.v0, bar, x, y, z);
     tma_load_box(P::vel(b, 2), &maps.w0, bar, x, y, z);
@@ -876,7 +935,7 @@ k_pdv_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr,
     tma_load_box(P::vel(b, 4), &maps.v1, bar, x, y, z);
     tma_load_box(P::vel(b, 5), &maps.w1, bar, x, y, z);
   };
-  pm.run(l0, l1, status, issue, [&](int l) {
+  pm.run(l0, l1, status + bt.x * kStatusStride, issue, [&](int l) {
     if (!in_jk) return;
     const R d0_s = c_d;
     const En e0_s = c_e;
@@ -1010,15 +1069,15 @@ __device__ __forceinline__ void x_box31(int t, int d, int& x, int& shift) {
   shift = c - x;
 }
 
-template <class S, int TYN, int RING, int MINB>
+template <class S, class M, int TYN, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TYN, MINB)
-k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_constant__ AccMaps maps,
-               typename S::rho_t* __restrict__ density1, const typename S::ene_t* __restrict__ energy0,
+k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ dt_ptr, typename S::rho_t* __restrict__ density1, const typename S::ene_t* __restrict__ energy0,
                typename S::ene_t* __restrict__ energy1, typename S::vel_t* __restrict__ xvel1,
                typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1,
                typename S::vf_t* __restrict__ vol_flux_x, typename S::vf_t* __restrict__ vol_flux_y,
                typename S::vf_t* __restrict__ vol_flux_z, typename S::vel_t* __restrict__ xvel0,
                typename S::vel_t* __restrict__ yvel0, bool xh, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = AccFluxPlane<S, TYN>;
   using A = typename S::arith_t;
   using V = typename S::vel_t;
@@ -1030,21 +1089,22 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
   __shared__ unsigned long long full[RING];
   V* const fresh = (V*)(ring + RING * P::kBytes);  // new velocities of node planes of both parities
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int j = g.x_min + 31 * (int)blockIdx.x + tx, k0 = g.y_min + (TYN - 1) * (int)blockIdx.y;
+  const int j = g.x_min + 31 * bt.y + tx, k0 = g.y_min + (TYN - 1) * bt.z;
   const int k = k0 + ty;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int seg = m.segment(g.z_max - g.z_min + 2);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max + 1 ? l0 + seg - 1 : g.z_max + 1;
   const int pfirst = l0 - 1, plast = l1 + 1 < g.z_max + 1 ? l1 + 1 : g.z_max + 1;
   const bool in_node = j <= g.x_max + 1 && k <= g.y_max + 1;
   const bool own = in_node && tx < TX - 1 && ty < TYN - 1;
   const bool jin = j <= g.x_max, kin = k <= g.y_max;
   const bool xe = xh && xh_edge(j, g.x_max);
-  const double dt = dt_ptr[0];
+  const double dt = dt_ptr[(long long)bt.x * kScalarStride];
   constexpr int WV = kTmaWidth<V>, WR = kTmaWidth<R>, WC = kTmaWidth<C>;
   int xr, cr, xc, cc, xv, cv;
-  x_box31<R>(blockIdx.x, -1, xr, cr);
-  x_box31<C>(blockIdx.x, -1, xc, cc);
-  x_box31<V>(blockIdx.x, 0, xv, cv);
+  x_box31<R>(bt.y, -1, xr, cr);
+  x_box31<C>(bt.y, -1, xc, cc);
+  x_box31<V>(bt.y, 0, xv, cv);
   // this thread's cell (j, k) and node (j, k) in the boxes
   cr += (ty + 1) * WR + tx + 1;
   cc += (ty + 1) * WC + tx + 1;
@@ -1242,7 +1302,7 @@ k_acc_flux_tma(Geom g, int seg, const double* __restrict__ dt_ptr, const __grid_
   if (l <= l1 && tid == 0) {
     // a plane's copies did not arrive in time: report it, and give the copies
     // still in flight a bounded wait before the shared memory is released
-    atomicOr(status, CLOVER_STATUS_TIMEOUT);
+    atomicOr(status + bt.x * kStatusStride, CLOVER_STATUS_TIMEOUT);
     for (int p = l + 1; p <= issued_hi; p++) wait(p);
   }
 }
@@ -1912,11 +1972,11 @@ __device__ __forceinline__ void x_box31(int t, int& x, int& shift) {
   shift = c - x;
 }
 
-template <class S, int DIR, int VAR, int RING, int MINB>
+template <class S, class M, int DIR, int VAR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_mom_node_tma(Geom g, int seg, const __grid_constant__ NodeMaps maps,
-               typename S::nd_t* __restrict__ node_flux, typename S::nd_t* __restrict__ node_mass_post,
+k_mom_node_tma(const __grid_constant__ M m, Geom gp, typename S::nd_t* __restrict__ node_flux, typename S::nd_t* __restrict__ node_mass_post,
                typename S::nd_t* __restrict__ node_mass_pre, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = NodePlane<S, VAR>;
   using MF = typename S::mf_t;
   using R = typename S::rho_t;
@@ -1928,18 +1988,19 @@ k_mom_node_tma(Geom g, int seg, const __grid_constant__ NodeMaps maps,
   const unsigned fullmask = 0xffffffffu;
   const MarchRange r = mom_node_range<DIR>(g);
   const int lane = threadIdx.x, ty = threadIdx.y;
-  const int j = r.jlo - 1 + 31 * (int)blockIdx.x + lane;
-  const int c0 = r.clo + TY * (int)blockIdx.y, c = c0 + ty;
+  const int j = r.jlo - 1 + 31 * bt.y + lane;
+  const int c0 = r.clo + TY * bt.z, c = c0 + ty;
   const bool row = c <= r.chi;      // the whole warp: c depends on the row only
   const bool lds = row && j <= r.jhi;
   const bool own = lds && lane >= 1;
-  const int p0 = r.plo + seg * (int)blockIdx.z;
+  const int seg = m.segment(r.phi - r.plo + 1);
+  const int p0 = r.plo + seg * bt.w;
   const int p1 = p0 + seg - 1 < r.phi ? p0 + seg - 1 : r.phi;
   const PlaneMarch<RING, 1, 1> pm{ring, P::kBytes, full, &stop, p0 - 1, p1 + 1};
   int xm, cm, xr, cr, xf, cf;
-  x_box31<MF>(blockIdx.x, xm, cm);
-  x_box31<R>(blockIdx.x, xr, cr);
-  x_box31<VF>(blockIdx.x, xf, cf);
+  x_box31<MF>(bt.y, xm, cm);
+  x_box31<R>(bt.y, xr, cr);
+  x_box31<VF>(bt.y, xf, cf);
   cm += lane; cr += lane; cf += lane;
   constexpr int WM = kTmaWidth<MF>, WR = kTmaWidth<R>, WF = kTmaWidth<VF>;
   auto issue = [&](int p) {
@@ -1999,7 +2060,7 @@ k_mom_node_tma(Geom g, int seg, const __grid_constant__ NodeMaps maps,
     }
     return u;
   };
-  pm.run(p0, p1, status, issue, [&](int p) {
+  pm.run(p0, p1, status + bt.x * kStatusStride, issue, [&](int p) {
     if (!row) return;
     unsigned char* bm = pm.buf(p - 1);
     unsigned char* b0 = pm.buf(p);
@@ -2044,15 +2105,15 @@ struct VelPlane {
   __device__ static V* vel(unsigned char* p, int q) { return (V*)(p + 3 * kNd + q * kVel); }
 };
 
-template <class S, int DIR, int RING, int MINB>
+template <class S, class M, int DIR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_mom_vel_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ VelMaps maps,
-              const typename S::nd_t* __restrict__ node_flux,
+k_mom_vel_tma(const __grid_constant__ M m, Geom gp, GeomArrays ga, const typename S::nd_t* __restrict__ node_flux,
               const typename S::nd_t* __restrict__ node_mass_pre,
               const typename S::vel_t* __restrict__ u_in, const typename S::vel_t* __restrict__ v_in,
               const typename S::vel_t* __restrict__ w_in, typename S::vel_t* __restrict__ u_out,
               typename S::vel_t* __restrict__ v_out, typename S::vel_t* __restrict__ w_out,
               Level0<S> lz, bool xh, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = VelPlane<S>;
   using W = typename S::nd_t;
   using V = typename S::vel_t;
@@ -2062,10 +2123,11 @@ k_mom_vel_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ VelMaps ma
   __shared__ int stop;
   const MarchRange r = mom_vel_range<DIR>(g);
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int j = r.jlo + TX * (int)blockIdx.x + tx;
-  const int c0 = r.clo + TY * (int)blockIdx.y, c = c0 + ty;
+  const int j = r.jlo + TX * bt.y + tx;
+  const int c0 = r.clo + TY * bt.z, c = c0 + ty;
   const bool in_jc = j <= r.jhi && c <= r.chi;
-  const int p0 = r.plo + seg * (int)blockIdx.z;
+  const int seg = m.segment(r.phi - r.plo + 1);
+  const int p0 = r.plo + seg * bt.w;
   const int p1 = p0 + seg - 1 < r.phi ? p0 + seg - 1 : r.phi;
   const PlaneMarch<RING, 0, 2> pm{ring, P::kBytes, full, &stop, p0, p1 + 2};
   constexpr int WW = kTmaWidth<W>, HW = kTmaHalo<W>, WV = kTmaWidth<V>, HV = kTmaHalo<V>;
@@ -2103,7 +2165,7 @@ k_mom_vel_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ VelMaps ma
     unsigned char* b = pm.buf(p);
     unsigned long long* bar = pm.bar(p);
     mbar_arrive_expect_tx(bar, P::kTx);
-    const int x = TX * (int)blockIdx.x;
+    const int x = TX * bt.y;
     const int y = DIR == 3 ? c0 - g.y_min + 2 : p - g.y_min + 2;
     const int z = DIR == 3 ? p - g.z_min + 2 : c0 - g.z_min + 2;
     tma_load_box(P::nd(b, 0), &maps.nf, bar, x, y, z);
@@ -2113,7 +2175,7 @@ k_mom_vel_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ VelMaps ma
     tma_load_box(P::vel(b, 1), &maps.v, bar, x, y, z);
     tma_load_box(P::vel(b, 2), &maps.w, bar, x, y, z);
   };
-  pm.run(p0, p1, status, issue, [&](int p) {
+  pm.run(p0, p1, status + bt.x * kStatusStride, issue, [&](int p) {
     if (!in_jc) return;
     unsigned char* b0 = pm.buf(p);
     unsigned char* b1 = pm.buf(p + 1);
@@ -2194,14 +2256,14 @@ struct CellPlane {
   __device__ static VF* vfr(unsigned char* p) { return (VF*)(p + kRho + kEne + kVfd + kVfx); }
 };
 
-template <class S, int DIR, int VAR, int RING, int MINB>
+template <class S, class M, int DIR, int VAR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMaps maps,
-                 const typename S::rho_t* __restrict__ d_in, const typename S::ene_t* __restrict__ e_in,
+k_cell_sweep_tma(const __grid_constant__ M m, Geom gp, GeomArrays ga, const typename S::rho_t* __restrict__ d_in, const typename S::ene_t* __restrict__ e_in,
                  typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
                  const typename S::vf_t* __restrict__ vfx, const typename S::vf_t* __restrict__ vfy,
                  const typename S::vf_t* __restrict__ vfz, typename S::mf_t* __restrict__ mass_flux,
                  Level0<S> lz, bool xh, int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = CellPlane<S, DIR, VAR>;
   using R = typename S::rho_t;
   using En = typename S::ene_t;
@@ -2213,14 +2275,15 @@ k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMap
   __shared__ int stop;
   const MarchRange r = cell_sweep_range<DIR>(g);
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int j = r.jlo + TX * (int)blockIdx.x + tx;
-  const int c0 = r.clo + TY * (int)blockIdx.y, c = c0 + ty;
+  const int j = r.jlo + TX * bt.y + tx;
+  const int c0 = r.clo + TY * bt.z, c = c0 + ty;
   const bool col = j <= r.jhi && c <= r.chi;
   const bool update = c <= r.cmax;
   const int pmin = DIR == 2 ? g.y_min : g.z_min;
   const int pmax = DIR == 2 ? g.y_max : g.z_max;
   const int top = pmax + 2;
-  const int q0 = pmin + seg * (int)blockIdx.z;  // cells of this segment: [q0, q1]
+  const int seg = m.segment(pmax - pmin + 1);
+  const int q0 = pmin + seg * bt.w;  // cells of this segment: [q0, q1]
   const int q1 = q0 + seg - 1 < pmax ? q0 + seg - 1 : pmax;
   const bool last = q1 == pmax;  // this segment also walks the faces pmax+1, pmax+2
   const int pend = last ? top : q1 + 1;
@@ -2286,7 +2349,7 @@ k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMap
     unsigned char* b = pm.buf(p);
     unsigned long long* bar = pm.bar(p);
     mbar_arrive_expect_tx(bar, P::kTx);
-    const int x = TX * (int)blockIdx.x;
+    const int x = TX * bt.y;
     const int y = DIR == 3 ? c0 - g.y_min + 2 : p - g.y_min + 2;
     const int z = DIR == 3 ? p - g.z_min + 2 : c0 - g.z_min + 2;
     tma_load_box(P::rho(b), &maps.d, bar, x, y, z);
@@ -2296,7 +2359,7 @@ k_cell_sweep_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellMap
     if (P::kR) tma_load_box(P::vfr(b), &maps.vfr, bar, x, y, z);
   };
   using MFT = MF;
-  pm.run(q0, pend, status, issue, [&](int p) {
+  pm.run(q0, pend, status + bt.x * kStatusStride, issue, [&](int p) {
     if (!col) return;
     unsigned char* b0 = pm.buf(p);
     unsigned char* b1 = pm.buf(p + 1);
@@ -2409,12 +2472,12 @@ struct CellXPlane {
   __device__ static VF* vfz(unsigned char* p) { return (VF*)(p + kRho + kEne + kVf8 + kVf9); }
 };
 
-template <class S, int VAR, int RING, int MINB>
+template <class S, class M, int VAR, int RING, int MINB>
 __global__ void __launch_bounds__(TX * TY, MINB)
-k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellXMaps maps,
-                   typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
+k_cell_sweep_x_tma(const __grid_constant__ M m, Geom gp, GeomArrays ga, typename S::rho_t* __restrict__ d_out, typename S::ene_t* __restrict__ e_out,
                    typename S::mf_t* __restrict__ mass_flux, Level0<S> lz, bool xh,
                    int* __restrict__ status) {
+  PLANE_BLOCK(m);
   using P = CellXPlane<S, VAR>;
   using R = typename S::rho_t;
   using En = typename S::ene_t;
@@ -2425,9 +2488,10 @@ k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellX
   __shared__ unsigned long long full[RING];
   __shared__ int stop;
   const int lane = threadIdx.x, ty = threadIdx.y;
-  const int c = g.x_min + kCellXLanes * (int)blockIdx.x + lane;  // this lane's face and cell
-  const int k0 = g.y_min + TY * (int)blockIdx.y, k = k0 + ty;
-  const int l0 = g.z_min + seg * (int)blockIdx.z;
+  const int c = g.x_min + kCellXLanes * bt.y + lane;  // this lane's face and cell
+  const int k0 = g.y_min + TY * bt.z, k = k0 + ty;
+  const int seg = m.segment(g.z_max - g.z_min + 1);
+  const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max ? l0 + seg - 1 : g.z_max;
   const bool row = k <= g.y_max;  // the whole warp: k is the row's
   const int top = g.x_max + 2;
@@ -2435,9 +2499,9 @@ k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellX
   const bool upd = row && lane < kCellXLanes && c <= g.x_max;
   const PlaneMarch<RING, 0, 1> pm{ring, P::kBytes, full, &stop, l0, l1 + 1};
   int xr, cr, xe, ce, xf, cf;
-  cell_x_box<R>(blockIdx.x, xr, cr);
-  cell_x_box<En>(blockIdx.x, xe, ce);
-  cell_x_box<VF>(blockIdx.x, xf, cf);
+  cell_x_box<R>(bt.y, xr, cr);
+  cell_x_box<En>(bt.y, xe, ce);
+  cell_x_box<VF>(bt.y, xf, cf);
   cr += lane; ce += lane; cf += lane;  // cell c in each box
   constexpr int WR = kTmaWidth<R>, WE = kTmaWidth<En>, WF = kTmaWidth<VF>;
   // vertexdx at c-1, c and MIN(c+1, x_max+2)
@@ -2458,7 +2522,7 @@ k_cell_sweep_x_tma(Geom g, int seg, GeomArrays ga, const __grid_constant__ CellX
       tma_load_box(P::vfz(b), &maps.vfz, bar, xf, y, z);
     }
   };
-  pm.run(l0, l1, status, issue, [&](int l) {
+  pm.run(l0, l1, status + bt.x * kStatusStride, issue, [&](int l) {
     if (!row) return;
     unsigned char* b = pm.buf(l);
     unsigned char* bz = pm.buf(l + 1);
@@ -2567,25 +2631,97 @@ int plane_seg(long long tiles, int planes) {
   return (planes + n - 1) / n;
 }
 
-// The launch grid of a staged march (x, y tiles; z segments), and its segment.
+// Launch a staged march: tiles(g, seg) is a chunk's grid with segments of at
+// most seg planes (tiles(g, 1).z = its planes). Over an ensemble the segment
+// follows from the tiles and planes of all its decks unless the autotuner chose
+// one; a block takes one item whatever grid the schedule has.
+template <class Maps, class KS, class KB, class... A>
+void launch_planes(const Target& tg, cudaStream_t s, unsigned key, GridFn tiles, int smem,
+                   const PlaneSrc<Maps>& src, KS ks, KB kb, const A&... a) {
+  if (!tg.plan) {
+    const dim3 one = tiles(tg.g, 1);
+    const int seg = plane_seg((long long)one.x * one.y, (int)one.z);
+    ks<<<dim3(one.x, one.y, (one.z + seg - 1) / seg), dim3(TX, TY), smem, s>>>(
+        PlaneSingle<Maps>{seg, src.one}, tg.g, a...);
+    return;
+  }
+  double work = 0.0;
+  for (const Geom& q : tg.plan->decks) {
+    const dim3 one = tiles(q, 1);
+    work += (double)one.x * one.y * one.z;
+  }
+  int seg = (int)(sqrt(work / 120.0) + 0.5);
+  seg = seg < 1 ? 1 : seg > 32 ? 32 : seg;
+  key |= kKeyStaged;
+  const BatchLaunch bl = batch_launch(tg.plan, s, key, tiles, seg, true, (const void*)kb, TX * TY);
+  if (bl.n <= 0) return;
+  batch_mark(tg.plan, key, s, true);
+  kb<<<bl.n, dim3(TX, TY), smem, s>>>(PlaneBatch<Maps>{bl.items, bl.decks, src.decks, bl.aux},
+                                        tg.g, a...);
+  batch_mark(tg.plan, key, s, false);
+}
+
+dim3 tiles_of(int tiles_x, int tiles_y, int planes, int seg) {
+  return dim3(tiles_x, tiles_y, (planes + seg - 1) / seg);
+}
+dim3 tiles_cells(const Geom& g, int seg) {
+  return tiles_of((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY, g.z_max - g.z_min + 1, seg);
+}
+dim3 tiles_nodes(const Geom& g, int seg) {
+  return tiles_of((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
+                  g.z_max - g.z_min + 2, seg);
+}
+// a block owns one lane and one row less than it has
+dim3 tiles_acc_flux(const Geom& g, int seg) {
+  return tiles_of((g.x_max + 1 - g.x_min + TX - 1) / (TX - 1), (g.y_max + 1 - g.y_min + TY - 1) / (TY - 1),
+                  g.z_max - g.z_min + 2, seg);
+}
+// nodes x_min-2.., 29 per warp
+dim3 tiles_mom_x(const Geom& g, int seg) {
+  return tiles_of((g.x_max + 1 - g.x_min + 1 + 28) / 29, (g.y_max + 1 - g.y_min + 1 + TY - 1) / TY,
+                  g.z_max - g.z_min + 2, seg);
+}
+// faces x_min..x_max+2, 31 per warp
+dim3 tiles_cell_x(const Geom& g, int seg) {
+  return tiles_of((g.x_max - g.x_min + 3 + kCellXLanes - 1) / kCellXLanes, (g.y_max - g.y_min + TY) / TY,
+                  g.z_max - g.z_min + 1, seg);
+}
+template <int DIR>
+dim3 tiles_mom_node(const Geom& g, int seg) {
+  const MarchRange r = mom_node_range<DIR>(g);
+  return tiles_of((r.jhi - r.jlo + 1 + 30) / 31, (r.chi - r.clo + 1 + TY - 1) / TY, r.phi - r.plo + 1, seg);
+}
+template <int DIR>
+dim3 tiles_mom_vel(const Geom& g, int seg) {
+  const MarchRange r = mom_vel_range<DIR>(g);
+  return tiles_of((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY, r.phi - r.plo + 1, seg);
+}
+template <int DIR>
+dim3 tiles_cell(const Geom& g, int seg) {
+  const MarchRange r = cell_sweep_range<DIR>(g);
+  return tiles_of((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY,
+                  (DIR == 2 ? g.y_max - g.y_min : g.z_max - g.z_min) + 1, seg);
+}
+template <class K>
+bool set_smem(K kern, int bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+// both forms of a staged kernel
+#define SET_BOTH(MAPS, BYTES, K, ...)                               \
+  (set_smem(K<S, PlaneSingle<MAPS>, __VA_ARGS__>, BYTES) &&         \
+   set_smem(K<S, PlaneBatch<MAPS>, __VA_ARGS__>, BYTES))
+#define GO_BOTH(KEY, TILES, BYTES, SRC, MAPS, K, KARGS, ...)        \
+  launch_planes(tg, s, KEY, TILES, BYTES, SRC, K<S, PlaneSingle<MAPS>, KTARGS KARGS>, \
+                K<S, PlaneBatch<MAPS>, KTARGS KARGS>, __VA_ARGS__)
+#define KTARGS(...) __VA_ARGS__
+
+// The launch grid of a drop-in march (x, y tiles; z segments), and its segment.
 dim3 plane_grid(int tiles_x, int tiles_y, int planes, int* seg) {
   *seg = plane_seg((long long)tiles_x * tiles_y, planes);
   return dim3(tiles_x, tiles_y, (planes + *seg - 1) / *seg);
 }
 
 }  // namespace
-
-template <class S>
-bool visc_dt_tma_maps(const Geom& g, const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
-                      const typename S::vel_t* zvel0, const typename S::rho_t* density0,
-                      const typename S::ene_t* energy0, ViscMaps* m) {
-  using V = typename S::vel_t;
-  return encode_plane_map(&m->u, xvel0, sizeof(V), g, TY + 1) &&
-         encode_plane_map(&m->v, yvel0, sizeof(V), g, TY + 1) &&
-         encode_plane_map(&m->w, zvel0, sizeof(V), g, TY + 1) &&
-         encode_plane_map(&m->d, density0, sizeof(typename S::rho_t), g, TY + 2) &&
-         encode_plane_map(&m->e, energy0, sizeof(typename S::ene_t), g, TY + 2);
-}
 
 // blocks per SM (measured at 512^3: FP64 2.90 ms at 3 against 3.15 ms at 2,
 // where the FP64 form spills no register)
@@ -2594,26 +2730,19 @@ constexpr int kViscMinBlocks = sizeof(typename S::arith_t) == 4 ? 4 : 3;
 
 template <class S>
 bool visc_dt_tma_prepare() {
-  return cudaFuncSetAttribute(k_visc_dt_tma<S, kViscRing, kViscMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kViscRing * ViscPlane<S>::kBytes) == cudaSuccess;
+  return SET_BOTH(ViscMaps, kViscRing * ViscPlane<S>::kBytes, k_visc_dt_tma, kViscRing, kViscMinBlocks<S>);
 }
 
 template <class S>
-void launch_visc_dt_tma(const Geom& g, cudaStream_t s, const ViscMaps& maps, const GeomArrays& ga,
-                        double g_small, double dtc_safe, double dtu_safe, double dtv_safe,
-                        double dtw_safe, double dtdiv_safe, typename S::cs_t* pressure,
-                        typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
-                        unsigned long long* min_key, typename S::rho_t* density0,
-                        typename S::ene_t* energy0, bool xh, int* status) {
-  auto kern = k_visc_dt_tma<S, kViscRing, kViscMinBlocks<S>>;
-  const int smem = kViscRing * ViscPlane<S>::kBytes;
-  int seg;
-  const dim3 grid = plane_grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
-                               g.z_max - g.z_min + 1, &seg);
-  kern<<<grid, dim3(TX, TY), smem, s>>>(g, seg, ga, g_small, dtc_safe, dtu_safe, dtv_safe,
-                                         dtw_safe, dtdiv_safe, maps, pressure,
-                                         viscosity, soundspeed, min_key, density0, energy0, xh, status);
+void launch_visc_dt_tma(const Target& tg, cudaStream_t s, const PlaneSrc<ViscMaps>& maps,
+                        const GeomArrays& ga, double g_small, double dtc_safe, double dtu_safe,
+                        double dtv_safe, double dtw_safe, double dtdiv_safe,
+                        typename S::cs_t* pressure, typename S::cs_t* viscosity,
+                        typename S::cs_t* soundspeed, unsigned long long* min_key,
+                        typename S::rho_t* density0, typename S::ene_t* energy0, bool xh, int* status) {
+  GO_BOTH(kKeyTimestepVisc, tiles_cells, kViscRing * ViscPlane<S>::kBytes, maps, ViscMaps, k_visc_dt_tma,
+          (kViscRing, kViscMinBlocks<S>), ga, g_small, dtc_safe, dtu_safe, dtv_safe, dtw_safe,
+          dtdiv_safe, pressure, viscosity, soundspeed, min_key, density0, energy0, xh, status);
 }
 
 constexpr int kMomXRing = 4;
@@ -2622,30 +2751,25 @@ constexpr int kMomXMinBlocks = sizeof(typename S::arith_t) == 4 ? 4 : 3;
 
 template <class S>
 bool mom_x_tma_prepare() {
-  return cudaFuncSetAttribute(k_mom_sweep_x_tma<S, 0, kMomXRing, kMomXMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kMomXRing * MomXPlane<S, 0>::kBytes) == cudaSuccess &&
-         cudaFuncSetAttribute(k_mom_sweep_x_tma<S, 4, kMomXRing, kMomXMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kMomXRing * MomXPlane<S, 4>::kBytes) == cudaSuccess;
+  return SET_BOTH(MomXMaps, (kMomXRing * MomXPlane<S, 0>::kBytes), k_mom_sweep_x_tma, 0, kMomXRing,
+                  kMomXMinBlocks<S>) &&
+         SET_BOTH(MomXMaps, (kMomXRing * MomXPlane<S, 4>::kBytes), k_mom_sweep_x_tma, 4, kMomXRing,
+                  kMomXMinBlocks<S>);
 }
 
 template <class S>
-void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& maps,
+void launch_mom_x_tma(const Target& tg, cudaStream_t s, int sweep, const PlaneSrc<MomXMaps>& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
                       const Level0<S>& level0, bool xh, int* status) {
-  int seg;
-  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + 1 + 28) / 29,
-                               (g.y_max + 1 - g.y_min + 1 + TY - 1) / TY, g.z_max - g.z_min + 2, &seg);
   // post_vol variant: 0 on sweep 1, 4 (the cell volume) on sweep 3
   if (sweep == 1)
-    k_mom_sweep_x_tma<S, 0, kMomXRing, kMomXMinBlocks<S>>
-        <<<grid, dim3(TX, TY), kMomXRing * MomXPlane<S, 0>::kBytes, s>>>(
-            g, seg, ga, maps, vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
+    GO_BOTH(kKeyMomSweepX, tiles_mom_x, (kMomXRing * MomXPlane<S, 0>::kBytes), maps, MomXMaps,
+            k_mom_sweep_x_tma, (0, kMomXRing, kMomXMinBlocks<S>), ga, vel_out[0], vel_out[1],
+            vel_out[2], level0, xh, status);
   else
-    k_mom_sweep_x_tma<S, 4, kMomXRing, kMomXMinBlocks<S>>
-        <<<grid, dim3(TX, TY), kMomXRing * MomXPlane<S, 4>::kBytes, s>>>(
-            g, seg, ga, maps, vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
+    GO_BOTH(kKeyMomSweepX | (4 << 4), tiles_mom_x, (kMomXRing * MomXPlane<S, 4>::kBytes), maps, MomXMaps,
+            k_mom_sweep_x_tma, (4, kMomXRing, kMomXMinBlocks<S>), ga, vel_out[0], vel_out[1],
+            vel_out[2], level0, xh, status);
 }
 
 // The bounded wait of the staged kernels, made to run out: one block arms a
@@ -2679,20 +2803,16 @@ constexpr int kAccFluxSmem = kStencilRing * AccFluxPlane<S, TY>::kBytes +
 
 template <class S>
 bool stencils_tma_prepare() {
-  if (cudaFuncSetAttribute(k_pdv_predict_eos_tma<S, kStencilRing, kStencilMinBlocks<S>>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kStencilRing * PdvPlane<S>::kBytes) != cudaSuccess)
+  if (!SET_BOTH(PdvMaps, kStencilRing * PdvPlane<S>::kBytes, k_pdv_predict_eos_tma, kStencilRing,
+                kStencilMinBlocks<S>))
     return false;
   if constexpr (kFusedAccFlux<S>)
-    return cudaFuncSetAttribute(k_acc_flux_tma<S, TY, kStencilRing, 3>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, kAccFluxSmem<S>) == cudaSuccess;
+    return SET_BOTH(AccMaps, kAccFluxSmem<S>, k_acc_flux_tma, TY, kStencilRing, 3);
   else
-    return cudaFuncSetAttribute(k_accelerate_tma<S, kStencilRing, kStencilMinBlocks<S>>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kStencilRing * AccPlane<S>::kBytes) == cudaSuccess &&
-           cudaFuncSetAttribute(k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kStencilRing * FluxPlane<S>::kBytes) == cudaSuccess;
+    return SET_BOTH(AccMaps, kStencilRing * AccPlane<S>::kBytes, k_accelerate_tma, kStencilRing,
+                    kStencilMinBlocks<S>) &&
+           SET_BOTH(FluxMaps, kStencilRing * FluxPlane<S>::kBytes, k_pdv_flux_tma, kStencilRing,
+                    kStencilMinBlocks<S>);
 }
 
 // blocks per SM of the drop-in PdV: the corrector's plane (six velocity
@@ -2822,128 +2942,106 @@ constexpr int kCellXMinBlocks = 4;
 
 template <class S>
 bool cell_sweep_x_tma_prepare() {
-  return cudaFuncSetAttribute(k_cell_sweep_x_tma<S, 0, kStencilRing, kCellXMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kStencilRing * CellXPlane<S, 0>::kBytes) == cudaSuccess &&
-         cudaFuncSetAttribute(k_cell_sweep_x_tma<S, 1, kStencilRing, kCellXMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kStencilRing * CellXPlane<S, 1>::kBytes) == cudaSuccess;
+  return SET_BOTH(CellXMaps, (kStencilRing * CellXPlane<S, 0>::kBytes), k_cell_sweep_x_tma, 0, kStencilRing,
+                  kCellXMinBlocks<S>) &&
+         SET_BOTH(CellXMaps, (kStencilRing * CellXPlane<S, 1>::kBytes), k_cell_sweep_x_tma, 1, kStencilRing,
+                  kCellXMinBlocks<S>);
 }
 
 template <class S>
-void launch_cell_sweep_x_tma(const Geom& g, cudaStream_t s, int sweep, const CellXMaps& maps,
+void launch_cell_sweep_x_tma(const Target& tg, cudaStream_t s, int sweep, const PlaneSrc<CellXMaps>& maps,
                              const GeomArrays& ga, typename S::rho_t* d_out,
                              typename S::ene_t* e_out, typename S::mf_t* mass_flux_x,
                              const Level0<S>& level0, bool xh, int* status) {
-  // faces x_min..x_max+2, 31 per warp
-  int seg;
-  const dim3 grid = plane_grid((g.x_max - g.x_min + 3 + kCellXLanes - 1) / kCellXLanes,
-                               (g.y_max - g.y_min + TY) / TY, g.z_max - g.z_min + 1, &seg);
   if (sweep == 1)
-    k_cell_sweep_x_tma<S, 0, kStencilRing, kCellXMinBlocks<S>>
-        <<<grid, dim3(TX, TY), kStencilRing * CellXPlane<S, 0>::kBytes, s>>>(
-            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, xh, status);
+    GO_BOTH(kKeyCellSweepX, tiles_cell_x, (kStencilRing * CellXPlane<S, 0>::kBytes), maps, CellXMaps,
+            k_cell_sweep_x_tma, (0, kStencilRing, kCellXMinBlocks<S>), ga, d_out, e_out, mass_flux_x,
+            level0, xh, status);
   else
-    k_cell_sweep_x_tma<S, 1, kStencilRing, kCellXMinBlocks<S>>
-        <<<grid, dim3(TX, TY), kStencilRing * CellXPlane<S, 1>::kBytes, s>>>(
-            g, seg, ga, maps, d_out, e_out, mass_flux_x, level0, xh, status);
+    GO_BOTH(kKeyCellSweepX | (1u << 4), tiles_cell_x, (kStencilRing * CellXPlane<S, 1>::kBytes), maps,
+            CellXMaps, k_cell_sweep_x_tma, (1, kStencilRing, kCellXMinBlocks<S>), ga, d_out, e_out,
+            mass_flux_x, level0, xh, status);
 }
 
 template <class S>
-void launch_pdv_predict_eos_tma(const Geom& g, cudaStream_t s, const double* dt_ptr,
-                                const PdvMaps& maps, typename S::cs_t* pressure, bool xh,
+void launch_pdv_predict_eos_tma(const Target& tg, cudaStream_t s, const double* dt_ptr,
+                                const PlaneSrc<PdvMaps>& maps, typename S::cs_t* pressure, bool xh,
                                 int* status) {
-  int seg;
-  const dim3 grid = plane_grid((g.x_max - g.x_min + TX) / TX, (g.y_max - g.y_min + TY) / TY,
-                               g.z_max - g.z_min + 1, &seg);
-  k_pdv_predict_eos_tma<S, kStencilRing, kStencilMinBlocks<S>>
-      <<<grid, dim3(TX, TY), kStencilRing * PdvPlane<S>::kBytes, s>>>(g, seg, dt_ptr, maps,
-                                                                       pressure, xh, status);
+  GO_BOTH(kKeyPdvPredict, tiles_cells, kStencilRing * PdvPlane<S>::kBytes, maps, PdvMaps,
+          k_pdv_predict_eos_tma, (kStencilRing, kStencilMinBlocks<S>), dt_ptr, pressure, xh, status);
 }
 
 template <class S>
-void launch_accelerate_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
-                           typename S::vel_t* xvel1, typename S::vel_t* yvel1,
-                           typename S::vel_t* zvel1, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
-                           bool xh, int* status) {
-  int seg;
-  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
-                               g.z_max - g.z_min + 2, &seg);
-  k_accelerate_tma<S, kStencilRing, kStencilMinBlocks<S>>
-      <<<grid, dim3(TX, TY), kStencilRing * AccPlane<S>::kBytes, s>>>(g, seg, dt_ptr, maps,
-                                                                      xvel1, yvel1, zvel1, xvel0, yvel0, xh, status);
+void launch_accelerate_tma(const Target& tg, cudaStream_t s, const double* dt_ptr,
+                           const PlaneSrc<AccMaps>& maps, typename S::vel_t* xvel1,
+                           typename S::vel_t* yvel1, typename S::vel_t* zvel1,
+                           typename S::vel_t* xvel0, typename S::vel_t* yvel0, bool xh, int* status) {
+  GO_BOTH(kKeyAccelerate, tiles_nodes, kStencilRing * AccPlane<S>::kBytes, maps, AccMaps, k_accelerate_tma,
+          (kStencilRing, kStencilMinBlocks<S>), dt_ptr, xvel1, yvel1, zvel1, xvel0, yvel0, xh, status);
 }
 
 template <class S>
-void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const FluxMaps& maps,
-                         const typename S::rho_t* density0, typename S::rho_t* density1,
-                         const typename S::ene_t* energy0, typename S::ene_t* energy1,
-                         const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
-                         typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                         typename S::vf_t* vol_flux_z, bool xh, int* status) {
-  int seg;
-  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX) / TX, (g.y_max + 1 - g.y_min + TY) / TY,
-                               g.z_max - g.z_min + 2, &seg);
-  k_pdv_flux_tma<S, kStencilRing, kStencilMinBlocks<S>>
-      <<<grid, dim3(TX, TY), kStencilRing * FluxPlane<S>::kBytes, s>>>(
-          g, seg, dt_ptr, maps, density0, density1, energy0, energy1, pressure, viscosity,
-          vol_flux_x, vol_flux_y, vol_flux_z, xh, status);
-}
-
-template <class S>
-void launch_acc_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
+void launch_pdv_flux_tma(const Target& tg, cudaStream_t s, const double* dt_ptr,
+                         const PlaneSrc<FluxMaps>& maps, const typename S::rho_t* density0,
                          typename S::rho_t* density1, const typename S::ene_t* energy0,
-                         typename S::ene_t* energy1, typename S::vel_t* xvel1,
-                         typename S::vel_t* yvel1, typename S::vel_t* zvel1,
+                         typename S::ene_t* energy1, const typename S::cs_t* pressure,
+                         const typename S::cs_t* viscosity, typename S::vf_t* vol_flux_x,
+                         typename S::vf_t* vol_flux_y, typename S::vf_t* vol_flux_z, bool xh,
+                         int* status) {
+  GO_BOTH(kKeyPdvFlux, tiles_nodes, kStencilRing * FluxPlane<S>::kBytes, maps, FluxMaps, k_pdv_flux_tma,
+          (kStencilRing, kStencilMinBlocks<S>), dt_ptr, density0, density1, energy0, energy1, pressure,
+          viscosity, vol_flux_x, vol_flux_y, vol_flux_z, xh, status);
+}
+
+template <class S>
+void launch_acc_flux_tma(const Target& tg, cudaStream_t s, const double* dt_ptr,
+                         const PlaneSrc<AccMaps>& maps, typename S::rho_t* density1,
+                         const typename S::ene_t* energy0, typename S::ene_t* energy1,
+                         typename S::vel_t* xvel1, typename S::vel_t* yvel1, typename S::vel_t* zvel1,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
-                         typename S::vf_t* vol_flux_z, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
-                           bool xh, int* status) {
-  int seg;
-  const dim3 grid = plane_grid((g.x_max + 1 - g.x_min + TX - 1) / (TX - 1),
-                               (g.y_max + 1 - g.y_min + TY - 1) / (TY - 1), g.z_max - g.z_min + 2, &seg);
-  k_acc_flux_tma<S, TY, kStencilRing, 3>
-      <<<grid, dim3(TX, TY), kAccFluxSmem<S>, s>>>(g, seg, dt_ptr, maps, density1, energy0, energy1,
-                                                     xvel1, yvel1, zvel1, vol_flux_x, vol_flux_y,
-                                                     vol_flux_z, xvel0, yvel0, xh, status);
+                         typename S::vf_t* vol_flux_z, typename S::vel_t* xvel0,
+                         typename S::vel_t* yvel0, bool xh, int* status) {
+  GO_BOTH(kKeyPdvFlux, tiles_acc_flux, kAccFluxSmem<S>, maps, AccMaps, k_acc_flux_tma,
+          (TY, kStencilRing, 3), dt_ptr, density1, energy0, energy1, xvel1, yvel1, zvel1, vol_flux_x,
+          vol_flux_y, vol_flux_z, xvel0, yvel0, xh, status);
 }
 
 template <class S>
 constexpr int kNodeMinBlocks = sizeof(typename S::arith_t) == 4 ? 5 : 5;
 
+// calls f with the integral constants of the sweep's direction and post-volume variant
+template <class F>
+void node_variant(int dir, int var, F f) {
+  using std::integral_constant;
+  if (dir == 3 && var == 1) f(integral_constant<int, 3>{}, integral_constant<int, 1>{});
+  else if (dir == 3) f(integral_constant<int, 3>{}, integral_constant<int, 4>{});
+  else if (var == 2) f(integral_constant<int, 2>{}, integral_constant<int, 2>{});
+  else f(integral_constant<int, 2>{}, integral_constant<int, 3>{});
+}
+
 template <class S>
 bool mom_node_tma_prepare() {
   bool ok = true;
-  auto set = [&](auto kern, int bytes) {
-    ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kStencilRing * bytes) == cudaSuccess;
-  };
-  set(k_mom_node_tma<S, 3, 1, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 1>::kBytes);
-  set(k_mom_node_tma<S, 3, 4, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 4>::kBytes);
-  set(k_mom_node_tma<S, 2, 2, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 2>::kBytes);
-  set(k_mom_node_tma<S, 2, 3, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 3>::kBytes);
+  const int dv[4][2] = {{3, 1}, {3, 4}, {2, 2}, {2, 3}};
+  for (const auto& q : dv)
+    node_variant(q[0], q[1], [&](auto d, auto v) {
+      constexpr int D = decltype(d)::value, V = decltype(v)::value;
+      ok = ok && SET_BOTH(NodeMaps, (kStencilRing * NodePlane<S, V>::kBytes), k_mom_node_tma, D, V,
+                          kStencilRing, kNodeMinBlocks<S>);
+    });
   return ok;
 }
 
 template <class S>
-void launch_mom_node_tma(const Geom& g, cudaStream_t s, int dir, int var, const NodeMaps& maps,
-                         typename S::nd_t* node_flux, typename S::nd_t* node_mass_post,
-                         typename S::nd_t* node_mass_pre, int* status) {
-  auto go = [&](auto kern, int bytes, const MarchRange& r) {
-    int seg;
-    const dim3 grid = plane_grid((r.jhi - r.jlo + 1 + 30) / 31, (r.chi - r.clo + 1 + TY - 1) / TY,
-                                 r.phi - r.plo + 1, &seg);
-    kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, seg, maps, node_flux,
-                                                          node_mass_post, node_mass_pre, status);
-  };
-  if (dir == 3) {
-    const MarchRange r = mom_node_range<3>(g);
-    if (var == 1) go(k_mom_node_tma<S, 3, 1, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 1>::kBytes, r);
-    else go(k_mom_node_tma<S, 3, 4, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 4>::kBytes, r);
-  } else {
-    const MarchRange r = mom_node_range<2>(g);
-    if (var == 2) go(k_mom_node_tma<S, 2, 2, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 2>::kBytes, r);
-    else go(k_mom_node_tma<S, 2, 3, kStencilRing, kNodeMinBlocks<S>>, NodePlane<S, 3>::kBytes, r);
-  }
+void launch_mom_node_tma(const Target& tg, cudaStream_t s, int dir, int var,
+                         const PlaneSrc<NodeMaps>& maps, typename S::nd_t* node_flux,
+                         typename S::nd_t* node_mass_post, typename S::nd_t* node_mass_pre, int* status) {
+  node_variant(dir, var, [&](auto d, auto v) {
+    constexpr int D = decltype(d)::value, V = decltype(v)::value;
+    GO_BOTH(kKeyMomNode | D | (V << 4), tiles_mom_node<D>, (kStencilRing * NodePlane<S, V>::kBytes), maps,
+            NodeMaps, k_mom_node_tma, (D, V, kStencilRing, kNodeMinBlocks<S>), node_flux,
+            node_mass_post, node_mass_pre, status);
+  });
 }
 
 template <class S>
@@ -2954,116 +3052,105 @@ constexpr int kVelRing = 5;
 
 template <class S>
 bool mom_vel_tma_prepare() {
-  return cudaFuncSetAttribute(k_mom_vel_tma<S, 2, kVelRing, kVelMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kVelRing * VelPlane<S>::kBytes) == cudaSuccess &&
-         cudaFuncSetAttribute(k_mom_vel_tma<S, 3, kVelRing, kVelMinBlocks<S>>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kVelRing * VelPlane<S>::kBytes) == cudaSuccess;
+  return SET_BOTH(VelMaps, kVelRing * VelPlane<S>::kBytes, k_mom_vel_tma, 2, kVelRing, kVelMinBlocks<S>) &&
+         SET_BOTH(VelMaps, kVelRing * VelPlane<S>::kBytes, k_mom_vel_tma, 3, kVelRing, kVelMinBlocks<S>);
 }
 
 template <class S>
-void launch_mom_vel_tma(const Geom& g, cudaStream_t s, int dir, const VelMaps& maps,
+void launch_mom_vel_tma(const Target& tg, cudaStream_t s, int dir, const PlaneSrc<VelMaps>& maps,
                         const GeomArrays& ga, const typename S::nd_t* node_flux,
                         const typename S::nd_t* node_mass_pre, typename S::vel_t* const* vel_in,
                         typename S::vel_t* const* vel_out, const Level0<S>& level0, bool xh,
                         int* status) {
-  auto go = [&](auto kern, const MarchRange& r) {
-    int seg;
-    const dim3 grid = plane_grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY,
-                                 r.phi - r.plo + 1, &seg);
-    kern<<<grid, dim3(TX, TY), kVelRing * VelPlane<S>::kBytes, s>>>(
-        g, seg, ga, maps, node_flux, node_mass_pre, vel_in[0], vel_in[1], vel_in[2],
-        vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
+  auto go = [&](auto d) {
+    constexpr int D = decltype(d)::value;
+    GO_BOTH(kKeyMomVel3 | D, tiles_mom_vel<D>, kVelRing * VelPlane<S>::kBytes, maps, VelMaps, k_mom_vel_tma,
+            (D, kVelRing, kVelMinBlocks<S>), ga, node_flux, node_mass_pre, vel_in[0], vel_in[1],
+            vel_in[2], vel_out[0], vel_out[1], vel_out[2], level0, xh, status);
   };
-  if (dir == 2) go(k_mom_vel_tma<S, 2, kVelRing, kVelMinBlocks<S>>, mom_vel_range<2>(g));
-  else go(k_mom_vel_tma<S, 3, kVelRing, kVelMinBlocks<S>>, mom_vel_range<3>(g));
+  if (dir == 2) go(std::integral_constant<int, 2>{});
+  else go(std::integral_constant<int, 3>{});
 }
 
 template <class S>
 constexpr int kCellMinBlocks = sizeof(typename S::arith_t) == 4 ? 4 : 3;
 
+// calls f with the integral constants of the sweep's direction and pre-volume variant
+template <class F>
+void cell_variant(int dir, int var, F f) {
+  using std::integral_constant;
+  if (dir == 2 && var == 2) f(integral_constant<int, 2>{}, integral_constant<int, 2>{});
+  else if (dir == 2) f(integral_constant<int, 2>{}, integral_constant<int, 3>{});
+  else if (var == 4) f(integral_constant<int, 3>{}, integral_constant<int, 4>{});
+  else f(integral_constant<int, 3>{}, integral_constant<int, 5>{});
+}
+
 template <class S>
 bool cell_sweep_tma_prepare() {
   bool ok = true;
-  auto set = [&](auto kern, int bytes) {
-    ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kStencilRing * bytes) == cudaSuccess;
-  };
-  set(k_cell_sweep_tma<S, 2, 2, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 2, 2>::kBytes);
-  set(k_cell_sweep_tma<S, 2, 3, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 2, 3>::kBytes);
-  set(k_cell_sweep_tma<S, 3, 4, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 3, 4>::kBytes);
-  set(k_cell_sweep_tma<S, 3, 5, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 3, 5>::kBytes);
+  const int dv[4][2] = {{2, 2}, {2, 3}, {3, 4}, {3, 5}};
+  for (const auto& q : dv)
+    cell_variant(q[0], q[1], [&](auto d, auto v) {
+      constexpr int D = decltype(d)::value, V = decltype(v)::value;
+      ok = ok && SET_BOTH(CellMaps, (kStencilRing * CellPlane<S, D, V>::kBytes), k_cell_sweep_tma, D, V,
+                          kStencilRing, kCellMinBlocks<S>);
+    });
   return ok;
 }
 
 template <class S>
-void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, const CellMaps& maps,
-                           const GeomArrays& ga, const typename S::rho_t* d_in,
-                           const typename S::ene_t* e_in, typename S::rho_t* d_out,
-                           typename S::ene_t* e_out, const typename S::vf_t* vfx,
-                           const typename S::vf_t* vfy, const typename S::vf_t* vfz,
-                           typename S::mf_t* mass_flux, const Level0<S>& level0, bool xh,
-                           int* status) {
-  auto go = [&](auto kern, int bytes, const MarchRange& r, int pcells) {
-    int seg;
-    const dim3 grid = plane_grid((r.jhi - r.jlo + TX) / TX, (r.chi - r.clo + TY) / TY, pcells, &seg);
-    kern<<<grid, dim3(TX, TY), kStencilRing * bytes, s>>>(g, seg, ga, maps, d_in, e_in,
-                                                          d_out, e_out, vfx, vfy, vfz, mass_flux,
-                                                          level0, xh, status);
-  };
-  const int ny = g.y_max - g.y_min + 1, nz = g.z_max - g.z_min + 1;
-  if (dir == 2) {
-    const MarchRange r = cell_sweep_range<2>(g);
-    if (var == 2) go(k_cell_sweep_tma<S, 2, 2, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 2, 2>::kBytes, r, ny);
-    else go(k_cell_sweep_tma<S, 2, 3, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 2, 3>::kBytes, r, ny);
-  } else {
-    const MarchRange r = cell_sweep_range<3>(g);
-    if (var == 4) go(k_cell_sweep_tma<S, 3, 4, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 3, 4>::kBytes, r, nz);
-    else go(k_cell_sweep_tma<S, 3, 5, kStencilRing, kCellMinBlocks<S>>, CellPlane<S, 3, 5>::kBytes, r, nz);
-  }
+void launch_cell_sweep_tma(const Target& tg, cudaStream_t s, int dir, int var,
+                           const PlaneSrc<CellMaps>& maps, const GeomArrays& ga,
+                           const typename S::rho_t* d_in, const typename S::ene_t* e_in,
+                           typename S::rho_t* d_out, typename S::ene_t* e_out,
+                           const typename S::vf_t* vfx, const typename S::vf_t* vfy,
+                           const typename S::vf_t* vfz, typename S::mf_t* mass_flux,
+                           const Level0<S>& level0, bool xh, int* status) {
+  cell_variant(dir, var, [&](auto d, auto v) {
+    constexpr int D = decltype(d)::value, V = decltype(v)::value;
+    GO_BOTH(kKeyCellSweep | D | (V << 4), tiles_cell<D>, (kStencilRing * CellPlane<S, D, V>::kBytes), maps,
+            CellMaps, k_cell_sweep_tma, (D, V, kStencilRing, kCellMinBlocks<S>), ga, d_in, e_in, d_out,
+            e_out, vfx, vfy, vfz, mass_flux, level0, xh, status);
+  });
 }
 
 #define INST_TMA(S)                                                                              \
-  template bool visc_dt_tma_maps<S>(const Geom&, const S::vel_t*, const S::vel_t*,              \
-                                    const S::vel_t*, const S::rho_t*, const S::ene_t*,          \
-                                    ViscMaps*);                                                  \
   template bool visc_dt_tma_prepare<S>();                                                        \
   template bool mom_x_tma_prepare<S>();                                                          \
   template bool stencils_tma_prepare<S>();                                                       \
   template bool mom_node_tma_prepare<S>();                                                       \
   template bool mom_vel_tma_prepare<S>();                                                        \
   template bool cell_sweep_tma_prepare<S>();                                                     \
-  template void launch_cell_sweep_tma<S>(const Geom&, cudaStream_t, int, int, const CellMaps&,   \
+  template void launch_cell_sweep_tma<S>(const Target&, cudaStream_t, int, int, const PlaneSrc<CellMaps>&,   \
                                          const GeomArrays&, const S::rho_t*, const S::ene_t*,    \
                                          S::rho_t*, S::ene_t*, const S::vf_t*, const S::vf_t*,   \
                                          const S::vf_t*, S::mf_t*, const Level0<S>&, bool, int*); \
-  template void launch_mom_vel_tma<S>(const Geom&, cudaStream_t, int, const VelMaps&,            \
+  template void launch_mom_vel_tma<S>(const Target&, cudaStream_t, int, const PlaneSrc<VelMaps>&,            \
                                       const GeomArrays&, const S::nd_t*, const S::nd_t*,         \
                                       S::vel_t* const*, S::vel_t* const*, const Level0<S>&, bool, int*); \
-  template void launch_mom_node_tma<S>(const Geom&, cudaStream_t, int, int, const NodeMaps&,     \
+  template void launch_mom_node_tma<S>(const Target&, cudaStream_t, int, int, const PlaneSrc<NodeMaps>&,     \
                                        S::nd_t*, S::nd_t*, S::nd_t*, int*);                      \
   template bool cell_sweep_x_tma_prepare<S>();                                                   \
-  template void launch_cell_sweep_x_tma<S>(const Geom&, cudaStream_t, int, const CellXMaps&,     \
+  template void launch_cell_sweep_x_tma<S>(const Target&, cudaStream_t, int, const PlaneSrc<CellXMaps>&,     \
                                            const GeomArrays&, S::rho_t*, S::ene_t*, S::mf_t*,    \
                                            const Level0<S>&, bool, int*);                        \
-  template void launch_pdv_predict_eos_tma<S>(const Geom&, cudaStream_t, const double*,         \
-                                              const PdvMaps&, S::cs_t*, bool, int*);             \
-  template void launch_mom_x_tma<S>(const Geom&, cudaStream_t, int, const MomXMaps&,             \
+  template void launch_pdv_predict_eos_tma<S>(const Target&, cudaStream_t, const double*,         \
+                                              const PlaneSrc<PdvMaps>&, S::cs_t*, bool, int*);             \
+  template void launch_mom_x_tma<S>(const Target&, cudaStream_t, int, const PlaneSrc<MomXMaps>&,             \
                                     const GeomArrays&, S::vel_t* const*, const Level0<S>&, bool, int*); \
-  template void launch_visc_dt_tma<S>(const Geom&, cudaStream_t, const ViscMaps&, const GeomArrays&, \
+  template void launch_visc_dt_tma<S>(const Target&, cudaStream_t, const PlaneSrc<ViscMaps>&, const GeomArrays&, \
                                       double, double, double, double, double, double, S::cs_t*,  \
                                       S::cs_t*, S::cs_t*, unsigned long long*, S::rho_t*, S::ene_t*, bool, int*);
 INST_TMA(F64)
 INST_TMA(F32Mixed)
-template void launch_acc_flux_tma<F64>(const Geom&, cudaStream_t, const double*, const AccMaps&,
+template void launch_acc_flux_tma<F64>(const Target&, cudaStream_t, const double*, const PlaneSrc<AccMaps>&,
                                        F64::rho_t*, const F64::ene_t*, F64::ene_t*, F64::vel_t*,
                                        F64::vel_t*, F64::vel_t*, F64::vf_t*, F64::vf_t*, F64::vf_t*, F64::vel_t*,
                                        F64::vel_t*, bool, int*);
-template void launch_accelerate_tma<F32Mixed>(const Geom&, cudaStream_t, const double*,
-                                         const AccMaps&, F32Mixed::vel_t*, F32Mixed::vel_t*, F32Mixed::vel_t*,
+template void launch_accelerate_tma<F32Mixed>(const Target&, cudaStream_t, const double*,
+                                         const PlaneSrc<AccMaps>&, F32Mixed::vel_t*, F32Mixed::vel_t*, F32Mixed::vel_t*,
                                          F32Mixed::vel_t*, F32Mixed::vel_t*, bool, int*);
-template void launch_pdv_flux_tma<F32Mixed>(const Geom&, cudaStream_t, const double*, const FluxMaps&,
+template void launch_pdv_flux_tma<F32Mixed>(const Target&, cudaStream_t, const double*, const PlaneSrc<FluxMaps>&,
                                        const F32Mixed::rho_t*, F32Mixed::rho_t*, const F32Mixed::ene_t*, F32Mixed::ene_t*,
                                        const F32Mixed::cs_t*, const F32Mixed::cs_t*, F32Mixed::vf_t*, F32Mixed::vf_t*,
                                        F32Mixed::vf_t*, bool, int*);

@@ -40,6 +40,14 @@ constexpr int kTmaWidth = 32 + 2 * kTmaHalo<T>;
 bool encode_plane_map(CUtensorMap* map, const void* base, int elem_bytes, const Geom& g,
                       int box_rows, bool rows_along_z = false);
 
+// The tensor maps a staged launch reads: one chunk's, or over an ensemble every
+// deck's, in deck order in device memory.
+template <class Maps>
+struct PlaneSrc {
+  Maps one;
+  const Maps* decks = nullptr;
+};
+
 // The tensor maps of the arrays the viscosity/calc_dt stencil reads.
 struct ViscMaps {
   CUtensorMap u, v, w, d, e;
@@ -56,7 +64,7 @@ bool mom_x_tma_prepare();
 // The x momentum sweep of one chunk (sweep 1 or 3 of the step), its planes
 // staged by bulk-tensor copies.
 template <class S>
-void launch_mom_x_tma(const Geom& g, cudaStream_t s, int sweep, const MomXMaps& maps,
+void launch_mom_x_tma(const Target& tg, cudaStream_t s, int sweep, const PlaneSrc<MomXMaps>& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
                       const Level0<S>& level0, bool xh, int* status);
 
@@ -81,23 +89,23 @@ constexpr bool kFusedAccFlux = sizeof(typename S::arith_t) == 8;
 template <class S>
 bool stencils_tma_prepare();
 template <class S>
-void launch_pdv_predict_eos_tma(const Geom& g, cudaStream_t s, const double* dt_ptr,
-                                const PdvMaps& maps, typename S::cs_t* pressure, bool xh,
+void launch_pdv_predict_eos_tma(const Target& tg, cudaStream_t s, const double* dt_ptr,
+                                const PlaneSrc<PdvMaps>& maps, typename S::cs_t* pressure, bool xh,
                                 int* status);
 template <class S>
-void launch_accelerate_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
+void launch_accelerate_tma(const Target& tg, cudaStream_t s, const double* dt_ptr, const PlaneSrc<AccMaps>& maps,
                            typename S::vel_t* xvel1, typename S::vel_t* yvel1,
                            typename S::vel_t* zvel1, typename S::vel_t* xvel0, typename S::vel_t* yvel0,
                            bool xh, int* status);
 template <class S>
-void launch_pdv_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const FluxMaps& maps,
+void launch_pdv_flux_tma(const Target& tg, cudaStream_t s, const double* dt_ptr, const PlaneSrc<FluxMaps>& maps,
                          const typename S::rho_t* density0, typename S::rho_t* density1,
                          const typename S::ene_t* energy0, typename S::ene_t* energy1,
                          const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
                          typename S::vf_t* vol_flux_x, typename S::vf_t* vol_flux_y,
                          typename S::vf_t* vol_flux_z, bool xh, int* status);
 template <class S>
-void launch_acc_flux_tma(const Geom& g, cudaStream_t s, const double* dt_ptr, const AccMaps& maps,
+void launch_acc_flux_tma(const Target& tg, cudaStream_t s, const double* dt_ptr, const PlaneSrc<AccMaps>& maps,
                          typename S::rho_t* density1, const typename S::ene_t* energy0,
                          typename S::ene_t* energy1, typename S::vel_t* xvel1,
                          typename S::vel_t* yvel1, typename S::vel_t* zvel1,
@@ -165,7 +173,7 @@ bool cell_sweep_x_tma_prepare();
 // The x cell sweep of the step's sweep 1 or 3, out of place into (d_out,
 // e_out), planes staged by bulk-tensor copies (interior cells only).
 template <class S>
-void launch_cell_sweep_x_tma(const Geom& g, cudaStream_t s, int sweep, const CellXMaps& maps,
+void launch_cell_sweep_x_tma(const Target& tg, cudaStream_t s, int sweep, const PlaneSrc<CellXMaps>& maps,
                              const GeomArrays& ga, typename S::rho_t* d_out,
                              typename S::ene_t* e_out, typename S::mf_t* mass_flux_x,
                              const Level0<S>& level0, bool xh, int* status);
@@ -188,7 +196,7 @@ bool mom_node_tma_prepare();
 // The node pass of the y (dir 2) or z (dir 3) momentum sweep with post-volume
 // variant var, planes staged by bulk-tensor copies.
 template <class S>
-void launch_mom_node_tma(const Geom& g, cudaStream_t s, int dir, int var, const NodeMaps& maps,
+void launch_mom_node_tma(const Target& tg, cudaStream_t s, int dir, int var, const PlaneSrc<NodeMaps>& maps,
                          typename S::nd_t* node_flux, typename S::nd_t* node_mass_post,
                          typename S::nd_t* node_mass_pre, int* status);
 
@@ -202,7 +210,7 @@ struct VelMaps {
 template <class S>
 bool mom_vel_tma_prepare();
 template <class S>
-void launch_mom_vel_tma(const Geom& g, cudaStream_t s, int dir, const VelMaps& maps,
+void launch_mom_vel_tma(const Target& tg, cudaStream_t s, int dir, const PlaneSrc<VelMaps>& maps,
                         const GeomArrays& ga, const typename S::nd_t* node_flux,
                         const typename S::nd_t* node_mass_pre, typename S::vel_t* const* vel_in,
                         typename S::vel_t* const* vel_out, const Level0<S>& level0, bool xh,
@@ -221,7 +229,7 @@ bool cell_sweep_tma_prepare();
 // place from (d_in, e_in) into (d_out, e_out), planes staged by bulk-tensor
 // copies. Needs a depth-2 halo update of density1/energy1 after it.
 template <class S>
-void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, const CellMaps& maps,
+void launch_cell_sweep_tma(const Target& tg, cudaStream_t s, int dir, int var, const PlaneSrc<CellMaps>& maps,
                            const GeomArrays& ga, const typename S::rho_t* d_in,
                            const typename S::ene_t* e_in, typename S::rho_t* d_out,
                            typename S::ene_t* e_out, const typename S::vf_t* vfx,
@@ -229,13 +237,6 @@ void launch_cell_sweep_tma(const Geom& g, cudaStream_t s, int dir, int var, cons
                            typename S::mf_t* mass_flux, const Level0<S>& level0, bool xh,
                            int* status);
 
-// The maps of a chunk's velocities (time level 0), density0 and energy0.
-template <class S>
-bool visc_dt_tma_maps(const Geom& g, const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
-                      const typename S::vel_t* zvel0, const typename S::rho_t* density0,
-                      const typename S::ene_t* energy0, ViscMaps* maps);
-// Once per process before the first launch (outside any stream capture):
-// the kernel's shared-memory size.
 template <class S>
 bool visc_dt_tma_prepare();
 // viscosity + calc_dt (+ ideal_gas) of every interior cell of one chunk, the
@@ -243,7 +244,7 @@ bool visc_dt_tma_prepare();
 // and a block whose copies do not arrive sets CLOVER_STATUS_TIMEOUT in
 // *status.
 template <class S>
-void launch_visc_dt_tma(const Geom& g, cudaStream_t s, const ViscMaps& maps, const GeomArrays& ga,
+void launch_visc_dt_tma(const Target& tg, cudaStream_t s, const PlaneSrc<ViscMaps>& maps, const GeomArrays& ga,
                         double g_small, double dtc_safe, double dtu_safe, double dtv_safe,
                         double dtw_safe, double dtdiv_safe, typename S::cs_t* pressure,
                         typename S::cs_t* viscosity, typename S::cs_t* soundspeed,

@@ -75,11 +75,12 @@ void clover_chunk_use_graphs(clover_chunk *c, int on);
 /* 1 (default) = the fused kernels, 0 = one kernel per reference loop nest.
  * Both give the same results bit for bit. Only before the first step. */
 void clover_chunk_use_fused(clover_chunk *c, int on);
-/* 1 (default) = the fused step's stencils that stage their input planes in
- * shared memory with bulk-tensor (TMA) copies, where the chunk could make
- * their tensor maps; 0 = their register-marching forms. Both give the same
- * results bit for bit. Returns 1 if the staged forms are in use. Ensembles
- * always use the register-marching forms. */
+/* 1 = the fused step's stencils that stage their input planes in shared
+ * memory with bulk-tensor (TMA) copies, where their tensor maps could be made
+ * (the default of a chunk, and of an ensemble whose decks fill the staged
+ * tiles); 0 = their register-marching forms. Both give the same results bit for
+ * bit. Returns 1 if the staged forms are in use. Ensembles with a deck of fewer
+ * than three cells on an axis run the register forms either way. */
 int clover_chunk_use_tma(clover_chunk *c, int on);
 
 /* Self-test of the staged kernels' failure detection (no counterpart in the

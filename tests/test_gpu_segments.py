@@ -36,3 +36,29 @@ def test_native_and_dropin_bitwise_over_segments(nx, ny, nz):
         ch.close()
     for a, b, name in zip(*out, C.FIELD_NAMES):
         assert np.array_equal(a, b), name
+
+
+@pytest.mark.parametrize("precision", [C.PRECISION_FP64, C.PRECISION_MIXED])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_ensemble_staged_and_register_forms(precision, graphs):
+    """Decks around the tiles' and warps' edges, side by side: staged and register forms, and each deck alone."""
+    sizes = [(3, 3, 3), (33, 9, 5), (31, 8, 61), (32, 32, 32), (29, 17, 40), (64, 3, 12), (62, 31, 7)]
+    ds = [decks.to_deck(decks.shock(*n, 6, states=decks.MIXED_STATES)) for n in sizes]
+    runs = []
+    for tma in (True, False):
+        e = C.Ensemble(ds, precision)
+        e.use_graphs(graphs)
+        assert e.use_tma(tma) == tma
+        e.run()
+        runs.append(e)
+    for i, d in enumerate(ds):
+        ch = C.Chunk(d, precision)
+        ch.run()
+        assert all(e.deck_status(i) == 0 for e in runs)
+        assert all(np.array_equal(e.deck_dt_history(i), ch.dt_history()) for e in runs)
+        for name in C.FIELD_NAMES:
+            want = ch.field(name)
+            assert all(np.array_equal(e.deck_field(i, name), want) for e in runs), (i, name)
+        ch.close()
+    for e in runs:
+        e.close()
