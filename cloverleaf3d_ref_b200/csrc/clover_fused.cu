@@ -194,12 +194,15 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
     using C = typename S::cs_t;
 #define PN(jj, kk, ll) \
   ((A)st<C>(((A(1.4) - A(1.0)) * LA(density0, jj, kk, ll) * LA(energy0, jj, kk, ll))))
-    // with xh the x-face halo of density0 and energy0 is written below: a
-    // cell at the face takes its own value, which that halo mirrors
+    // with xh density0's and energy0's halo is still the last step's (its x
+    // faces are written below, the others by a later launch): a cell at a face
+    // takes its own value, which that halo mirrors
     const int jm = xh && j == g.x_min ? j : j - 1, jp = xh && j == g.x_max ? j : j + 1;
+    const int km = xh && k == g.y_min ? k : k - 1, kp = xh && k == g.y_max ? k : k + 1;
+    const int lm = xh && l == g.z_min ? l : l - 1, lp = xh && l == g.z_max ? l : l + 1;
     A pgradx = (PN(jp, k, l) - PN(jm, k, l)) / (cdx + AG(GX, ga.celldx, j + 1));
-    A pgrady = (PN(j, k + 1, l) - PN(j, k - 1, l)) / (cdy + AG(GY, ga.celldy, k + 1));
-    A pgradz = (PN(j, k, l + 1) - PN(j, k, l - 1)) / (cdz + AG(GZ, ga.celldz, l + 1));
+    A pgrady = (PN(j, kp, l) - PN(j, km, l)) / (cdy + AG(GY, ga.celldy, k + 1));
+    A pgradz = (PN(j, k, lp) - PN(j, k, lm)) / (cdz + AG(GZ, ga.celldz, l + 1));
 #undef PN
     const A pgradx2 = pgradx * pgradx;
     const A pgrady2 = pgrady * pgrady;

@@ -366,7 +366,8 @@ void launch_generate_chunk(const Geom& g, cudaStream_t s, const GeomArrays& ga,
 // the rows it stores, as the update_halo that follows would, which then leaves
 // the x faces out (launch_update_halo's x_faces). For decks whose face passes
 // compose. accelerate writes it for xvel0 and yvel0 too, and the viscosity
-// kernel for density0 and energy0 (the step-start update, one layer).
+// kernel for density0 and energy0 (the step-start update, one layer), whose
+// neighbours' values it takes from the interior cells their halo mirrors.
 // viscosity and calc_dt of every interior cell in one pass; the cell minimum
 // folds into min_key (per deck over a plan).
 template <class S>

@@ -33,14 +33,17 @@ std::string g_last_error;
 const double kGSmall = (double)1.0e-16f;
 const double kGBig = (double)1.0e+21f;
 
-// One thread per deck: the key of the calc_dt reduction starts at g_big.
+// One thread per deck: the key of the calc_dt reduction starts at g_big (at
+// set-up and after a restore; k_dt_finalize sets it for the next step).
 __global__ void k_dt_prepare(DevScalars* sc, int nd, unsigned long long init) {
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d < nd) sc[d].key = init;
 }
 
-// timestep.f90:90-126 after the calc_dt reduction, one thread per deck
-__global__ void k_dt_finalize(DevScalars* scs, int nd, double* dt_hist) {
+// timestep.f90:90-126 after the calc_dt reduction, one thread per deck; then the
+// step's hydro.f90:68 (time = time + dt, which no kernel of the step reads) and
+// the key of the next step's reduction, so that neither takes a launch
+__global__ void k_dt_finalize(DevScalars* scs, int nd, double* dt_hist, unsigned long long init) {
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= nd) return;
   DevScalars* sc = scs + d;
@@ -60,12 +63,8 @@ __global__ void k_dt_finalize(DevScalars* scs, int nd, double* dt_hist) {
   const int s = sc->step;
   if (s < sc->dt_cap) dt_hist[(long long)d * sc->dt_cap + s] = dt;
   sc->step = s + 1;
-}
-
-// hydro.f90:68, one thread per deck
-__global__ void k_step_end(DevScalars* sc, int nd) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d < nd) sc[d].time = sc[d].time + sc[d].dt;
+  sc->time = sc->time + dt;
+  sc->key = init;
 }
 
 // Rows of hx elements of a field (row pitch px, plane pitch pxy) to contiguous
@@ -551,6 +550,7 @@ struct Chunk : ChunkBase {
     }
     cudaMemcpyAsync(sc, h.data(), (size_t)nd * sizeof(DevScalars), cudaMemcpyHostToDevice, stream);
     cudaStreamSynchronize(stream);  // h is released at return
+    k_dt_prepare<<<deck_blocks(), 128, 0, stream>>>(sc, nd, min_key_of(kGBig));
     for (int i = 0; i < nd; i++) {
       const clover_deck& d = decks[i];
       const Geom& q = geoms[i];
@@ -706,6 +706,7 @@ struct Chunk : ChunkBase {
       return -5;
     }
     drop_graphs();
+    k_dt_prepare<<<deck_blocks(), 128, 0, stream>>>(sc, nd, min_key_of(kGBig));
     host_step = h.host_step;
     advect_x = h.advect_x != 0;
     fused = h.fused != 0;
@@ -888,15 +889,19 @@ struct Chunk : ChunkBase {
     int vc = ax ? 0 : 1;  // buffer of the velocity pairs at the start of this step
     int cb = ax ? 0 : 1;  // buffer of the density1/energy1 pair at the start of this step
     // timestep.f90:56-126
-    k_dt_prepare<<<deck_blocks(), 128, 0, stream>>>(sc, nd, min_key_of(kGBig));
     // ideal_gas runs inside the viscosity/calc_dt kernel: it stores every
     // cell's pressure and sound speed and forms the neighbours' pressures
-    // from density0/energy0, whose halo is updated first. The step-start
-    // update of the pressure's halo is left out: the depth-1 update after the
-    // predictor rewrites the same cells before anything reads them.
-    pbeg();
-    halo({3, 1, 8, 10}, 1, vc, cb, -1, !xh);
-    pend("update_halo", 0);
+    // from density0/energy0. With xh it mirrors those at the faces itself, and
+    // the step-start update of time level 0 and the viscosity's update join the
+    // pressure's after the predictor (nothing before accelerate reads their
+    // halos); otherwise density0's and energy0's halo is updated first. The
+    // step-start update of the pressure's halo is left out: the depth-1 update
+    // after the predictor rewrites the same cells before anything reads them.
+    if (!xh) {
+      pbeg();
+      halo({3, 1, 8, 10}, 1, vc, cb);
+      pend("update_halo", 0);
+    }
     pbeg();
     PlaneSrc<ViscMaps> visc_m;
     if (maps_for(kKeyTimestepVisc, &visc_m, [&](ViscMaps* m) {
@@ -911,11 +916,13 @@ struct Chunk : ChunkBase {
       launch_visc_dt<S>(tg, stream, ga, kGSmall, deck.dtc_safe, deck.dtu_safe, deck.dtv_safe,
                         deck.dtw_safe, deck.dtdiv_safe, density0, energy0, pressure, viscosity,
                         soundspeed, xvel0, yvel0, zvel0, &sc->key, xh);
-    k_dt_finalize<<<deck_blocks(), 128, 0, stream>>>(sc, nd, dt_hist);
+    k_dt_finalize<<<deck_blocks(), 128, 0, stream>>>(sc, nd, dt_hist, min_key_of(kGBig));
     pend("eos_viscosity_calc_dt", n * (3 * V8 + R8 + E8 + 3 * C8));
-    pbeg();
-    halo({6}, 1, vc, cb, -1, !xh);  // read by accelerate at its neighbours
-    pend("update_halo", 0);
+    if (!xh) {
+      pbeg();
+      halo({6}, 1, vc, cb);  // read by accelerate at its neighbours
+      pend("update_halo", 0);
+    }
     // PdV.f90:50-107: predictor + EOS on the predicted state; revert is implied
     pbeg();
     PlaneSrc<PdvMaps> pdv_m;
@@ -931,7 +938,8 @@ struct Chunk : ChunkBase {
                                 yvel0, zvel0, xh);
     pend("pdv", n * (R8 + E8 + 3 * C8 + 3 * V8));
     pbeg();
-    halo({5}, 1, vc, cb, -1, !xh);
+    if (xh) halo({1, 3, 5, 6, 8, 10}, 1, vc, cb, -1, false);
+    else halo({5}, 1, vc, cb);
     pend("update_halo", 0);
     pbeg();
     PlaneSrc<AccMaps> acc_m;
@@ -1076,7 +1084,6 @@ struct Chunk : ChunkBase {
     sweep(1, ax ? 1 : 3, true);
     sweep(2, 2, true);
     sweep(3, ax ? 3 : 1, false);
-    k_step_end<<<deck_blocks(), 128, 0, stream>>>(sc, nd);
   }
 
   // One hydro step, hydro.f90:52-68 (timestep .. time = time + dt).
@@ -1090,7 +1097,6 @@ struct Chunk : ChunkBase {
     const double R8 = sizeof(R), E8 = sizeof(En), C8 = sizeof(C), V8 = sizeof(V),
                  VF8 = sizeof(VF), MF8 = sizeof(MF), W8 = sizeof(W), G8 = sizeof(double);
     // timestep.f90:56-126
-    k_dt_prepare<<<1, 128, 0, stream>>>(sc, 1, min_key_of(kGBig));
     pbeg();
     launch_ideal_gas<S>(g, stream, density0, energy0, pressure, soundspeed);
     pend("ideal_gas", n * (R8 + E8 + 2 * C8));
@@ -1107,7 +1113,7 @@ struct Chunk : ChunkBase {
     launch_calc_dt<S>(g, stream, ga, kGSmall, deck.dtc_safe, deck.dtu_safe, deck.dtv_safe,
                       deck.dtw_safe, deck.dtdiv_safe, density0, viscosity, soundspeed, xvel0,
                       yvel0, zvel0, (W*)nullptr, &sc->key);
-    k_dt_finalize<<<1, 128, 0, stream>>>(sc, 1, dt_hist);
+    k_dt_finalize<<<1, 128, 0, stream>>>(sc, 1, dt_hist, min_key_of(kGBig));
     pend("calc_dt", n * (4 * G8 + R8 + 2 * C8 + 3 * V8));
     // PdV.f90:50-107 (predictor), accelerate, PdV (corrector), flux_calc
     pbeg();
@@ -1175,7 +1181,6 @@ struct Chunk : ChunkBase {
     launch_reset_field<S>(g, stream, density0, density1, energy0, energy1, xvel0, xvel1, yvel0,
                           yvel1, zvel0, zvel1);
     pend("reset_field", n * (2 * R8 + 2 * E8 + 6 * V8));
-    k_step_end<<<1, 128, 0, stream>>>(sc, 1);
   }
 
   // An ensemble's schedules are built by eager steps (one per sweep order)

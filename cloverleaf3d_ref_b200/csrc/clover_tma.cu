@@ -253,14 +253,18 @@ k_visc_dt_tma(const __grid_constant__ M m, Geom gp, GeomArrays ga, double g_smal
         const A yz = A(0.25) * (vgradz2 - vgradz1) / cdz + A(0.25) * (wgrady2 - wgrady1) / cdy;
         // the neighbours' pressures as ideal_gas stores them
 #define PN(bb, a, b) ((A)st<C>(((A(1.4) - A(1.0)) * DN(bb, a, b) * EN(bb, a, b))))
-        // with xh the x-face halo of density0 and energy0 is written below: a cell at
-        // the face takes its own value, which that halo mirrors
+        // with xh density0's and energy0's halo is still the last step's (its x
+        // faces are written below, the others by a later launch): a cell at a
+        // face takes its own value, which that halo mirrors
         const int jm = xh && j == g.x_min ? 0 : -1, jp = xh && j == g.x_max ? 0 : 1;
+        const int km = xh && k == g.y_min ? 0 : -1, kp = xh && k == g.y_max ? 0 : 1;
+        unsigned char* bzu = xh && l == g.z_max ? bl : bu;
+        unsigned char* bzd = xh && l == g.z_min ? bl : bd;
         A pgradx = (PN(bl, jp, 0) - PN(bl, jm, 0)) /
                    (cdx + (A)ga.celldx[g.o1 + j + 1 - g.x_min + 2]);
-        A pgrady = (PN(bl, 0, 1) - PN(bl, 0, -1)) /
+        A pgrady = (PN(bl, 0, kp) - PN(bl, 0, km)) /
                    (cdy + (A)ga.celldy[g.o1 + k + 1 - g.y_min + 2]);
-        A pgradz = (PN(bu, 0, 0) - PN(bd, 0, 0)) /
+        A pgradz = (PN(bzu, 0, 0) - PN(bzd, 0, 0)) /
                    (cdz + (A)ga.celldz[g.o1 + l + 1 - g.z_min + 2]);
 #undef PN
         const A pgradx2 = pgradx * pgradx;
