@@ -78,8 +78,8 @@ void clover_chunk_use_fused(clover_chunk *c, int on);
 /* 1 = the fused step's stencils that stage their input planes in shared
  * memory with bulk-tensor (TMA) copies, where their tensor maps could be made
  * (the default of a chunk, and of an ensemble whose decks fill the staged
- * tiles); 0 = their register-marching forms. Both give the same results bit for
- * bit. Returns 1 if the staged forms are in use. Ensembles with a deck of fewer
+ * tiles); 0 = their register-marching forms. Both give the same results, in FP64
+ * bit for bit (mixed: but for FP32 values near the subnormal range). Returns 1 if the staged forms are in use. Ensembles with a deck of fewer
  * than three cells on an axis run the register forms either way. */
 int clover_chunk_use_tma(clover_chunk *c, int on);
 
