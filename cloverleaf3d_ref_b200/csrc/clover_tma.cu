@@ -43,9 +43,13 @@ bool encode_plane_map(CUtensorMap* map, const void* base, int elem_bytes, const 
   }
   const int halo = 16 / elem_bytes;
   // the map starts halo columns before x_min (16-byte aligned: x_min is
-  // 128-byte aligned); base points at column x_min - 2
+  // 128-byte aligned); base points at column x_min - 2. A row of the map ends
+  // with the array's row, so an FP32 row is two columns longer than the pitch
+  // and its first two are the row before's last (the front pad's, in the first
+  // row): with px columns the last two, which grids of 26 and 27 (mod 32) cells
+  // along x use, would lie outside the map and read as zeros.
   const char* start = (const char*)base - (long long)(halo - 2) * elem_bytes;
-  const cuuint64_t dims[3] = {(cuuint64_t)g.px, (cuuint64_t)(g.pxy / g.px),
+  const cuuint64_t dims[3] = {(cuuint64_t)(g.px + halo - 2), (cuuint64_t)(g.pxy / g.px),
                               (cuuint64_t)(g.z_max - g.z_min + 6)};
   const cuuint64_t strides[2] = {(cuuint64_t)g.px * elem_bytes, (cuuint64_t)g.pxy * elem_bytes};
   // a box is one plane of box_rows rows: rows along y (x-y planes), or along

@@ -9,13 +9,14 @@
 // neighbour from shared memory.
 //
 // Tensor maps describe one array of one chunk in the chunk layout
-// (clover_layout.cuh): dimensions (px, rows, planes), row and plane strides
-// in bytes. A copy must start on a 16-byte boundary along x, so the map's
-// base is the element H = 16 / sizeof(T) columns before x_min (element
+// (clover_layout.cuh). A copy must start on a 16-byte boundary along x, so the
+// map's base is the element H = 16 / sizeof(T) columns before x_min (element
 // x_min is 128-byte aligned in every array) and a tile whose first column is
 // x_min + 32 t starts its box at x coordinate 32 t, H columns before it; the
-// box is 32 + 2 H columns wide. Rows and planes have no alignment rule, and a
-// box that runs past the array's end reads zeros there.
+// box is 32 + 2 H columns wide. A row of the map ends with the array's row:
+// dimensions (px + H - 2, rows, planes), the array's row and plane strides in
+// bytes. Rows and planes have no alignment rule, and a box that runs past the
+// array's end reads zeros there.
 //
 // Only loads (no multicast): each block reads this GPU's own arrays.
 #pragma once

@@ -62,3 +62,35 @@ def test_ensemble_staged_and_register_forms(precision, graphs):
         ch.close()
     for e in runs:
         e.close()
+
+
+ROWS = (24, 25, 26, 27, 28, 29, 58, 59, 91)
+
+
+def test_mixed_forms_agree_at_every_row_length():
+    """Flow along x up to the far wall, rows that end at each place in their pitch: staged and register forms of a
+    chunk, and of ensembles, whichever decks share them."""
+    ds = [decks.to_deck(decks.shock(nx, 9, 6, 14, states=decks.MIXED_STATES)) for nx in ROWS]
+    want = []
+    for d in ds:
+        out = []
+        for tma in (True, False):
+            ch = C.Chunk(d, C.PRECISION_MIXED)
+            assert ch.use_tma(tma) == tma
+            ch.run()
+            assert ch.status == 0
+            out.append({n: ch.field(n) for n in C.FIELD_NAMES})
+            ch.close()
+        want.append(out[1])
+        for n in C.FIELD_NAMES:
+            assert np.array_equal(out[0][n], out[1][n]), (d.s.x_cells, n)
+    for tma in (True, False):
+        for part in (ds, ds[2:4]):
+            e = C.Ensemble(part, C.PRECISION_MIXED)
+            assert e.use_tma(tma) == tma
+            e.run()
+            for i, d in enumerate(part):
+                ref = want[ds.index(d)]
+                for n in C.FIELD_NAMES:
+                    assert np.array_equal(e.deck_field(i, n), ref[n]), (d.s.x_cells, n, tma)
+            e.close()
