@@ -1,4 +1,6 @@
 """Fields written and read back: one piece, and several pieces of whole planes."""
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -35,4 +37,27 @@ def test_summaries_of_each_deck_of_an_ensemble():
         short, s2 = e.deck_summaries(i, cap=2)
         assert np.array_equal(short, got[:2]) and np.array_equal(s2, steps[:2])
         ch.close()
+    e.close()
+
+
+@pytest.mark.parametrize("precision", [C.PRECISION_FP64, C.PRECISION_MIXED])
+def test_threads_read_one_chunk(precision):
+    """Every field of a chunk (each in several pieces), and of an ensemble's decks, read by eight threads at once."""
+    n = (150, 190, 190)  # 45 MB of doubles a field
+    ch = C.Chunk(decks.to_deck(decks.shock(*n, 4)), precision)
+    rng = np.random.default_rng(11)
+    for name in C.FIELD_NAMES:
+        ch.set_field(name, np.asfortranarray(rng.standard_normal(C.field_shape(name, *n), dtype=np.float32)
+                                             .astype(np.float64)))
+    e = C.Ensemble([decks.to_deck(decks.shock(*s, 4)) for s in ((8, 9, 10), (70, 61, 50), (33, 20, 90))], precision)
+    e.run()
+    with ThreadPoolExecutor(8) as pool:
+        got = list(pool.map(ch.field, C.FIELD_NAMES))
+        jobs = [(i, name) for _ in range(4) for name in C.FIELD_NAMES for i in range(3)]
+        parts = list(pool.map(lambda job: e.deck_field(*job), jobs))
+    for name, a in zip(C.FIELD_NAMES, got):
+        assert np.array_equal(a, ch.field(name)), name
+    for (i, name), a in zip(jobs, parts):
+        assert np.array_equal(a, e.deck_field(i, name)), (i, name)
+    ch.close()
     e.close()
