@@ -319,6 +319,13 @@ __device__ __forceinline__ void tma_load_box(void* dst, const CUtensorMap* map,
       : "memory");
 }
 
+// Order this thread's later loads through a map in global memory after the host
+// copy that wrote it (the map is read by another proxy than the copy wrote through).
+__device__ __forceinline__ void tma_map_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"((unsigned long long)map)
+               : "memory");
+}
+
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)map) : "memory");
 }

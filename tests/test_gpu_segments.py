@@ -94,3 +94,27 @@ def test_mixed_forms_agree_at_every_row_length():
                 for n in C.FIELD_NAMES:
                     assert np.array_equal(e.deck_field(i, n), ref[n]), (d.s.x_cells, n, tma)
             e.close()
+
+
+@pytest.mark.parametrize("precision", [C.PRECISION_FP64, C.PRECISION_MIXED])
+def test_ensembles_one_after_another(precision):
+    """Ensembles of other sizes and numbers of decks, whose device memory lies where the last one's lay: each deck of
+    each against itself alone."""
+    sizes = [(40, 33, 12), (33, 40, 9), (64, 20, 7), (31, 31, 31), (70, 16, 10), (20, 48, 24)]
+    ds = [decks.to_deck(decks.shock(*n, 5, states=decks.MIXED_STATES)) for n in sizes]
+    want = []
+    for d in ds:
+        ch = C.Chunk(d, precision)
+        ch.run()
+        want.append([ch.field(n) for n in C.FIELD_NAMES])
+        ch.close()
+    for r in range(12):
+        part = [(r + i * (1 + r % 2)) % 6 for i in range(1 + r % 4)]
+        e = C.Ensemble([ds[i] for i in part], precision)
+        assert e.use_tma(True)
+        e.run()
+        for at, i in enumerate(part):
+            assert e.deck_status(at) == 0
+            for n, w in zip(C.FIELD_NAMES, want[i]):
+                assert np.array_equal(e.deck_field(at, n), w), (r, sizes[i], n)
+        e.close()
