@@ -165,54 +165,154 @@ struct Chunk : ChunkBase {
   bool advect_x = true;  // start.f90:99
   bool use_graphs = true;
   bool fused = true;  // fused kernels (clover_fused.cu) instead of one kernel per reference pass
-  // stencils staged through shared memory by bulk-tensor copies (clover_tma.cu)
-  // where their tensor maps could be made; their register-marching forms otherwise
-  bool tma = false;
-  bool use_tma = true;
-  // tensor maps of the arrays the staged kernels read, by (array, box rows
-  // and orientation): both buffers of the density1 and velocity pairs occur
-  std::map<std::pair<const void*, int>, CUtensorMap> tmaps;
-  const Geom* mg = &g;  // the deck whose part of an array tmap() describes
-  // an ensemble's maps, every deck's, in device memory (null: the driver refused one)
-  std::map<unsigned, void*> deck_maps;
-  // The maps of a staged launch, filled by fill(Maps*) for one deck at a time;
-  // key: the launch and the buffers it reads (ensembles, built on first use
-  // like the schedules). False: the register form runs.
+  // stencils staged through shared memory by bulk-tensor copies (clover_tma.cu),
+  // or their register-marching forms
+  bool tma = false;      // the staged kernels could be set up
+  bool use_tma = false;  // they run; only with their maps made (make_maps)
+  // The tensor maps of the staged launches are made before the first of them
+  // runs, all or none: the buffer a step leaves density1 and energy1 in follows
+  // from the number of sweeps that write out of place. One chunk: by (array, box
+  // rows and orientation), since both buffers of the density1 and velocity pairs
+  // occur. An ensemble: every deck's maps of a launch side by side, in one table
+  // in device memory.
+  std::map<std::pair<const void*, int>, CUtensorMap> tmaps;  // of the deck mg
+  const Geom* mg = &g;                                       // the deck whose part of an array tmap() describes
+  bool maps_made = false;
+  unsigned char* deck_maps = nullptr;   // ensemble: the table
+  std::map<unsigned, size_t> maps_at;   // a launch's place in it
+  std::vector<unsigned char>* map_image = nullptr;  // the table's host copy, while it is made
+  // The maps of a staged launch, which fill(Maps*) sets for one deck; key: the
+  // launch and the buffers it reads. False: the register form runs.
   template <class Maps, class F>
   bool maps_for(unsigned key, PlaneSrc<Maps>* src, F fill) {
-    if (!(tma && use_tma)) return false;
+    if (map_image) {
+      Maps m{};
+      if (!fill(&m)) return false;
+      if (plan) {
+        const size_t at = maps_at.emplace(key, map_image->size()).first->second;
+        if (at == map_image->size()) map_image->resize(at + nd * sizeof(Maps));
+        memcpy(map_image->data() + at + (mg - geoms.data()) * sizeof(Maps), &m, sizeof(m));
+      }
+      return true;
+    }
+    if (!use_tma) return false;
     if (!plan) return fill(&src->one);
-    if (!halo_repeat_free) return false;
-    auto it = deck_maps.find(key);
-    if (it == deck_maps.end()) {
-      if (plan->capturing) {
-        plan->missing = true;
-        return false;
-      }
-      std::vector<Maps> all(nd);
-      bool ok = true;
-      for (int d = 0; d < nd && ok; d++) {
+    src->decks = (const Maps*)(deck_maps + maps_at.find(key)->second);
+    return true;
+  }
+  // Make the maps of every staged launch of both sweep orders; false, with none
+  // of them in use, if the driver refuses one or the table finds no room.
+  bool make_maps() {
+    if (maps_made || !tma || (plan && !halo_repeat_free)) return maps_made;
+    std::vector<unsigned char> image;
+    map_image = &image;
+    maps_at.clear();
+    bool ok = true;
+    for (int d = 0; d < nd && ok; d++) {
+      if (plan) {
         mg = &geoms[d];
-        ok = fill(&all[d]);
+        tmaps.clear();
       }
-      mg = &g;
+      ok = step_maps(true) && step_maps(false);
+    }
+    map_image = nullptr;
+    mg = &g;
+    if (plan) {
+      tmaps.clear();
       void* dev = nullptr;
-      if (ok && cudaMalloc(&dev, nd * sizeof(Maps)) != cudaSuccess) {
-        cudaGetLastError();
-        dev = nullptr;
-      }
-      // on the launch's stream, and complete before the host copy goes away
-      if (dev && (cudaMemcpyAsync(dev, all.data(), nd * sizeof(Maps), cudaMemcpyHostToDevice, stream) !=
-                      cudaSuccess ||
-                  cudaStreamSynchronize(stream) != cudaSuccess)) {
+      ok = ok && cudaMalloc(&dev, image.size()) == cudaSuccess;
+      // on the launches' stream, and complete before the host copy goes away
+      ok = ok && cudaMemcpyAsync(dev, image.data(), image.size(), cudaMemcpyHostToDevice, stream) == cudaSuccess &&
+           cudaStreamSynchronize(stream) == cudaSuccess;
+      if (!ok) {
         cudaGetLastError();
         cudaFree(dev);
         dev = nullptr;
       }
-      it = deck_maps.emplace(key, dev).first;
+      deck_maps = (unsigned char*)dev;
     }
-    src->decks = (const Maps*)it->second;
-    return it->second != nullptr;
+    return maps_made = ok;
+  }
+  // the staged launches of one step, in enqueue_step_fused's order
+  bool step_maps(bool ax) {
+    int vc = ax ? 0 : 1, cb = ax ? 0 : 1;
+    PlaneSrc<ViscMaps> visc_m;
+    PlaneSrc<PdvMaps> pdv_m;
+    PlaneSrc<AccMaps> acc_m;
+    PlaneSrc<FluxMaps> flux_m;
+    bool ok = visc_src(&visc_m) && pdv_src(&pdv_m) && acc_src(&acc_m) && (kFusedAccFlux<S> || flux_src(vc, &flux_m));
+    for (int sweep = 1; sweep <= 3 && ok; sweep++) {
+      const int dir = sweep == 2 ? 2 : (sweep == 1) == ax ? 1 : 3;
+      PlaneSrc<CellXMaps> cx;
+      PlaneSrc<CellMaps> cm;
+      PlaneSrc<MomXMaps> xm;
+      PlaneSrc<NodeMaps> nm;
+      PlaneSrc<VelMaps> vm;
+      if (dir == 1) ok = cell_x_src(sweep, cb, &cx);
+      else if (halo_repeat_free) ok = cell_src(ax, sweep, dir, cb, &cm);
+      if (dir == 1 || halo_repeat_free) cb ^= 1;
+      ok = ok && (dir == 1 ? mom_x_src(sweep, cb, vc, &xm)
+                           : node_src(ax, sweep, dir, cb, &nm) && vel_src(dir, vc, &vm));
+      vc ^= 1;
+    }
+    return ok;
+  }
+  bool visc_src(PlaneSrc<ViscMaps>* p) {
+    return maps_for(kKeyTimestepVisc, p, [&](ViscMaps* m) {
+      return tmap(xvel0, sizeof(V), 9, &m->u) && tmap(yvel0, sizeof(V), 9, &m->v) &&
+             tmap(zvel0, sizeof(V), 9, &m->w) && tmap(density0, sizeof(R), 10, &m->d) &&
+             tmap(energy0, sizeof(En), 10, &m->e);
+    });
+  }
+  bool pdv_src(PlaneSrc<PdvMaps>* p) {
+    return maps_for(kKeyPdvPredict, p, [&](PdvMaps* m) {
+      return tmap(xvel0, sizeof(V), 9, &m->u) && tmap(yvel0, sizeof(V), 9, &m->v) &&
+             tmap(zvel0, sizeof(V), 9, &m->w) && tmap(density0, sizeof(R), 8, &m->d) &&
+             tmap(energy0, sizeof(En), 8, &m->e) && tmap(pressure, sizeof(C), 8, &m->p) &&
+             tmap(viscosity, sizeof(C), 8, &m->q);
+    });
+  }
+  bool acc_src(PlaneSrc<AccMaps>* p) {
+    return maps_for(kKeyAccelerate, p, [&](AccMaps* m) {
+      return tmap(density0, sizeof(R), 9, &m->d) && tmap(pressure, sizeof(C), 9, &m->p) &&
+             tmap(viscosity, sizeof(C), 9, &m->q) && tmap(xvel0, sizeof(V), 8, &m->u) &&
+             tmap(yvel0, sizeof(V), 8, &m->v) && tmap(zvel0, sizeof(V), 8, &m->w);
+    });
+  }
+  bool flux_src(int vc, PlaneSrc<FluxMaps>* p) {
+    return maps_for(kKeyPdvFlux | (unsigned)vc, p, [&](FluxMaps* m) {
+      return tmap(xvel0, sizeof(V), 9, &m->u0) && tmap(yvel0, sizeof(V), 9, &m->v0) &&
+             tmap(zvel0, sizeof(V), 9, &m->w0) && tmap(vel1(0, vc), sizeof(V), 9, &m->u1) &&
+             tmap(vel1(1, vc), sizeof(V), 9, &m->v1) && tmap(vel1(2, vc), sizeof(V), 9, &m->w1);
+    });
+  }
+  bool cell_x_src(int sweep, int cb, PlaneSrc<CellXMaps>* p) {
+    return maps_for(kKeyCellSweepX | (unsigned)(sweep << 1 | cb), p,
+                    [&](CellXMaps* m) { return cell_x_maps(sweep, cb, m); });
+  }
+  // the pre-volume variant of the y or z cell sweep, the post-volume variant of
+  // the node pass
+  static int cell_var(bool ax, int sweep, int dir) { return dir == 2 ? (ax ? 2 : 3) : (sweep == 1 ? 4 : 5); }
+  static int node_var(bool ax, int sweep, int dir) { return dir == 2 ? (ax ? 2 : 3) : (sweep == 1 ? 1 : 4); }
+  bool cell_src(bool ax, int sweep, int dir, int cb, PlaneSrc<CellMaps>* p) {
+    const int var = cell_var(ax, sweep, dir);
+    return maps_for(kKeyCellSweep | (unsigned)(dir << 6 | var << 1 | cb), p,
+                    [&](CellMaps* m) { return cell_maps(dir, var, cb, m); });
+  }
+  bool mom_x_src(int sweep, int cb, int vc, PlaneSrc<MomXMaps>* p) {
+    V* vin[3] = {vel1(0, vc), vel1(1, vc), vel1(2, vc)};
+    return maps_for(kKeyMomSweepX | (unsigned)(sweep << 2 | cb << 1 | vc), p,
+                    [&](MomXMaps* m) { return mom_x_maps(rho1(cb), vin, m); });
+  }
+  bool node_src(bool ax, int sweep, int dir, int cb, PlaneSrc<NodeMaps>* p) {
+    const int var = node_var(ax, sweep, dir);
+    return maps_for(kKeyMomNode | (unsigned)(dir << 6 | var << 1 | cb), p,
+                    [&](NodeMaps* m) { return mom_node_maps(dir, var, rho1(cb), m); });
+  }
+  bool vel_src(int dir, int vc, PlaneSrc<VelMaps>* p) {
+    V* vin[3] = {vel1(0, vc), vel1(1, vc), vel1(2, vc)};
+    return maps_for(kKeyMomVel3 | (unsigned)(dir << 6 | vc), p,
+                    [&](VelMaps* m) { return mom_vel_maps(dir, vin, m); });
   }
   bool tmap(const void* base, int elem_bytes, int rows, CUtensorMap* out, bool zrows = false) {
     const void* at = (const char*)base + mg->o3 * elem_bytes;
@@ -226,8 +326,6 @@ struct Chunk : ChunkBase {
     *out = it->second;
     return true;
   }
-  // the maps of the x momentum sweep reading density1 buffer rho and the
-  // velocity buffers vin
   // the maps of the y (dir 2) or z (dir 3) node pass reading density1 buffer
   // rho, with the post-volume variant of the sweep
   bool mom_node_maps(int dir, int var, const R* rho, NodeMaps* m) {
@@ -250,8 +348,6 @@ struct Chunk : ChunkBase {
            tmap(vin[0], sizeof(V), 8, &m->u, zr) &&
            tmap(vin[1], sizeof(V), 8, &m->v, zr) && tmap(vin[2], sizeof(V), 8, &m->w, zr);
   }
-  // the maps of the staged y (dir 2) or z (dir 3) cell sweep reading buffer cb
-  // of the density1/energy1 pair, with pre-volume variant var
   // the maps of the staged x cell sweep of sweep 1 or 3 reading buffer cb of
   // the density1/energy1 pair
   bool cell_x_maps(int sweep, int cb, CellXMaps* m) {
@@ -261,6 +357,8 @@ struct Chunk : ChunkBase {
       ok = tmap(vol_flux_y, sizeof(VF), 9, &m->vfy) && tmap(vol_flux_z, sizeof(VF), 8, &m->vfz);
     return ok;
   }
+  // the maps of the staged y (dir 2) or z (dir 3) cell sweep reading buffer cb
+  // of the density1/energy1 pair, with pre-volume variant var
   bool cell_maps(int dir, int var, int cb, CellMaps* m) {
     const bool zr = dir == 2;
     bool ok = tmap(rho1(cb), sizeof(R), 8, &m->d, zr) && tmap(ene1(cb), sizeof(En), 8, &m->e, zr) &&
@@ -271,6 +369,8 @@ struct Chunk : ChunkBase {
     if (ok && var == 4) ok = tmap(vol_flux_y, sizeof(VF), 9, &m->vfr, false);
     return ok;
   }
+  // the maps of the x momentum sweep reading density1 buffer rho and the
+  // velocity buffers vin
   bool mom_x_maps(const R* rho, V* const* vin, MomXMaps* m) {
     return tmap(mass_flux_x, sizeof(MF), 9, &m->mf) && tmap(rho, sizeof(R), 9, &m->d) &&
            tmap(vol_flux_y, sizeof(VF), 10, &m->vfy) && tmap(vol_flux_z, sizeof(VF), 9, &m->vfz) &&
@@ -471,12 +571,12 @@ struct Chunk : ChunkBase {
     }
     ga = GeomArrays{volume, xarea, yarea, zarea, cellx, celly, cellz, celldx, celldy, celldz,
                     vertexx, vertexy, vertexz, vertexdx, vertexdy, vertexdz};
-    // the stencils that stage their planes with bulk-tensor copies get their
-    // tensor maps when they first run (the arrays they read never move)
+    // the stencils that stage their planes with bulk-tensor copies, and their
+    // tensor maps (the arrays they read never move)
     tma = visc_dt_tma_prepare<S>() && mom_x_tma_prepare<S>() && stencils_tma_prepare<S>() &&
           mom_node_tma_prepare<S>() && mom_vel_tma_prepare<S>() && cell_sweep_tma_prepare<S>() &&
           cell_sweep_x_tma_prepare<S>();
-    use_tma = staged_by_default();
+    use_tma = staged_by_default() && make_maps();
 
     dt_cap = deck.end_step < (1 << 22) ? deck.end_step + 16 : (1 << 22);
     sum_cap = dt_cap / (deck.summary_frequency > 0 ? deck.summary_frequency : dt_cap) + 8;
@@ -905,11 +1005,7 @@ struct Chunk : ChunkBase {
     }
     pbeg();
     PlaneSrc<ViscMaps> visc_m;
-    if (maps_for(kKeyTimestepVisc, &visc_m, [&](ViscMaps* m) {
-          return tmap(xvel0, sizeof(V), 9, &m->u) && tmap(yvel0, sizeof(V), 9, &m->v) &&
-                 tmap(zvel0, sizeof(V), 9, &m->w) && tmap(density0, sizeof(R), 10, &m->d) &&
-                 tmap(energy0, sizeof(En), 10, &m->e);
-        }))
+    if (visc_src(&visc_m))
       launch_visc_dt_tma<S>(tg, stream, visc_m, ga, kGSmall, deck.dtc_safe, deck.dtu_safe,
                             deck.dtv_safe, deck.dtw_safe, deck.dtdiv_safe, pressure, viscosity,
                             soundspeed, &sc->key, density0, energy0, xh, &sc->status);
@@ -927,12 +1023,7 @@ struct Chunk : ChunkBase {
     // PdV.f90:50-107: predictor + EOS on the predicted state; revert is implied
     pbeg();
     PlaneSrc<PdvMaps> pdv_m;
-    if (maps_for(kKeyPdvPredict, &pdv_m, [&](PdvMaps* m) {
-          return tmap(xvel0, sizeof(V), 9, &m->u) && tmap(yvel0, sizeof(V), 9, &m->v) &&
-                 tmap(zvel0, sizeof(V), 9, &m->w) && tmap(density0, sizeof(R), 8, &m->d) &&
-                 tmap(energy0, sizeof(En), 8, &m->e) && tmap(pressure, sizeof(C), 8, &m->p) &&
-                 tmap(viscosity, sizeof(C), 8, &m->q);
-        }))
+    if (pdv_src(&pdv_m))
       launch_pdv_predict_eos_tma<S>(tg, stream, dtp, pdv_m, pressure, xh, &sc->status);
     else
       launch_pdv_predict_eos<S>(tg, stream, dtp, ga, density0, energy0, pressure, viscosity, xvel0,
@@ -944,11 +1035,7 @@ struct Chunk : ChunkBase {
     pend("update_halo", 0);
     pbeg();
     PlaneSrc<AccMaps> acc_m;
-    const bool acc_tma = maps_for(kKeyAccelerate, &acc_m, [&](AccMaps* m) {
-      return tmap(density0, sizeof(R), 9, &m->d) && tmap(pressure, sizeof(C), 9, &m->p) &&
-             tmap(viscosity, sizeof(C), 9, &m->q) && tmap(xvel0, sizeof(V), 8, &m->u) &&
-             tmap(yvel0, sizeof(V), 8, &m->v) && tmap(zvel0, sizeof(V), 8, &m->w);
-    });
+    const bool acc_tma = acc_src(&acc_m);
     bool fused_flux = false;
     if constexpr (kFusedAccFlux<S>) {
       fused_flux = acc_tma;
@@ -975,11 +1062,7 @@ struct Chunk : ChunkBase {
       staged = false;
       if constexpr (!kFusedAccFlux<S>) {
         PlaneSrc<FluxMaps> flux_m;
-        staged = maps_for(kKeyPdvFlux | (unsigned)vc, &flux_m, [&](FluxMaps* m) {
-          return tmap(xvel0, sizeof(V), 9, &m->u0) && tmap(yvel0, sizeof(V), 9, &m->v0) &&
-                 tmap(zvel0, sizeof(V), 9, &m->w0) && tmap(vel1(0, vc), sizeof(V), 9, &m->u1) &&
-                 tmap(vel1(1, vc), sizeof(V), 9, &m->v1) && tmap(vel1(2, vc), sizeof(V), 9, &m->w1);
-        });
+        staged = flux_src(vc, &flux_m);
         if (staged)
           launch_pdv_flux_tma<S>(tg, stream, dtp, flux_m, density0, rho1(cb), energy0, ene1(cb),
                                  pressure, viscosity, vol_flux_x, vol_flux_y, vol_flux_z, xh,
@@ -1016,9 +1099,7 @@ struct Chunk : ChunkBase {
         // one pass, out of place into the other buffer of the pair
         // the post-sweep depth-2 halo update rewrites the output pair's shell
         PlaneSrc<CellXMaps> xm;
-        const bool x_tma =
-            maps_for(kKeyCellSweepX | (unsigned)(sweep_number << 1 | cb), &xm,
-                     [&](CellXMaps* m) { return cell_x_maps(sweep_number, cb, m); });
+        const bool x_tma = cell_x_src(sweep_number, cb, &xm);
         launch_advec_cell_x<S>(tg, stream, sweep_number, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
                                ene1(cb ^ 1), vol_flux_x, vol_flux_y, vol_flux_z, mass_flux_x,
                                !halo_repeat_free, l0, xh, x_tma ? &xm : nullptr, &sc->status);
@@ -1028,11 +1109,9 @@ struct Chunk : ChunkBase {
         // one marching pass: staged and out of place into the other buffer of
         // the pair where the depth-2 halo update that follows rewrites the
         // output's shell, in place otherwise
-        const int cvar = dir == 2 ? (axi ? 2 : 3) : (sweep_number == 1 ? 4 : 5);
         PlaneSrc<CellMaps> cm;
-        if (halo_repeat_free && maps_for(kKeyCellSweep | (unsigned)(dir << 6 | cvar << 1 | cb), &cm,
-                                         [&](CellMaps* m) { return cell_maps(dir, cvar, cb, m); })) {
-          launch_cell_sweep_tma<S>(tg, stream, dir, cvar, cm, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
+        if (halo_repeat_free && cell_src(ax, sweep_number, dir, cb, &cm)) {
+          launch_cell_sweep_tma<S>(tg, stream, dir, cell_var(ax, sweep_number, dir), cm, ga, rho1(cb), ene1(cb), rho1(cb ^ 1),
                                    ene1(cb ^ 1), vol_flux_x, vol_flux_y, vol_flux_z,
                                    dir == 2 ? mass_flux_y : mass_flux_z, l0, xh, &sc->status);
           cb ^= 1;
@@ -1060,14 +1139,9 @@ struct Chunk : ChunkBase {
       PlaneSrc<MomXMaps> xm;
       PlaneSrc<NodeMaps> nm;
       PlaneSrc<VelMaps> vm;
-      const int node_var = dir == 2 ? (axi ? 2 : 3) : (sweep_number == 1 ? 1 : 4);
-      const bool x_tma = dir == 1 && maps_for(kKeyMomSweepX | (unsigned)(sweep_number << 2 | cb << 1 | vc), &xm,
-                                              [&](MomXMaps* m) { return mom_x_maps(rho1(cb), vin, m); });
-      const bool node_tma =
-          dir != 1 && maps_for(kKeyMomNode | (unsigned)(dir << 6 | node_var << 1 | cb), &nm,
-                               [&](NodeMaps* m) { return mom_node_maps(dir, node_var, rho1(cb), m); });
-      const bool vel_tma = dir != 1 && maps_for(kKeyMomVel3 | (unsigned)(dir << 6 | vc), &vm,
-                                                [&](VelMaps* m) { return mom_vel_maps(dir, vin, m); });
+      const bool x_tma = dir == 1 && mom_x_src(sweep_number, cb, vc, &xm);
+      const bool node_tma = dir != 1 && node_src(ax, sweep_number, dir, cb, &nm);
+      const bool vel_tma = dir != 1 && vel_src(dir, vc, &vm);
       launch_advec_mom_fused<S>(tg, stream, axi, sweep_number, dir, cell_volume, ga, rho1(cb),
                                 mass_flux_x, mass_flux_y, mass_flux_z, vol_flux_x, vol_flux_y,
                                 vol_flux_z, work[0], work[1], work[2], vin, vout,
@@ -1385,7 +1459,7 @@ struct Chunk : ChunkBase {
     delete plan;
     cudaFree(plane_base);
     cudaFree(read_buf);
-    for (auto& kv : deck_maps) cudaFree(kv.second);
+    cudaFree(deck_maps);
     cudaFree(sc);
     cudaFree(dt_hist);
     cudaFree(sum_hist);
@@ -1713,11 +1787,12 @@ void clover_chunk_use_fused(clover_chunk* c, int on) {
 
 int clover_chunk_use_tma(clover_chunk* c, int on) {
   auto set = [&](auto* ch) {
-    if (ch->use_tma != (on != 0)) {
-      ch->use_tma = on != 0;
+    const bool staged = on != 0 && ch->make_maps();
+    if (ch->use_tma != staged) {
+      ch->use_tma = staged;
       ch->drop_graphs();  // the captured steps hold the other kernels
     }
-    return ch->tma && ch->use_tma && (!ch->plan || ch->halo_repeat_free) ? 1 : 0;
+    return staged ? 1 : 0;
   };
   return c->f64 ? set(c->f64) : set(c->mixed);
 }

@@ -5,6 +5,7 @@ the first, last and shortest segments fall on other planes as a grid grows: one
 plane per block on the smallest grids, up to 32 on the largest."""
 import numpy as np
 import pytest
+import torch
 
 import cloverleaf3d_ref_b200 as C
 import decks
@@ -118,3 +119,34 @@ def test_ensembles_one_after_another(precision):
             for n, w in zip(C.FIELD_NAMES, want[i]):
                 assert np.array_equal(e.deck_field(at, n), w), (r, sizes[i], n)
         e.close()
+
+
+def test_no_room_for_the_maps():
+    """An ensemble whose tensor maps find no room on the device says so, keeps the register forms for every launch and
+    runs on; with room again it takes the staged forms."""
+    ds = [decks.to_deck(decks.shock(8 + i % 5, 8 + i % 3, 9, 12, states=decks.MIXED_STATES)) for i in range(400)]
+    e = C.Ensemble(ds)  # too small for the staged forms by default
+    e.step(4)
+    e.sync()
+    ballast, size = [], 1 << 34
+    try:
+        while size >= 1 << 18:
+            try:
+                ballast.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.cuda.OutOfMemoryError:
+                size //= 2
+        assert not e.use_tma(True)
+    finally:
+        ballast.clear()
+        torch.cuda.empty_cache()
+    e.step(3)
+    assert e.use_tma(True)
+    e.step(5)
+    for i in range(0, 400, 41):
+        ch = C.Chunk(ds[i])
+        ch.step(12)
+        assert np.array_equal(e.deck_dt_history(i), ch.dt_history())
+        for n in C.FIELD_NAMES:
+            assert np.array_equal(e.deck_field(i, n), ch.field(n)), (i, n)
+        ch.close()
+    e.close()
