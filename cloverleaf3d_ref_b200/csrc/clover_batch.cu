@@ -8,7 +8,7 @@
 //             by deck from the deck with the most tiles down, 2 round robin
 //             over the decks (tile i of every deck before tile i+1)
 //   grid_div  0: one block per item; n > 0: the blocks that fit on the GPU
-//             at the kernel's occupancy, divided by n
+//             at the kernel's occupancy, divided by n (staged launches: always 0)
 //   seg       segment length of a marching kernel (planes per thread)
 // Schedules are built on first use and cached by (key, order, grid_div,
 // seg); building allocates and copies, so it runs outside stream capture.
@@ -59,6 +59,9 @@ SchedCfg BatchPlan::cfg_for(unsigned key) const {
     if (trial.grid_div >= 0) c.grid_div = trial.grid_div;
     if (trial.seg >= 0) c.seg = trial.seg;
   }
+  // a staged block takes one item: other divisors would be the same launch under
+  // more schedules, each with its list of items in device memory
+  if (key & kKeyStaged) c.grid_div = 0;
   return c;
 }
 

@@ -2653,7 +2653,7 @@ int plane_seg(long long tiles, int planes) {
 // Launch a staged march: tiles(g, seg) is a chunk's grid with segments of at
 // most seg planes (tiles(g, 1).z = its planes). Over an ensemble the segment
 // follows from the tiles and planes of all its decks unless the autotuner chose
-// one; a block takes one item whatever grid the schedule has.
+// one; a block takes one item.
 template <class Maps, class KS, class KB, class... A>
 void launch_planes(const Target& tg, cudaStream_t s, unsigned key, GridFn tiles, int smem,
                    const PlaneSrc<Maps>& src, KS ks, KB kb, const A&... a) {

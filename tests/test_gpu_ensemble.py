@@ -183,3 +183,17 @@ def test_ensemble_rejects_inconsistent_decks():
     ds[1] = ds[1].replace(end_step=5)
     with pytest.raises(C.CloverError):
         C.Ensemble(ds)
+
+
+def test_staged_launches_have_one_schedule_per_order():
+    """A staged block takes one item: the grid divisor changes neither its launch nor its schedule."""
+    ds = [decks.to_deck(decks.shock(34 + i % 3, 40, 36, 4)) for i in range(24)]
+    e = C.Ensemble(ds)
+    assert e.use_tma(True)
+    for div in (0, 1, 4):
+        e.set_schedule(2, div, 0)
+        e.step(1)
+        staged = [q for q in e.schedule() if q["key"] >> 16 & 1]
+        assert len(staged) >= 8
+        assert all(q["grid_div"] == 0 and q["blocks"] == q["items"] > 0 for q in staged)
+    e.close()
