@@ -103,11 +103,12 @@ __device__ __forceinline__ double ld(const float* p) { return (double)__ldg(p); 
 // no halo of the viscosity just computed. The viscosity's
 // IF((limiter.GT.0.0).OR.(div.GE.0.0)) is taken as "div >= 0 -> 0, else
 // limiter > 0 -> 0, else ..." (the same outcome). The cell minimum folds into
-// deck d's key at min_key[d * kScalarStride] (warp, block, one atomic).
+// deck d's key at min_key[d * kScalarStride] (warp, block, one atomic). With xh
+// the x-face halo of density0 and energy0 is written, which no thread reads here.
 template <class S, class M>
 __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M::kFlat ? 4 : 3) k_visc_dt(M m, GeomArrays ga, double g_small,
     double dtc_safe, double dtu_safe, double dtv_safe, double dtw_safe, double dtdiv_safe,
-    const typename S::rho_t* __restrict__ density0, const typename S::ene_t* __restrict__ energy0,
+    typename S::rho_t* __restrict__ density0, typename S::ene_t* __restrict__ energy0,
     typename S::cs_t* __restrict__ pressure, typename S::cs_t* __restrict__ viscosity,
     typename S::cs_t* __restrict__ soundspeed,
     const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
@@ -228,8 +229,8 @@ __global__ void __launch_bounds__(BX * BY, sizeof(typename S::arith_t) == 4 || M
   if (xh && xh_edge(j, g.x_max)) {
     const long long o = off3(g, j, k, l);
     xh_cell<1>(viscosity, o, j, g.x_max, st<C>(q));
-    xh_cell<1>(const_cast<typename S::rho_t*>(density0), o, j, g.x_max, __ldg(density0 + o));
-    xh_cell<1>(const_cast<typename S::ene_t*>(energy0), o, j, g.x_max, __ldg(energy0 + o));
+    xh_cell<1>(density0, o, j, g.x_max, __ldg(density0 + o));
+    xh_cell<1>(energy0, o, j, g.x_max, __ldg(energy0 + o));
   }
   // calc_dt_kernel.f90:102-149 (the viscosity as stored)
   const A visc = (A)st<C>(q);
@@ -1237,8 +1238,8 @@ const dim3 kBlk(BX, BY);
 template <class S>
 void launch_visc_dt(const Target& tg, cudaStream_t s, const GeomArrays& ga, double g_small,
                     double dtc_safe, double dtu_safe, double dtv_safe, double dtw_safe,
-                    double dtdiv_safe, const typename S::rho_t* density0,
-                    const typename S::ene_t* energy0, typename S::cs_t* pressure,
+                    double dtdiv_safe, typename S::rho_t* density0,
+                    typename S::ene_t* energy0, typename S::cs_t* pressure,
                     typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
                     const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
                     const typename S::vel_t* zvel0, unsigned long long* min_key, bool xh) {
@@ -1419,8 +1420,8 @@ void launch_advec_mom_fused(const Target& tg, cudaStream_t s, int advect_x, int 
 
 #define INSTF(S)                                                                               \
   template void launch_visc_dt<S>(const Target&, cudaStream_t, const GeomArrays&, double, double,  \
-                                  double, double, double, double, const S::rho_t*,             \
-                                  const S::ene_t*, S::cs_t*, S::cs_t*, S::cs_t*,               \
+                                  double, double, double, double, S::rho_t*,                   \
+                                  S::ene_t*, S::cs_t*, S::cs_t*, S::cs_t*,                     \
                                   const S::vel_t*, const S::vel_t*, const S::vel_t*,           \
                                   unsigned long long*, bool);                                  \
   template void launch_pdv_predict_eos<S>(const Target&, cudaStream_t, const double*,            \

@@ -391,12 +391,13 @@ __global__ void __launch_bounds__(BX * BY) k_revert(Geom g, Box b,
 // ---------------------------------------------------------------------------
 // accelerate_kernel.f90:61-109. UM: the cell volume and face areas come from
 // the chunk's uniform-mesh constants (Geom::vol, xa, ya, za) instead of the
-// arrays.
+// arrays. With xh the x-face halo of xvel0 and yvel0 is written, which no thread
+// reads here.
 template <class S, class M, bool UM>
 __global__ void __launch_bounds__(BX * BY, UM ? 5 : 4) k_accelerate(M m, double dt_val,
     const double* dt_ptr, GeomArrays ga, const typename S::rho_t* __restrict__ density0,
     const typename S::cs_t* __restrict__ pressure, const typename S::cs_t* __restrict__ viscosity,
-    const typename S::vel_t* __restrict__ xvel0, const typename S::vel_t* __restrict__ yvel0,
+    typename S::vel_t* __restrict__ xvel0, typename S::vel_t* __restrict__ yvel0,
     const typename S::vel_t* __restrict__ zvel0, typename S::vel_t* __restrict__ xvel1,
     typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1, bool xh) {
   m.run([&](const Geom& g, const Tile& t) {
@@ -458,8 +459,8 @@ __global__ void __launch_bounds__(BX * BY, UM ? 5 : 4) k_accelerate(M m, double 
     xh_node<2>(xvel1, o, j, g.x_max, -un);
     xh_node<2>(yvel1, o, j, g.x_max, vn);
     xh_node<2>(zvel1, o, j, g.x_max, wn);
-    xh_node<1>(const_cast<V*>(xvel0), o, j, g.x_max, -__ldg(xvel0 + o));
-    xh_node<1>(const_cast<V*>(yvel0), o, j, g.x_max, __ldg(yvel0 + o));
+    xh_node<1>(xvel0, o, j, g.x_max, -__ldg(xvel0 + o));
+    xh_node<1>(yvel0, o, j, g.x_max, __ldg(yvel0 + o));
   }
   });
 }
@@ -1736,7 +1737,7 @@ template <class S>
 void launch_accelerate(const Target& tg, cudaStream_t s, double dt_val, const double* dt_ptr,
                        const GeomArrays& ga, const typename S::rho_t* density0,
                        const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
-                       const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
+                       typename S::vel_t* xvel0, typename S::vel_t* yvel0,
                        const typename S::vel_t* zvel0, typename S::vel_t* xvel1,
                        typename S::vel_t* yvel1, typename S::vel_t* zvel1, bool uniform_mesh, bool xh) {
   if (uniform_mesh)
@@ -2043,7 +2044,7 @@ void launch_fill(cudaStream_t s, T* p, long long elems, T value) {
                                  const S::ene_t*, S::ene_t*);                                  \
   template void launch_accelerate<S>(const Target&, cudaStream_t, double, const double*,           \
                                      const GeomArrays&, const S::rho_t*, const S::cs_t*,       \
-                                     const S::cs_t*, const S::vel_t*, const S::vel_t*,          \
+                                     const S::cs_t*, S::vel_t*, S::vel_t*,                      \
                                      const S::vel_t*, S::vel_t*, S::vel_t*, S::vel_t*, bool, bool); \
   template void launch_flux_calc<S>(const Geom&, cudaStream_t, double, const double*,            \
                                     const GeomArrays&, const S::vel_t*, const S::vel_t*,       \

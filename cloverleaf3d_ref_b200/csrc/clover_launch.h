@@ -250,7 +250,7 @@ template <class S>
 void launch_accelerate(const Target& tg, cudaStream_t s, double dt_val, const double* dt_ptr,
                        const GeomArrays& ga, const typename S::rho_t* density0,
                        const typename S::cs_t* pressure, const typename S::cs_t* viscosity,
-                       const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
+                       typename S::vel_t* xvel0, typename S::vel_t* yvel0,
                        const typename S::vel_t* zvel0, typename S::vel_t* xvel1,
                        typename S::vel_t* yvel1, typename S::vel_t* zvel1,
                        bool uniform_mesh = false,  // volume and areas from Geom::vol, xa, ya, za
@@ -373,8 +373,8 @@ void launch_generate_chunk(const Geom& g, cudaStream_t s, const GeomArrays& ga,
 template <class S>
 void launch_visc_dt(const Target& tg, cudaStream_t s, const GeomArrays& ga, double g_small,
                     double dtc_safe, double dtu_safe, double dtv_safe, double dtw_safe,
-                    double dtdiv_safe, const typename S::rho_t* density0,
-                    const typename S::ene_t* energy0, typename S::cs_t* pressure,
+                    double dtdiv_safe, typename S::rho_t* density0,
+                    typename S::ene_t* energy0, typename S::cs_t* pressure,
                     typename S::cs_t* viscosity, typename S::cs_t* soundspeed,
                     const typename S::vel_t* xvel0, const typename S::vel_t* yvel0,
                     const typename S::vel_t* zvel0, unsigned long long* min_key, bool xh);
