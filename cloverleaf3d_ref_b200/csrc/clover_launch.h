@@ -422,10 +422,10 @@ void launch_advec_cell_x(const Target& tg, cudaStream_t s, int sweep, const Geom
 // copied across (left out where a depth-2 halo update of the velocities
 // comes before the next read of the shell, or has written it to both buffers).
 // vol: the uniform cell volume of the chunk (dx*dy*dz).
-// x_maps (one chunk, x sweep): the tensor maps of the sweep's inputs, to run
+// x_maps (x sweep): the tensor maps of the sweep's inputs, to run
 // its shared-memory staged form (clover_tma.cu), which reports a copy that
 // did not arrive in *status; null: the register-marching form.
-// node_maps, vel_maps (one chunk, y/z sweep): the maps of the node pass's and
+// node_maps, vel_maps (y/z sweep): the maps of the node pass's and
 // the velocity pass's inputs, to run their staged forms.
 struct MomXMaps;
 struct NodeMaps;

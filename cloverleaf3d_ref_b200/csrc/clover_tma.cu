@@ -886,7 +886,8 @@ k_accelerate_tma(const __grid_constant__ M m, Geom gp, const double* __restrict_
 // PdV_kernel.f90:120-166 (corrector) + flux_calc_kernel.f90:58-91 over the
 // node box [min, max+1]^3, as k_pdv_flux (clover_fused.cu) forms them. Plane p:
 // the time level 0 and 1 velocities of node plane p (rows k0..k0+8); the
-// cell's own density0, energy0, pressure and viscosity are read directly.
+// cell's own density0, energy0, pressure and viscosity are read directly. The
+// mixed policy's step.
 template <class S>
 struct FluxPlane {
   using V = typename S::vel_t;
@@ -954,6 +955,7 @@ k_pdv_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
     tma_load_box(P::vel(b, 4), &maps.v1, bar, x, y, z);
     tma_load_box(P::vel(b, 5), &maps.w1, bar, x, y, z);
   };
+  static_assert(sizeof(F) == 4, "the mixed policy's form: face fluxes as stored");
   pm.run(l0, l1, status + bt.x * kStatusStride, issue, [&](int l) {
     if (!in_jk) return;
     const R d0_s = c_d;
@@ -1005,25 +1007,12 @@ k_pdv_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
     }
 #undef NV
     if (!(jin && kin && lin)) return;
-    double left_flux, right_flux, bottom_flux, top_flux, back_flux, front_flux;
-    if (sizeof(F) == 8) {  // PdV_kernel.f90:120-131 order
-      left_flux = (g.xa * sx) * 0.125 * dt;
-      right_flux = (g.xa * xsum(1)) * 0.125 * dt;
-      bottom_flux = (g.ya * sy) * 0.125 * dt;
-      top_flux = (g.ya * ysum(1)) * 0.125 * dt;
-      back_flux = (g.za * sz) * 0.125 * dt;
-      front_flux = (g.za * zsum(bu)) * 0.125 * dt;
-    } else {
-      // FP32 volume fluxes: the corrector's face fluxes as the volume fluxes
-      // are stored (the z faces from the corrector's own node sums)
-      auto stored = [&](double area, double s) { return (double)st<F>(0.125 * dt * area * s); };
-      left_flux = (double)vfx0;
-      right_flux = stored(g.xa, xsum(1));
-      bottom_flux = (double)vfy0;
-      top_flux = stored(g.ya, ysum(1));
-      back_flux = stored(g.za, sz);
-      front_flux = stored(g.za, zsum(bu));
-    }
+    // the corrector's face fluxes as the volume fluxes are stored (the z faces
+    // from the corrector's own node sums)
+    auto stored = [&](double area, double s) { return (double)st<F>(0.125 * dt * area * s); };
+    const double left_flux = (double)vfx0, right_flux = stored(g.xa, xsum(1));
+    const double bottom_flux = (double)vfy0, top_flux = stored(g.ya, ysum(1));
+    const double back_flux = stored(g.za, sz), front_flux = stored(g.za, zsum(bu));
     const double total_flux = right_flux - left_flux + top_flux - bottom_flux + front_flux - back_flux;
     const double vol = g.vol;
     const double vol_change_s = vol / (vol + total_flux);
@@ -1046,10 +1035,10 @@ k_pdv_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
 // flux_calc_kernel.f90:58-91 on the velocities just formed, operation for
 // operation as k_accelerate (clover_kernels.cu) and k_pdv_flux
 // (clover_fused.cu). Plane p: density0, pressure and viscosity of cell plane p
-// (rows k0-1..k0+TYN-1) and the three time-level-0 velocities of node plane p
-// (rows k0..). A block's 32 x TYN threads form the new velocities of node
+// (rows k0-1..k0+7) and the three time-level-0 velocities of node plane p
+// (rows k0..). A block's 32 x 8 threads form the new velocities of node
 // plane l+1 into one of two planes in shared memory (and store the nodes the
-// block owns, 31 x (TYN-1) of segment planes), then the corrector, the face
+// block owns, 31 x 7 of segment planes), then the corrector, the face
 // fluxes and their sums of index plane l from node planes l and l+1. The last
 // lane, the last row and one plane per segment are formed twice, by the block
 // that owns them and by its neighbour.
@@ -1062,17 +1051,17 @@ k_pdv_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
 // and two blocks per SM (6.1 ms) lose more warps than they save. The mixed
 // policy keeps the separate kernels: its 136 B per cell fall to 68 B, but its
 // FP32 arithmetic issues longer fused (2.77 -> 2.91 ms).
-template <class S, int TYN>
+template <class S>
 struct AccFluxPlane {
   using V = typename S::vel_t;
   using R = typename S::rho_t;
   using C = typename S::cs_t;
-  static constexpr int kRho = round128((TYN + 1) * kTmaWidth<R> * (int)sizeof(R));
-  static constexpr int kCs = round128((TYN + 1) * kTmaWidth<C> * (int)sizeof(C));
-  static constexpr int kVel = round128(TYN * kTmaWidth<V> * (int)sizeof(V));
+  static constexpr int kRho = round128((TY + 1) * kTmaWidth<R> * (int)sizeof(R));
+  static constexpr int kCs = round128((TY + 1) * kTmaWidth<C> * (int)sizeof(C));
+  static constexpr int kVel = round128(TY * kTmaWidth<V> * (int)sizeof(V));
   static constexpr int kBytes = kRho + 2 * kCs + 3 * kVel;
-  static constexpr int kNew = 3 * TYN * TX * (int)sizeof(V);  // one plane of new velocities
-  static constexpr unsigned kTx = box_bytes<R>(TYN + 1) + 2 * box_bytes<C>(TYN + 1) + 3 * box_bytes<V>(TYN);
+  static constexpr int kNew = 3 * TY * TX * (int)sizeof(V);  // one plane of new velocities
+  static constexpr unsigned kTx = box_bytes<R>(TY + 1) + 2 * box_bytes<C>(TY + 1) + 3 * box_bytes<V>(TY);
   __device__ static R* rho(unsigned char* p) { return (R*)p; }
   __device__ static C* cs(unsigned char* p, int q) { return (C*)(p + kRho + q * kCs); }
   __device__ static V* vel(unsigned char* p, int q) { return (V*)(p + kRho + 2 * kCs + q * kVel); }
@@ -1088,8 +1077,8 @@ __device__ __forceinline__ void x_box31(int t, int d, int& x, int& shift) {
   shift = c - x;
 }
 
-template <class S, class M, int TYN, int RING, int MINB>
-__global__ void __launch_bounds__(TX * TYN, MINB)
+template <class S, class M, int RING, int MINB>
+__global__ void __launch_bounds__(TX * TY, MINB)
 k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ dt_ptr, typename S::rho_t* __restrict__ density1, const typename S::ene_t* __restrict__ energy0,
                typename S::ene_t* __restrict__ energy1, typename S::vel_t* __restrict__ xvel1,
                typename S::vel_t* __restrict__ yvel1, typename S::vel_t* __restrict__ zvel1,
@@ -1097,7 +1086,8 @@ k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
                typename S::vf_t* __restrict__ vol_flux_z, typename S::vel_t* __restrict__ xvel0,
                typename S::vel_t* __restrict__ yvel0, bool xh, int* __restrict__ status) {
   PLANE_BLOCK(m);
-  using P = AccFluxPlane<S, TYN>;
+  using P = AccFluxPlane<S>;
+  static_assert(sizeof(typename S::vf_t) == 8, "the FP64 policy's form: face fluxes unrounded");
   using A = typename S::arith_t;
   using V = typename S::vel_t;
   using R = typename S::rho_t;
@@ -1108,14 +1098,14 @@ k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
   __shared__ unsigned long long full[RING];
   V* const fresh = (V*)(ring + RING * P::kBytes);  // new velocities of node planes of both parities
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int j = g.x_min + 31 * bt.y + tx, k0 = g.y_min + (TYN - 1) * bt.z;
+  const int j = g.x_min + 31 * bt.y + tx, k0 = g.y_min + (TY - 1) * bt.z;
   const int k = k0 + ty;
   const int seg = m.segment(g.z_max - g.z_min + 2);
   const int l0 = g.z_min + seg * bt.w;
   const int l1 = l0 + seg - 1 < g.z_max + 1 ? l0 + seg - 1 : g.z_max + 1;
   const int pfirst = l0 - 1, plast = l1 + 1 < g.z_max + 1 ? l1 + 1 : g.z_max + 1;
   const bool in_node = j <= g.x_max + 1 && k <= g.y_max + 1;
-  const bool own = in_node && tx < TX - 1 && ty < TYN - 1;
+  const bool own = in_node && tx < TX - 1 && ty < TY - 1;
   const bool jin = j <= g.x_max, kin = k <= g.y_max;
   const bool xe = xh && xh_edge(j, g.x_max);
   const double dt = dt_ptr[(long long)bt.x * kScalarStride];
@@ -1210,8 +1200,8 @@ k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
       vn = st<V>((A)P::vel(bu, 1)[cv] - gy(up, lp) - gy(uq, lq));
       wn = st<V>((A)P::vel(bu, 2)[cv] - gz(up, lp) - gz(uq, lq));
       n1[tid] = un;
-      n1[TYN * TX + tid] = vn;
-      n1[2 * TYN * TX + tid] = wn;
+      n1[TY * TX + tid] = vn;
+      n1[2 * TY * TX + tid] = wn;
       if (own && l + 1 >= l0 && l + 1 <= l1) {
         const long long o = off3(g, j, k, l + 1);
         xvel1[o] = un;
@@ -1230,7 +1220,7 @@ k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
     if (own) {
       // velocity q of node (j+a, k+b): time level 0 of buffer bb, level 1 of plane nn
 #define N0(bb, q, a, b) ((A)P::vel(bb, q)[cv + (b) * WV + (a)])
-#define N1(nn, q, a, b) ((A)nn[(q) * TYN * TX + tid + (b) * TX + (a)])
+#define N1(nn, q, a, b) ((A)nn[(q) * TY * TX + tid + (b) * TX + (a)])
       // node plane l+1: its z face flux (the plane the segment owns) and sum
       double zsu = 0.0;
       if (more && jin && kin) {
@@ -1273,25 +1263,13 @@ k_acc_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
         if (jin && kin) {
           const En e0_s = c_e;
           fetch(l + 1);
-          double left_flux, right_flux, bottom_flux, top_flux, back_flux, front_flux;
-          if (sizeof(F) == 8) {  // PdV_kernel.f90:120-131 order
-            left_flux = (g.xa * sx) * 0.125 * dt;
-            right_flux = (g.xa * xsum(1)) * 0.125 * dt;
-            bottom_flux = (g.ya * sy) * 0.125 * dt;
-            top_flux = (g.ya * ysum(1)) * 0.125 * dt;
-            back_flux = (g.za * zs) * 0.125 * dt;
-            front_flux = (g.za * zsu) * 0.125 * dt;
-          } else {
-            // FP32 volume fluxes: the corrector's face fluxes as the volume
-            // fluxes are stored (the z faces from the corrector's own node sums)
-            auto stored = [&](double area, double s) { return (double)st<F>(0.125 * dt * area * s); };
-            left_flux = (double)vfx0;
-            right_flux = stored(g.xa, xsum(1));
-            bottom_flux = (double)vfy0;
-            top_flux = stored(g.ya, ysum(1));
-            back_flux = stored(g.za, zs);
-            front_flux = stored(g.za, zsu);
-          }
+          // PdV_kernel.f90:120-131 order
+          const double left_flux = (g.xa * sx) * 0.125 * dt;
+          const double right_flux = (g.xa * xsum(1)) * 0.125 * dt;
+          const double bottom_flux = (g.ya * sy) * 0.125 * dt;
+          const double top_flux = (g.ya * ysum(1)) * 0.125 * dt;
+          const double back_flux = (g.za * zs) * 0.125 * dt;
+          const double front_flux = (g.za * zsu) * 0.125 * dt;
           const double total_flux =
               right_flux - left_flux + top_flux - bottom_flux + front_flux - back_flux;
           const double vol = g.vol;
@@ -2817,8 +2795,8 @@ constexpr int kStencilMinBlocks = sizeof(typename S::arith_t) == 4 ? 4 : 3;
 
 // shared memory of the accelerate + corrector + flux kernel
 template <class S>
-constexpr int kAccFluxSmem = kStencilRing * AccFluxPlane<S, TY>::kBytes +
-                             2 * AccFluxPlane<S, TY>::kNew;
+constexpr int kAccFluxSmem = kStencilRing * AccFluxPlane<S>::kBytes +
+                             2 * AccFluxPlane<S>::kNew;
 
 template <class S>
 bool stencils_tma_prepare() {
@@ -2826,7 +2804,7 @@ bool stencils_tma_prepare() {
                 kStencilMinBlocks<S>))
     return false;
   if constexpr (kFusedAccFlux<S>)
-    return SET_BOTH(AccMaps, kAccFluxSmem<S>, k_acc_flux_tma, TY, kStencilRing, 3);
+    return SET_BOTH(AccMaps, kAccFluxSmem<S>, k_acc_flux_tma, kStencilRing, 3);
   else
     return SET_BOTH(AccMaps, kStencilRing * AccPlane<S>::kBytes, k_accelerate_tma, kStencilRing,
                     kStencilMinBlocks<S>) &&
@@ -3021,12 +2999,11 @@ void launch_acc_flux_tma(const Target& tg, cudaStream_t s, const double* dt_ptr,
                          typename S::vf_t* vol_flux_z, typename S::vel_t* xvel0,
                          typename S::vel_t* yvel0, bool xh, int* status) {
   GO_BOTH(kKeyPdvFlux, tiles_acc_flux, kAccFluxSmem<S>, maps, AccMaps, k_acc_flux_tma,
-          (TY, kStencilRing, 3), dt_ptr, density1, energy0, energy1, xvel1, yvel1, zvel1, vol_flux_x,
+          (kStencilRing, 3), dt_ptr, density1, energy0, energy1, xvel1, yvel1, zvel1, vol_flux_x,
           vol_flux_y, vol_flux_z, xvel0, yvel0, xh, status);
 }
 
-template <class S>
-constexpr int kNodeMinBlocks = sizeof(typename S::arith_t) == 4 ? 5 : 5;
+constexpr int kNodeMinBlocks = 5;
 
 // calls f with the integral constants of the sweep's direction and post-volume variant
 template <class F>
@@ -3046,7 +3023,7 @@ bool mom_node_tma_prepare() {
     node_variant(q[0], q[1], [&](auto d, auto v) {
       constexpr int D = decltype(d)::value, V = decltype(v)::value;
       ok = ok && SET_BOTH(NodeMaps, (kStencilRing * NodePlane<S, V>::kBytes), k_mom_node_tma, D, V,
-                          kStencilRing, kNodeMinBlocks<S>);
+                          kStencilRing, kNodeMinBlocks);
     });
   return ok;
 }
@@ -3058,7 +3035,7 @@ void launch_mom_node_tma(const Target& tg, cudaStream_t s, int dir, int var,
   node_variant(dir, var, [&](auto d, auto v) {
     constexpr int D = decltype(d)::value, V = decltype(v)::value;
     GO_BOTH(kKeyMomNode | D | (V << 4), tiles_mom_node<D>, (kStencilRing * NodePlane<S, V>::kBytes), maps,
-            NodeMaps, k_mom_node_tma, (D, V, kStencilRing, kNodeMinBlocks<S>), node_flux,
+            NodeMaps, k_mom_node_tma, (D, V, kStencilRing, kNodeMinBlocks), node_flux,
             node_mass_post, node_mass_pre, status);
   });
 }

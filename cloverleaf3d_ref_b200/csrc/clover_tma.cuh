@@ -62,8 +62,8 @@ struct MomXMaps {
 };
 template <class S>
 bool mom_x_tma_prepare();
-// The x momentum sweep of one chunk (sweep 1 or 3 of the step), its planes
-// staged by bulk-tensor copies.
+// The x momentum sweep (sweep 1 or 3 of the step), its planes staged by
+// bulk-tensor copies.
 template <class S>
 void launch_mom_x_tma(const Target& tg, cudaStream_t s, int sweep, const PlaneSrc<MomXMaps>& maps,
                       const GeomArrays& ga, typename S::vel_t* const* vel_out,
@@ -240,10 +240,10 @@ void launch_cell_sweep_tma(const Target& tg, cudaStream_t s, int dir, int var, c
 
 template <class S>
 bool visc_dt_tma_prepare();
-// viscosity + calc_dt (+ ideal_gas) of every interior cell of one chunk, the
-// planes staged by bulk-tensor copies; the cell minimum folds into *min_key,
-// and a block whose copies do not arrive sets CLOVER_STATUS_TIMEOUT in
-// *status.
+// viscosity + calc_dt (+ ideal_gas) of every interior cell, the planes staged
+// by bulk-tensor copies; the cell minimum folds into *min_key, and a block
+// whose copies do not arrive sets CLOVER_STATUS_TIMEOUT in *status (over an
+// ensemble, both of the block's deck).
 template <class S>
 void launch_visc_dt_tma(const Target& tg, cudaStream_t s, const PlaneSrc<ViscMaps>& maps, const GeomArrays& ga,
                         double g_small, double dtc_safe, double dtu_safe, double dtv_safe,
@@ -324,10 +324,6 @@ __device__ __forceinline__ void tma_load_box(void* dst, const CUtensorMap* map,
 __device__ __forceinline__ void tma_map_acquire(const CUtensorMap* map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"((unsigned long long)map)
                : "memory");
-}
-
-__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)map) : "memory");
 }
 #endif
 
