@@ -168,7 +168,7 @@ struct Chunk : ChunkBase {
   // stencils staged through shared memory by bulk-tensor copies (clover_tma.cu),
   // or their register-marching forms
   bool tma = false;      // the staged kernels could be set up
-  bool use_tma = false;  // they run; only with their maps made (make_maps)
+  bool use_tma = false;  // they run (from the first step on, with their maps made: ready_maps)
   // The tensor maps of the staged launches are made before the first of them
   // runs, all or none: the buffer a step leaves density1 and energy1 in follows
   // from the number of sweeps that write out of place. One chunk: by (array, box
@@ -205,6 +205,7 @@ struct Chunk : ChunkBase {
   bool make_maps() {
     if (maps_made || !tma || (plan && !halo_repeat_free)) return maps_made;
     std::vector<unsigned char> image;
+    image.reserve(plan ? (size_t)nd << 14 : 0);  // up to 128 maps a deck
     map_image = &image;
     maps_at.clear();
     bool ok = true;
@@ -232,6 +233,11 @@ struct Chunk : ChunkBase {
       deck_maps = (unsigned char*)dev;
     }
     return maps_made = ok;
+  }
+  // before a step is enqueued or captured: a chunk that is only set up, read or
+  // restored does not pay for the maps
+  void ready_maps() {
+    if (use_tma) use_tma = make_maps();
   }
   // the staged launches of one step, in enqueue_step_fused's order
   bool step_maps(bool ax) {
@@ -571,12 +577,11 @@ struct Chunk : ChunkBase {
     }
     ga = GeomArrays{volume, xarea, yarea, zarea, cellx, celly, cellz, celldx, celldy, celldz,
                     vertexx, vertexy, vertexz, vertexdx, vertexdy, vertexdz};
-    // the stencils that stage their planes with bulk-tensor copies, and their
-    // tensor maps (the arrays they read never move)
+    // the stencils that stage their planes with bulk-tensor copies
     tma = visc_dt_tma_prepare<S>() && mom_x_tma_prepare<S>() && stencils_tma_prepare<S>() &&
           mom_node_tma_prepare<S>() && mom_vel_tma_prepare<S>() && cell_sweep_tma_prepare<S>() &&
           cell_sweep_x_tma_prepare<S>();
-    use_tma = staged_by_default() && make_maps();
+    use_tma = tma && (!plan || halo_repeat_free) && staged_by_default();
 
     dt_cap = deck.end_step < (1 << 22) ? deck.end_step + 16 : (1 << 22);
     sum_cap = dt_cap / (deck.summary_frequency > 0 ? deck.summary_frequency : dt_cap) + 8;
@@ -1262,6 +1267,7 @@ struct Chunk : ChunkBase {
   // before its graphs are captured: a capture cannot allocate them.
   bool capture_graphs() {
     if (plan && !(warm[0] && warm[1])) return false;
+    ready_maps();
     for (int i = 0; i < 2; i++) {
       if (graph[i]) continue;
       cudaGraph_t gr;
@@ -1291,6 +1297,7 @@ struct Chunk : ChunkBase {
   }
 
   int step(int n) {
+    ready_maps();
     if (visit_pending && n > 0) {
       visit_pending = false;
       if (visit() != 0) return -1;
