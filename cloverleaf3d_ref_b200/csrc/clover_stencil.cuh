@@ -61,7 +61,9 @@ __device__ __forceinline__ A lda(const float* p) { return (A)__ldg(p); }
 // the kernels that produce an interior row write its halo columns with it, while
 // the row's ends are at hand. A pass of its own would fetch and rewrite a 32-byte
 // sector per row end (at 512^3 FP64 the x faces were 1.4 ms of the 1.7 ms of a
-// step's halo updates). o: the element's offset; v: the value, negated by the
+// step's halo updates), and the step would take two more halo launches (256
+// decks of 8..12 cells FP64 0.64 ms per step, 0.68 with the halo launches
+// writing the x faces; 1024 of 8..16 2.78 / 2.99). o: the element's offset; v: the value, negated by the
 // caller where the reference negates.
 // cells: 1-m <- m, nx+m <- nx+1-m
 template <int D, class T>

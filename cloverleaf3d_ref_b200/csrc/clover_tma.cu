@@ -1045,9 +1045,11 @@ k_pdv_flux_tma(const __grid_constant__ M m, Geom gp, const double* __restrict__ 
 //
 // The FP64 step's form: the separate kernels move 192 B per cell, this one 120
 // B (the new velocities are not read back, density0, pressure, viscosity and
-// the old velocities are read once), 4.63 -> 4.22 ms at 512^3. It is not bound
-// by HBM any more (2.6 ms): three blocks per SM wait on shared memory, two
-// barriers a plane and FP64 issue. Taller blocks (12 rows, two per SM: 4.39 ms)
+// the old velocities are read once), 4.63 -> 4.22 ms at 512^3 (4.47 with the x
+// faces' halo). It is not bound by HBM any more (2.6 ms): at 192^3 it
+// runs at 41% of DRAM, 40% of the FP64 pipe and 59% of the issue slots, the 5.7
+// warps a scheduler of three blocks per SM waiting on FP64 chains, two barriers
+// a plane and shared memory. Taller blocks (12 rows, two per SM: 4.39 ms)
 // and two blocks per SM (6.1 ms) lose more warps than they save. The mixed
 // policy keeps the separate kernels: its 136 B per cell fall to 68 B, but its
 // FP32 arithmetic issues longer fused (2.77 -> 2.91 ms).
