@@ -107,8 +107,11 @@ struct PlaneBatch {
     // The host copied the maps into device memory, where another ensemble's may
     // have lain: without this fence a load may take the map that its address
     // held before. It is the issuing thread's (kernel parameters need none).
-    // 0.3-1.6% of an ensemble's step: 64 decks of 24..128 cells FP64 8.83 -> 8.89 ms,
-    // 16 of 33..60 0.994 -> 1.009, 512 of 16..48 mixed 5.23 -> 5.25.
+    // It costs 2-3 us a launch where the blocks are few, and less than 1% of a large
+    // ensemble's step (ms per step without and with): 2 decks of 60..90 cells FP64
+    // 0.564 / 0.597, 4 of 30..64 0.343 / 0.351, 16 of 33..60 0.993 / 1.008, 64 of
+    // 24..128 8.83 / 8.90, 512 of 16..48 mixed 5.24 / 5.26. One lane per map and the
+    // block's barrier instead of one thread took as long.
     static_assert(sizeof(Maps) % sizeof(CUtensorMap) == 0, "maps only");
     if (threadIdx.x == 0 && threadIdx.y == 0)
       for (int q = 0; q < (int)(sizeof(Maps) / sizeof(CUtensorMap)); q++)
